@@ -114,6 +114,50 @@ __device__ __forceinline__ i128 mul_wide(int64_t a, int64_t b) {
     return (i128)(((u128)(uint64_t)hi << 64) | (u128)lo);
 }
 
+// Exact sums of 54-bit x 57-bit products in 32-bit multiply-adds.  A vector
+// element |q| < 2^54 and a coefficient |c| < 2^57 are split at 27 bits
+// (value = h 2^27 + l, 0 <= l < 2^27); the four partial products go to three
+// 64-bit accumulators of weights 2^54, 2^27 and 1, one 32 x 32 + 64
+// multiply-add each, where a double-precision multiply-add would hold the
+// FP64 pipe for 16 cycles a warp.  Each term adds less than 2^57.2 to mid, so
+// limb_carry is due every kLimbRun terms; hi stays in range while the |c| of
+// a sum total at most 2^61.
+constexpr int kLimbBits = 27;
+constexpr int kLimbRun = 16;
+
+struct LimbSum {
+    int64_t hi, mid, lo;
+};
+
+__device__ __forceinline__ void limb_split(int64_t v, int& h, int& l) {
+    l = (int)((uint32_t)v & ((1u << kLimbBits) - 1u));
+    h = (int)(v >> kLimbBits);
+}
+
+__device__ __forceinline__ void mad_wide(int64_t& a, int x, int y) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a) : "r"(x), "r"(y));
+}
+
+__device__ __forceinline__ void limb_mac(LimbSum& a, int qh, int ql, int ch, int cl) {
+    mad_wide(a.hi, qh, ch);
+    mad_wide(a.mid, qh, cl);
+    mad_wide(a.mid, ql, ch);
+    mad_wide(a.lo, ql, cl);
+}
+
+__device__ __forceinline__ void limb_carry(LimbSum& a) {
+    constexpr int64_t m = (1LL << kLimbBits) - 1;
+    a.mid += a.lo >> kLimbBits;
+    a.lo &= m;
+    a.hi += a.mid >> kLimbBits;
+    a.mid &= m;
+}
+
+// The sum (after limb_carry) as a 128-bit integer.
+__device__ __forceinline__ i128 limb_total(const LimbSum& a) {
+    return ((i128)a.hi << (2 * kLimbBits)) + (i128)((a.mid << kLimbBits) | a.lo);
+}
+
 // round(v / 2^s), ties toward +inf, s >= 0.
 __device__ __forceinline__ i128 shr_round(i128 v, int s) {
     if (s <= 0) return v;

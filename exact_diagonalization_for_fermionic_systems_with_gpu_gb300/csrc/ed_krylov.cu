@@ -11,8 +11,8 @@
 // FX format (v_k = q_k 2^e_k / beta_k); T's propagator column
 // exp(-i T t) e_0 comes from the host QR solver (ed_tridiag.cpp); and one
 // kernel forms psi(t) = beta_0 sum_k c_k(t) v_k for up to kKrTimes times per
-// pass over the basis.  Each time costs one read of the basis instead of
-// the reference's n matvecs.
+// pass over the basis.  Each time costs a quarter of a read of the basis
+// instead of the reference's n matvecs.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/ed_hubbard.h"
+#include "ed_device.cuh"
 #include "ed_internal.hpp"
 #include "ed_tridiag.hpp"
 
@@ -27,7 +28,11 @@ namespace ed {
 namespace {
 
 constexpr int kKrThreads = 256;
-constexpr int kKrTimes = 8;  // times formed per pass over the basis
+constexpr int kKrTimes = 4;  // times formed per pass over the basis
+constexpr int kKcThreads = 128;
+constexpr int kKcGroup = 8;    // basis vectors per copy group (a complex product adds two terms: kLimbRun / 2)
+constexpr int kKcChunk = 128;  // basis vectors whose coefficients are staged at a time
+static_assert(2 * kKcGroup <= dev::kLimbRun && kKcChunk % kKcGroup == 0, "carry interval");
 constexpr int kKrBlocks = 152 * 8;
 
 int kr_grid(int64_t n) {
@@ -66,40 +71,121 @@ __global__ void k_part(const double* __restrict__ z, int64_t n, int p, double* _
         out[i] = z[2 * i + p];
 }
 
-// out[t] = (accumulate ? out[t] : 0) + f * sum_k coef[t][k] q_k for t < nt,
-// f = i when times_i, else 1; q_k real (CPLX false) or complex.
-template <bool CPLX>
-__global__ void __launch_bounds__(kKrThreads) k_krylov_combine(const int64_t* __restrict__ basis, int64_t stride,
-                                                               int64_t n, int nk, const double2* __restrict__ coef,
-                                                               int nt, double2* __restrict__ out, int64_t out_stride,
-                                                               int accumulate, int times_i) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double2 acc[kKrTimes];
+// out[t] = (accumulate ? out[t] : 0) + f * sum_k c_k(t) q_k for t < NT,
+// f = i when times_i, else 1; q_k real (CPLX false) or complex.  coef holds
+// for each k the NT times' (re high, re low, im high, im low) limbs, scaled
+// by 2^F[t].
+//
+// Bound by instruction issue: the sums are exact integers (limb_mac, four
+// 32-bit multiplies and their 64-bit adds per real product), where FP64
+// multiply-adds issue at 1/64 of the FP32 rate.  A thread forms two adjacent
+// real elements (or one complex one) at NT = 4 times from 16 bytes of every
+// basis vector; at the 48 accumulator registers x 2 that takes, 12 warps an
+// SM are resident, too few to hide load latency, so each thread copies its
+// own words of the next kKcGroup vectors into shared memory (cp.async, no
+// barrier: only the copying thread reads them) while it sums the current
+// ones, and the coefficients are staged for the block kKcChunk vectors at a
+// time.
+struct KrShift {
+    int F[kKrTimes];
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+
+template <bool CPLX, int NT>
+__global__ void __launch_bounds__(kKcThreads, 3) k_krylov_combine(const int64_t* __restrict__ basis, int64_t stride,
+                                                                  int64_t n, int nk, const int4* __restrict__ coef,
+                                                                  const KrShift sh, double2* __restrict__ out,
+                                                                  int64_t out_stride, int accumulate, int times_i) {
+    using namespace dev;
+    constexpr int E = CPLX ? 1 : 2;  // elements per thread
+    __shared__ longlong2 sq[2][kKcGroup][kKcThreads];
+    __shared__ int4 sc[kKcChunk * NT];
+    const int tid = threadIdx.x;
+    const int64_t items = (n + E - 1) / E;
+    const int ngroups = (nk + kKcGroup - 1) / kKcGroup;
+    // every thread of the block runs the same iterations (the coefficient
+    // staging has barriers); threads past the end sum nothing and write nothing
+    for (int64_t i0 = (int64_t)blockIdx.x * kKcThreads; i0 < items; i0 += (int64_t)gridDim.x * kKcThreads) {
+        const int64_t i = i0 + tid;
+        const bool live = i < items;
+        const bool pair = CPLX || 2 * i + 1 < n;  // the second 8-byte word exists
+        const int bytes = live ? (pair ? 16 : 8) : 0;
+        const int64_t* q = basis + (live ? 2 * i : 0);
+        LimbSum re[E][NT], im[E][NT];
 #pragma unroll
-        for (int t = 0; t < kKrTimes; ++t) acc[t] = make_double2(0.0, 0.0);
-        for (int k = 0; k < nk; ++k) {
-            double wr, wi = 0.0;
-            if (CPLX) {
-                const longlong2 q = __ldg(reinterpret_cast<const longlong2*>(basis + (size_t)k * stride) + i);
-                wr = (double)q.x;
-                wi = (double)q.y;
-            } else {
-                wr = (double)__ldg(basis + (size_t)k * stride + i);
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) re[e][t] = im[e][t] = LimbSum{0, 0, 0};
+        auto fetch = [&](int g) {
+#pragma unroll
+            for (int kk = 0; kk < kKcGroup; ++kk) {
+                const int k = g * kKcGroup + kk;
+                if (k < nk) cp_async16(&sq[g & 1][kk][tid], q + (int64_t)k * stride, bytes);  // zero past `bytes`
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        fetch(0);
+        for (int g = 0; g < ngroups; ++g) {
+            const int k0 = g * kKcGroup;
+            if (k0 % kKcChunk == 0) {
+                __syncthreads();  // the previous chunk is no longer read
+                const int m = min(kKcChunk, nk - k0) * NT;
+                for (int c = tid; c < m; c += kKcThreads) sc[c] = __ldg(coef + (size_t)k0 * NT + c);
+                __syncthreads();
+            }
+            if (g + 1 < ngroups) {
+                fetch(g + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            const int4* cg = sc + (size_t)(k0 % kKcChunk) * NT;
+            const int kn = min(kKcGroup, nk - k0);
+#pragma unroll 2
+            for (int kk = 0; kk < kn; ++kk) {
+                const longlong2 v = sq[g & 1][kk][tid];
+                int xh, xl, yh, yl, nh = 0, nl = 0;
+                limb_split(v.x, xh, xl);
+                limb_split(v.y, yh, yl);
+                if (CPLX) limb_split(-v.y, nh, nl);
 #pragma unroll
-            for (int t = 0; t < kKrTimes; ++t) {
-                if (t < nt) {
-                    const double2 c = __ldg(coef + (size_t)t * nk + k);
-                    acc[t].x = fma(c.x, wr, fma(-c.y, wi, acc[t].x));
-                    acc[t].y = fma(c.x, wi, fma(c.y, wr, acc[t].y));
+                for (int t = 0; t < NT; ++t) {
+                    const int4 c = cg[kk * NT + t];
+                    limb_mac(re[0][t], xh, xl, c.x, c.y);
+                    limb_mac(im[0][t], xh, xl, c.z, c.w);
+                    if (CPLX) {
+                        limb_mac(re[0][t], nh, nl, c.z, c.w);
+                        limb_mac(im[0][t], yh, yl, c.x, c.y);
+                    } else {
+                        limb_mac(re[E - 1][t], yh, yl, c.x, c.y);
+                        limb_mac(im[E - 1][t], yh, yl, c.z, c.w);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int t = 0; t < kKrTimes; ++t) {
-            if (t < nt) {
-                double2 v = times_i ? make_double2(-acc[t].y, acc[t].x) : acc[t];
-                double2* o = out + (size_t)t * out_stride + i;
+            for (int e = 0; e < E; ++e)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    limb_carry(re[e][t]);
+                    limb_carry(im[e][t]);
+                }
+        }
+        if (!live) continue;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (e == 1 && !pair) break;
+                double2 v;
+                v.x = i128_to_f64(limb_total(re[e][t]), -sh.F[t]);
+                v.y = i128_to_f64(limb_total(im[e][t]), -sh.F[t]);
+                if (times_i) v = make_double2(-v.y, v.x);
+                double2* o = out + (size_t)t * out_stride + E * i + e;
                 if (accumulate) {
                     const double2 p = *o;
                     v.x += p.x;
@@ -109,6 +195,19 @@ __global__ void __launch_bounds__(kKrThreads) k_krylov_combine(const int64_t* __
             }
         }
     }
+}
+
+template <bool CPLX>
+void launch_combine(int nt, const int64_t* basis, int64_t stride, int64_t n, int nk, const int4* coef, const KrShift& sh,
+                    double2* out, int64_t out_stride, int accumulate, int times_i, cudaStream_t s) {
+    const int64_t items = CPLX ? n : (n + 1) / 2;
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((items + kKcThreads - 1) / kKcThreads, 152 * 32));
+    if (nt == 4)
+        k_krylov_combine<CPLX, 4><<<g, kKcThreads, 0, s>>>(basis, stride, n, nk, coef, sh, out, out_stride, accumulate, times_i);
+    else if (nt == 2)
+        k_krylov_combine<CPLX, 2><<<g, kKcThreads, 0, s>>>(basis, stride, n, nk, coef, sh, out, out_stride, accumulate, times_i);
+    else
+        k_krylov_combine<CPLX, 1><<<g, kKcThreads, 0, s>>>(basis, stride, n, nk, coef, sh, out, out_stride, accumulate, times_i);
 }
 
 // Two-pass-matvec operators (the basis is not kept): out[t][p(i)] +=
@@ -237,14 +336,14 @@ ed_status ed_krylov_evolve(ed_op* op, const ed_krylov_cfg* cfg, const double* ps
         release();
         return ED_ERR_ALLOC;
     }
-    for (const Run& r : runs) {
-        if (r.part >= 0) {
-            k_part<<<kr_grid(D), kKrThreads, 0, s>>>(d0, D, r.part, tmp);
+    for (const Run& run : runs) {
+        if (run.part >= 0) {
+            k_part<<<kr_grid(D), kKrThreads, 0, s>>>(d0, D, run.part, tmp);
             KR_CK(cudaGetLastError());
             ++launches;
         }
         ed_lanczos_result lr{};
-        st = lanczos_run(op, lanczos_ws_slot(op), &lc, r.start, ED_MEM_DEVICE, nullptr, ED_MEM_DEVICE, alpha.data(),
+        st = lanczos_run(op, lanczos_ws_slot(op), &lc, run.start, ED_MEM_DEVICE, nullptr, ED_MEM_DEVICE, alpha.data(),
                          beta.data(), &lr, s, cfg->tol);
         if (st != ED_OK) { release(); return st; }
         launches += lr.launches;
@@ -280,7 +379,7 @@ ed_status ed_krylov_evolve(ed_op* op, const ed_krylov_cfg* cfg, const double* ps
                 for (int k = 0; k < n; ++k) coefk[(size_t)k * n_times + t] = coef[(size_t)t * n + k];
             KR_CK(cudaMemcpyAsync(dcoef, coefk.data(), sizeof(double2) * coefk.size(), cudaMemcpyHostToDevice, s));
             const int cg = kr_grid(D);
-            const int ti = r.part == 1 ? 1 : 0;
+            const int ti = run.part == 1 ? 1 : 0;
             double2* o = reinterpret_cast<double2*>(dout);
             st = lanczos_replay(op, *lanczos_ws_slot(op), n, [&](int k, const int64_t* qk) -> cudaError_t {
                 k_krylov_acc_perm<<<cg, kKrThreads, 0, s>>>(qk, op->dimUP, op->dimDN, op->d_permDN,
@@ -293,18 +392,37 @@ ed_status ed_krylov_evolve(ed_op* op, const ed_krylov_cfg* cfg, const double* ps
             written = true;
             continue;
         }
-        KR_CK(cudaMemcpyAsync(dcoef, coef.data(), sizeof(double2) * coef.size(), cudaMemcpyHostToDevice, s));
-        const int cg = kr_grid(D);
-        for (int t0 = 0; t0 < n_times; t0 += kKrTimes) {
-            const int nt = std::min(kKrTimes, n_times - t0);
-            double2* o = reinterpret_cast<double2*>(dout) + (size_t)t0 * D;
-            const double2* cf = dcoef + (size_t)t0 * n;
+        // groups of 4 times, then 2 and 1: (re, im) limbs, vector-major inside a group
+        struct Group { int t0, nt; size_t at; KrShift sh; };
+        std::vector<Group> groups;
+        std::vector<int4> limbs((size_t)n * n_times);
+        std::vector<double> r(2 * (size_t)n);
+        std::vector<int32_t> hl(4 * (size_t)n);
+        for (int t0 = 0; t0 < n_times;) {
+            const int left = n_times - t0, nt = left >= 4 ? 4 : (left >= 2 ? 2 : 1);
+            Group gr{t0, nt, (size_t)n * t0, {}};
+            for (int t = 0; t < nt; ++t) {
+                for (int k = 0; k < n; ++k) {
+                    const double2 cf = coef[(size_t)(t0 + t) * n + k];
+                    r[2 * k] = cf.x;
+                    r[2 * k + 1] = cf.y;
+                }
+                gr.sh.F[t] = limb_coefs(r.data(), 2 * n, hl.data());
+                for (int k = 0; k < n; ++k)
+                    limbs[gr.at + (size_t)k * nt + t] = make_int4(hl[4 * k], hl[4 * k + 1], hl[4 * k + 2], hl[4 * k + 3]);
+            }
+            groups.push_back(gr);
+            t0 += nt;
+        }
+        static_assert(sizeof(int4) == sizeof(double2), "dcoef holds either form");
+        KR_CK(cudaMemcpyAsync(dcoef, limbs.data(), sizeof(int4) * limbs.size(), cudaMemcpyHostToDevice, s));
+        for (const Group& gr : groups) {
+            double2* o = reinterpret_cast<double2*>(dout) + (size_t)gr.t0 * D;
+            const int4* cf = reinterpret_cast<const int4*>(dcoef) + gr.at;
             if (op->cplx)
-                k_krylov_combine<true><<<cg, kKrThreads, 0, s>>>(basis, stride, D, n, cf, nt, o, D, written ? 1 : 0,
-                                                                 r.part == 1 ? 1 : 0);
+                launch_combine<true>(gr.nt, basis, stride, D, n, cf, gr.sh, o, D, written ? 1 : 0, run.part == 1 ? 1 : 0, s);
             else
-                k_krylov_combine<false><<<cg, kKrThreads, 0, s>>>(basis, stride, D, n, cf, nt, o, D, written ? 1 : 0,
-                                                                  r.part == 1 ? 1 : 0);
+                launch_combine<false>(gr.nt, basis, stride, D, n, cf, gr.sh, o, D, written ? 1 : 0, run.part == 1 ? 1 : 0, s);
             KR_CK(cudaGetLastError());
             ++launches;
         }

@@ -550,6 +550,27 @@ void fx_coefs(const std::vector<double>& r, std::vector<int64_t>* rt, std::vecto
 
 }  // namespace
 
+int limb_coefs(const double* r, int n, int32_t* hl) {
+    double mx = 0.0, sum = 0.0;
+    for (int k = 0; k < n; ++k) {
+        mx = std::max(mx, std::fabs(r[k]));
+        sum += std::fabs(r[k]);
+    }
+    int F = 0;
+    if (mx > 0.0) {
+        int ka, kb;
+        std::frexp(mx, &ka);
+        std::frexp(sum, &kb);
+        F = std::min(56 - ka, 60 - kb);  // one bit below the limits: the roundings of sum and of c_k
+    }
+    for (int k = 0; k < n; ++k) {
+        const int64_t c = (int64_t)std::llrint(std::ldexp(r[k], F));
+        hl[2 * k + 1] = (int32_t)(c & ((1 << dev::kLimbBits) - 1));
+        hl[2 * k] = (int32_t)(c >> dev::kLimbBits);
+    }
+    return F;
+}
+
 }  // namespace ed
 
 namespace ed {

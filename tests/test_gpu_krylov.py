@@ -148,3 +148,32 @@ def test_krylov_two_pass_operator_regenerates_basis(ed, monkeypatch):
         b = ev.krylov_evolve(op2, psi0, [0.2, 0.7, 1.5], max_steps=120, tol=1e-12, result=ib)
         assert ia["steps"] == ib["steps"] and ia["runs"] == ib["runs"]
         assert np.max(np.abs(a - b)) < 1e-13
+
+
+@pytest.mark.parametrize("n_times", [1, 2, 3, 4, 7])
+@pytest.mark.parametrize("case", ["odd_real", "even_real", "complex"])
+def test_krylov_combine_time_groups(ed, orc, case, n_times):
+    """The basis combination at every grouping of times (4, 2, 1) over an odd
+    and an even number of real elements and over complex ones, written and
+    added to, against dense exp(-iHt).  The Krylov dimension (37) is no
+    multiple of the carry interval.  T = 0.4 leaves a truncation error far
+    below 1e-12; the sums are exact, so 1e-11 |psi0| covers T's rounding."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import evolution as ev, lattices as L
+    from conftest import philox_uniform
+    if case == "complex":
+        N, qu, qd, t = 12, 1, 2, L.kagome12(flux=0.7)
+    else:
+        N, qu, qd = (7, 3, 2) if case == "odd_real" else (8, 3, 4)
+        t = L.chain(N, eps=list(philox_uniform(5, N, 2.0)))
+    op = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 2.0)
+    assert op.rows() % 2 == (1 if case == "odd_real" else 0)
+    x = philox_uniform(17, 2 * op.rows())
+    psi0 = x[0::2] + 1j * x[1::2]
+    times = [0.4 * (k + 1) / n_times for k in range(n_times)]
+    ref = dense_evolve(orc.hamiltonian(N, qu, qd, t, t, 2.0).toarray(), psi0, times)
+    got = ev.krylov_evolve(op, psi0, times, max_steps=37)
+    nrm = np.linalg.norm(psi0)
+    assert np.max(np.linalg.norm(got - ref, axis=1)) < 1e-11 * nrm
+    twice = ev.krylov_evolve(op, psi0, times, max_steps=37, out=got.copy())
+    assert np.max(np.linalg.norm(twice - 2 * ref, axis=1)) < 2e-11 * nrm
+    op.close()
