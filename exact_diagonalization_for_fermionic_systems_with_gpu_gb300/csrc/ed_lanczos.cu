@@ -275,23 +275,28 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_reorth(int64_t* __restrict__ 
     }
 }
 
-// evec = sum_k (rt_k q_k >> rs_k) * 2^-F as FP64, plus |evec|^2 partials.
+// evec = sum_k c_k q_k * 2^-F as FP64 (the sum exact, rounded once), plus
+// |evec|^2 partials; c holds the split coefficients of limb_coefs.
 // A thread forms two adjacent elements from 16-byte loads of every slot
 // (slots are 256-byte aligned), kRitzSlots slots per iteration with all their
 // loads issued before the sums; the basis is read once.
-constexpr int kRitzSlots = 16;
+constexpr int kRitzSlots = kLimbRun;
 
 __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__ basis, int64_t n, int64_t stride,
-                                                     int nk, const int64_t* __restrict__ rt,
-                                                     const int* __restrict__ rs, int F, double* __restrict__ out,
-                                                     double* __restrict__ part, unsigned int* counter,
-                                                     double* inv_norm) {
+                                                     int nk, const int2* __restrict__ c, int F,
+                                                     double* __restrict__ out, double* __restrict__ part,
+                                                     unsigned int* counter, double* inv_norm) {
     double ss = 0.0;
     const int64_t npair = n >> 1;
+    auto add = [](LimbSum& a, int64_t q, int2 ck) {
+        int h, l;
+        limb_split(q, h, l);
+        limb_mac(a, h, l, ck.x, ck.y);
+    };
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npair; i += (int64_t)gridDim.x * blockDim.x) {
         const longlong2* q = reinterpret_cast<const longlong2*>(basis) + i;
         const int64_t s2 = stride >> 1;
-        i128 a0 = 0, a1 = 0;
+        LimbSum a0{0, 0, 0}, a1{0, 0, 0};
         int k = 0;
         for (; k + kRitzSlots <= nk; k += kRitzSlots) {
             longlong2 v[kRitzSlots];
@@ -299,20 +304,22 @@ __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__
             for (int t = 0; t < kRitzSlots; ++t) v[t] = __ldg(q + (k + t) * s2);
 #pragma unroll
             for (int t = 0; t < kRitzSlots; ++t) {
-                const int64_t c = __ldg(rt + k + t);
-                const int r = __ldg(rs + k + t);
-                a0 += mul_wide(c, v[t].x) >> r;
-                a1 += mul_wide(c, v[t].y) >> r;
+                const int2 ck = __ldg(c + k + t);
+                add(a0, v[t].x, ck);
+                add(a1, v[t].y, ck);
             }
+            limb_carry(a0);
+            limb_carry(a1);
         }
         for (; k < nk; ++k) {
             const longlong2 v = __ldg(q + k * s2);
-            const int64_t c = __ldg(rt + k);
-            const int r = __ldg(rs + k);
-            a0 += mul_wide(c, v.x) >> r;
-            a1 += mul_wide(c, v.y) >> r;
+            const int2 ck = __ldg(c + k);
+            add(a0, v.x, ck);
+            add(a1, v.y, ck);
         }
-        const double x0 = i128_to_f64(a0, -F), x1 = i128_to_f64(a1, -F);
+        limb_carry(a0);
+        limb_carry(a1);
+        const double x0 = i128_to_f64(limb_total(a0), -F), x1 = i128_to_f64(limb_total(a1), -F);
         out[2 * i] = x0;
         out[2 * i + 1] = x1;
         ss = fma(x0, x0, ss);
@@ -320,9 +327,13 @@ __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__
     }
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
         const int64_t i = n - 1;
-        i128 acc = 0;
-        for (int k = 0; k < nk; ++k) acc += mul_wide(rt[k], basis[(int64_t)k * stride + i]) >> rs[k];
-        const double v = i128_to_f64(acc, -F);
+        LimbSum a{0, 0, 0};
+        for (int k = 0; k < nk; ++k) {
+            add(a, basis[(int64_t)k * stride + i], __ldg(c + k));
+            if (k % kLimbRun == kLimbRun - 1) limb_carry(a);
+        }
+        limb_carry(a);
+        const double v = i128_to_f64(limb_total(a), -F);
         out[i] = v;
         ss = fma(v, v, ss);
     }
@@ -581,6 +592,28 @@ struct WsHolder {
     Workspace ws;
 };
 }  // namespace
+
+// The normalised Ritz vector sum_k (z_k / beta_k) w_k of the stored basis,
+// into out (device): n terms, w_k = q_k 2^e_k.  k_ritz and k_scale, queued on s.
+static ed_status ritz_stored(ed_op* op, Workspace* w, int n, const double* z, const double* beta, double* out,
+                             cudaStream_t s) {
+    std::vector<int> e(n);
+    LZ_CK(cudaMemcpyAsync(e.data(), w->h.e, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+    LZ_CK(cudaStreamSynchronize(s));
+    std::vector<double> r(n);
+    for (int k = 0; k < n; ++k) r[k] = z[k] / beta[k] * std::ldexp(1.0, e[k]);
+    std::vector<int32_t> hl(2 * (size_t)n);
+    const int F = limb_coefs(r.data(), n, hl.data());
+    LZ_CK(cudaMemcpyAsync(w->coef_rt, hl.data(), sizeof(int2) * n, cudaMemcpyHostToDevice, s));
+    // one pair of elements per thread where the grid allows
+    const int64_t gr = std::max<int64_t>(1, std::min<int64_t>((w->DW / 2 + kLzThreads - 1) / kLzThreads, kLzMaxPartials));
+    k_ritz<<<(int)gr, kLzThreads, 0, s>>>(w->basis, w->DW, w->stride, n, reinterpret_cast<const int2*>(w->coef_rt), F,
+                                          out, w->ritz_part, w->ritz_ctr, w->inv_norm);
+    LZ_CK(cudaGetLastError());
+    k_scale<<<lz_grid(w->DW), kLzThreads, 0, s>>>(out, w->DW, w->inv_norm);
+    LZ_CK(cudaGetLastError());
+    return ED_OK;
+}
 
 void lanczos_free_ws(void* p) {
     if (!p) return;
@@ -860,30 +893,11 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     resid = std::fabs(hb[n] * tri[n]);
 
     if (evec && ritz == ED_RITZ_STORED) {
-        std::vector<int> ev(n);
-        std::vector<uint64_t> mv(n);
-        LZ_CK(cudaMemcpyAsync(ev.data(), H.e, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
-        LZ_CK(cudaStreamSynchronize(s));
-        std::vector<double> r(n);
-        for (int k = 0; k < n; ++k) r[k] = tri[1 + k] / hb[k] * std::ldexp(1.0, ev[k]);
-        std::vector<int64_t> rt;
-        std::vector<int> rs;
-        int F;
-        fx_coefs(r, &rt, &rs, &F);
-        LZ_CK(cudaMemcpyAsync(w->coef_rt, rt.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, s));
-        LZ_CK(cudaMemcpyAsync(w->coef_rs, rs.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
         double* out = evec_mem == ED_MEM_DEVICE ? evec : w->fbuf;
-        const int g = lz_grid(DW);
-        // one pair of elements per thread where the grid allows
-        int64_t gr = (DW / 2 + kLzThreads - 1) / kLzThreads;
-        gr = std::max<int64_t>(1, std::min<int64_t>(gr, kLzMaxPartials));
         // in the two-pass matvec's permuted order the sum goes through u
         double* rv = op->striped ? reinterpret_cast<double*>(w->u) : out;
-        k_ritz<<<(int)gr, kLzThreads, 0, s>>>(w->basis, DW, w->stride, n, w->coef_rt, w->coef_rs, F, rv, w->ritz_part,
-                                        w->ritz_ctr, w->inv_norm);
-        LZ_CK(cudaGetLastError());
-        k_scale<<<g, kLzThreads, 0, s>>>(rv, DW, w->inv_norm);
-        LZ_CK(cudaGetLastError());
+        const ed_status rst = ritz_stored(op, w, n, tri.data() + 1, hb.data(), rv, s);
+        if (rst != ED_OK) return rst;
         launches += 2;
         if (op->striped) {
             LZ_CK(launch_permute_f64(op, rv, out, 0, s));
@@ -1193,33 +1207,10 @@ static ed_status lanczos_multi_run(ed_op* const* ops, int B, const ed_lanczos_cf
         }
         tri[0] = tridiag_lowest_host(n, ha.data(), hb.data() + 1, tri.data() + 1);
         if (want_ritz) {
-            std::vector<int> ev(n);
-            if (cudaMemcpy(ev.data(), H.e, sizeof(int) * n, cudaMemcpyDeviceToHost) != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
-            std::vector<double> r(n);
-            for (int k = 0; k < n; ++k) r[k] = tri[1 + k] / hb[k] * std::ldexp(1.0, ev[k]);
-            std::vector<int64_t> rt;
-            std::vector<int> rs;
-            int F;
-            fx_coefs(r, &rt, &rs, &F);
             double* out = evec_mem == ED_MEM_DEVICE ? evecs + offs[b] : w->fbuf;
-            int64_t gr = (DW / 2 + kLzThreads - 1) / kLzThreads;
-            gr = std::max<int64_t>(1, std::min<int64_t>(gr, kLzMaxPartials));
-            if (cudaMemcpyAsync(w->coef_rt, rt.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-                cudaMemcpyAsync(w->coef_rs, rs.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s) != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
-            k_ritz<<<(int)gr, kLzThreads, 0, s>>>(w->basis, DW, w->stride, n, w->coef_rt, w->coef_rs, F, out,
-                                                  w->ritz_part, w->ritz_ctr, w->inv_norm);
-            k_scale<<<lz_grid(DW), kLzThreads, 0, s>>>(out, DW, w->inv_norm);
+            result = ritz_stored(ops[b], w, n, tri.data() + 1, hb.data(), out, s);
+            if (result != ED_OK) break;
             launches += 2;
-            if (cudaGetLastError() != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
             if (evec_mem != ED_MEM_DEVICE &&
                 cudaMemcpyAsync(evecs + offs[b], out, sizeof(double) * DW, cudaMemcpyDeviceToHost, s) != cudaSuccess) {
                 result = ED_ERR_CUDA;
@@ -1381,33 +1372,10 @@ ed_status lanczos_batch_run(ed_op* const* ops, int B, const ed_lanczos_cfg* cfg,
         }
         tri[0] = tridiag_lowest_host(n, ha.data(), hb.data() + 1, tri.data() + 1);
         if (want_ritz) {
-            std::vector<int> ev(n);
-            if (cudaMemcpy(ev.data(), H.e, sizeof(int) * n, cudaMemcpyDeviceToHost) != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
-            std::vector<double> r(n);
-            for (int k = 0; k < n; ++k) r[k] = tri[1 + k] / hb[k] * std::ldexp(1.0, ev[k]);
-            std::vector<int64_t> rt;
-            std::vector<int> rs;
-            int F;
-            fx_coefs(r, &rt, &rs, &F);
             double* out = evec_mem == ED_MEM_DEVICE ? evecs + (size_t)b * DW : w->fbuf;
-            int64_t gr = (DW / 2 + kLzThreads - 1) / kLzThreads;
-            gr = std::max<int64_t>(1, std::min<int64_t>(gr, kLzMaxPartials));
-            if (cudaMemcpyAsync(w->coef_rt, rt.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-                cudaMemcpyAsync(w->coef_rs, rs.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s) != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
-            k_ritz<<<(int)gr, kLzThreads, 0, s>>>(w->basis, DW, w->stride, n, w->coef_rt, w->coef_rs, F, out,
-                                                  w->ritz_part, w->ritz_ctr, w->inv_norm);
-            k_scale<<<lz_grid(DW), kLzThreads, 0, s>>>(out, DW, w->inv_norm);
+            result = ritz_stored(ops[b], w, n, tri.data() + 1, hb.data(), out, s);
+            if (result != ED_OK) break;
             launches += 2;
-            if (cudaGetLastError() != cudaSuccess) {
-                result = ED_ERR_CUDA;
-                break;
-            }
             if (evec_mem != ED_MEM_DEVICE &&
                 cudaMemcpyAsync(evecs + (size_t)b * DW, out, sizeof(double) * DW, cudaMemcpyDeviceToHost, s) != cudaSuccess) {
                 result = ED_ERR_CUDA;

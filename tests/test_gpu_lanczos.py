@@ -410,3 +410,23 @@ def test_autotune_two_pass_chunk_keeps_results(ed):
     lz1.eigen(op, max_steps=6, mode="fixed", ritz="none", seed=2)
     assert lz1.a == lz0.a and lz1.b == lz0.b
     op.close()
+
+
+@pytest.mark.parametrize("steps", [1, 2, 15, 16, 17, 33])
+@pytest.mark.parametrize("qu,qd", [(3, 2), (3, 4), (0, 3)])
+def test_ritz_sum_lengths(ed, qu, qd, steps):
+    """The stored-basis Ritz sum (exact, carried every 16 terms) at term
+    counts around the carry interval, for odd and even row counts, against the
+    second-pass sum, which adds the same vectors one at a time in FP64: at
+    most one rounding of 2^-53 a term apart, 1e-14 in norm."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    from conftest import philox_uniform
+    t = L.chain(7, eps=list(philox_uniform(9, 7, 1.5)))
+    op = ed.Hubbard(ed.H_TBq(7, qu).extend(t), ed.H_TBq(7, qd).extend(t), 3.0)
+    if steps > op.rows() // 3:
+        pytest.skip("more steps than the sector's Krylov space")
+    e1, v1 = ed.Lanczos().eigen(op, max_steps=steps, mode="fixed", ritz="stored", seed=4)
+    e2, v2 = ed.Lanczos().eigen(op, max_steps=steps, mode="fixed", ritz="recompute", seed=4)
+    assert e1 == e2
+    assert np.linalg.norm(v1 - v2) < 1e-14
+    op.close()
