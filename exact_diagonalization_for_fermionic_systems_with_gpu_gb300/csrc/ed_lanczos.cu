@@ -32,6 +32,7 @@ using namespace dev;
 cudaError_t launch_lz_fused(const ed_op* op, const LzFusedArgs& f, cudaStream_t s);
 cudaError_t launch_lz_batch(const ed_op* op, const LzBatchArgs& f, cudaStream_t s);
 cudaError_t launch_lz_multi(int device, int kinds, const LzMultiArgs& f, cudaStream_t s);
+cudaError_t launch_lz_reorth(const ed_op* op, const LzReorthArgs& f, cudaStream_t s);
 
 constexpr int kLzThreads = 256;
 
@@ -182,40 +183,28 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_dots(const int64_t* __restric
     }
 }
 
-// Coefficient on q_k of one Gram-Schmidt pass, from the exact dot
-// <w_k, w> = sum_c part[k][c] 2^(e_k + e_w + 24): <w_k, w> / beta_k^2 in units
-// of w's exponent (the i128 total rounded once, as a host conversion of it
-// would be; IEEE divide and exact scalings).
-__device__ __forceinline__ double reorth_r(const uint64_t* lo, const uint64_t* hi, int k, int chunks, const int* e,
-                                           const double* beta, int ew) {
-    i128 acc = 0;
-    for (int c = 0; c < chunks; ++c)
-        acc += (i128)(((u128)hi[(size_t)k * chunks + c] << 64) | (u128)lo[(size_t)k * chunks + c]);
-    const double dotv = i128_to_f64(acc, e[k] + ew + 24);
-    return dotv / (beta[k] * beta[k]) * ldexp(1.0, e[k] - ew);
-}
-
 // One block: the integer coefficients (rt_k, rs_k) and common shift F of a
-// Gram-Schmidt pass against w_0 .. w_{nk-1} (fx_coefs' rule: 62 - exponent
-// bits per coefficient, less the guard bits of the sum of nk terms), so that
-// no step of a reorthogonalised run waits for the host.
+// Gram-Schmidt pass against w_0 .. w_{nk-1} (62 - exponent bits per
+// coefficient, less the guard bits of the sum of nk terms), so that no step
+// of a reorthogonalised run waits for the host.
 __global__ void __launch_bounds__(kLzThreads) k_reorth_coefs(const uint64_t* __restrict__ lo,
                                                              const uint64_t* __restrict__ hi, int nk, int chunks,
                                                              const int* __restrict__ e, const double* __restrict__ beta,
                                                              int64_t* __restrict__ rt, int* __restrict__ rs,
                                                              int* __restrict__ Fout) {
     __shared__ int sm[kLzThreads / 32];
-    int extra = 0;
-    while ((1 << (10 + extra)) < nk) ++extra;
+    const int extra = reorth_guard(nk);
     const int ew = e[nk];
+    auto coef = [&](int k) {
+        i128 acc = 0;
+        for (int c = 0; c < chunks; ++c)
+            acc += (i128)(((u128)hi[(size_t)k * chunks + c] << 64) | (u128)lo[(size_t)k * chunks + c]);
+        return reorth_r(acc, e[k], beta[k], ew);
+    };
     int fmin = 1 << 20;
     for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-        const double r = reorth_r(lo, hi, k, chunks, e, beta, ew);
-        if (r != 0.0) {
-            int ka;
-            frexp(fabs(r), &ka);
-            fmin = min(fmin, 62 - ka - extra);
-        }
+        const double r = coef(k);
+        if (r != 0.0) fmin = min(fmin, reorth_bits(r, extra));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) fmin = min(fmin, __shfl_xor_sync(0xffffffffu, fmin, o));
@@ -224,22 +213,7 @@ __global__ void __launch_bounds__(kLzThreads) k_reorth_coefs(const uint64_t* __r
     int Fmin = 1 << 20;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) Fmin = min(Fmin, sm[w]);
     if (Fmin == (1 << 20)) Fmin = 0;
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-        const double r = reorth_r(lo, hi, k, chunks, e, beta, ew);
-        int64_t t = 0;
-        int sh = 0;
-        if (r != 0.0) {
-            int ka;
-            frexp(fabs(r), &ka);
-            const int F = 62 - ka - extra;
-            if (F - Fmin < 120) {
-                t = (int64_t)llrint(ldexp(r, F));
-                sh = F - Fmin;
-            }
-        }
-        rt[k] = t;
-        rs[k] = sh;
-    }
+    for (int k = threadIdx.x; k < nk; k += blockDim.x) reorth_fix(coef(k), extra, Fmin, &rt[k], &rs[k]);
     if (threadIdx.x == 0) *Fout = Fmin;
 }
 
@@ -485,7 +459,7 @@ static cudaError_t ensure_mirror(Workspace* w, int max_steps) {
 }
 
 constexpr int kDotChunks = 64;
-constexpr size_t kFusedSync = 192;  // barrier counter at 0, LzRedSet[4] at 32, row-queue counters at 160
+constexpr size_t kFusedSync = 256;  // barrier counter at 0, LzRedSet[4] at 32 ([6] in reorthogonalised runs), row-queue counters at 160
 
 ed_status ensure_ws(ed_op* op, Workspace* w, size_t slots, int64_t DW, int max_steps) {
     if (w->basis && w->basis_slots >= slots && w->DW == DW && w->max_steps >= max_steps) return ED_OK;
@@ -724,6 +698,10 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     const bool rule = fz ? (force || op->mv.dnSched != nullptr)
                          : (op->lz_mode == 2 || (op->lz_mode == 0 && op->mv.dnSched != nullptr));
     bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && rule;
+    // Reorthogonalised runs of small sectors: all steps in one cooperative
+    // launch (ed_lanczos_reorth.cu).
+    bool fused_reorth = cfg->reorth && !op->striped && !prof && !never && max_steps <= kReorthMaxSteps &&
+                        DW <= kReorthMaxN;
     int steps_run = 0;
     int n_fused = 0;  // persistent launches
     int j = 0;
@@ -796,6 +774,23 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
                 j = max_steps;
                 break;
             }
+            j = j1;
+        } else if (fused_reorth) {
+            const int j1 = (cfg->mode == ED_LANCZOS_REFERENCE || stop_beta >= 0.0) ? std::min(max_steps, (j / 10 + 1) * 10)
+                                                                                  : max_steps;
+            LZ_CK(cudaMemsetAsync(w->gbar, 0, kFusedSync, s));
+            LZ_CK(cudaMemsetAsync(w->dot_lo, 0, sizeof(unsigned long long) * 6 * max_steps, s));
+            LzReorthArgs ra{w->basis, w->stride, j, j1, DW, lz, w->gbar,
+                            reinterpret_cast<LzRedSet*>(reinterpret_cast<char*>(w->gbar) + 32),
+                            reinterpret_cast<unsigned long long*>(w->dot_lo), max_steps, grid_wait_limits()};
+            const cudaError_t e = launch_lz_reorth(op, ra, s);
+            if (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge) {
+                cudaGetLastError();
+                fused_reorth = false;
+                continue;
+            }
+            LZ_CK(e);
+            ++launches;
             j = j1;
         } else {
             if (prof) LZ_CK(cudaEventRecord(w->events[4 * j], s));

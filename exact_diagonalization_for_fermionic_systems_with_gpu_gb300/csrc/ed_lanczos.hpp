@@ -94,6 +94,24 @@ struct LzFusedArgs {
     int* stop_word;      // device word, zero at launch
 };
 
+// Arguments of the reorthogonalised run in one launch (k_lz_reorth_run):
+// steps j0 .. j1-1 on the stored basis.
+constexpr int kReorthMaxSteps = 1024;        // coefficients of a pass held in shared memory
+constexpr int64_t kReorthMaxN = 1LL << 20;   // stored values up to which one launch is the faster form
+
+struct LzReorthArgs {
+    int64_t* basis;            // slot j at basis + j * stride
+    int64_t stride;
+    int j0, j1;
+    int64_t n;                 // stored values (rows, or 2 rows complex)
+    LzState* lz;
+    unsigned int* gbar;        // grid-barrier arrivals, zero at launch
+    LzRedSet* red;             // six accumulator sets (step parity, reduction), zero at launch
+    unsigned long long* acc;   // limb sums of the dots, [pass][max_steps][3], zero at launch
+    int max_steps;
+    GridWait wait;
+};
+
 // One instance of a batched run (k_lz_batch): instances share the hopping
 // tables of the first operator (same sector and lattice terms) and differ in
 // their folded diagonals and scalars.

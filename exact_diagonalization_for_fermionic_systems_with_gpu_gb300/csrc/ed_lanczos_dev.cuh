@@ -107,6 +107,40 @@ __device__ inline double lz_inv(double b) { return b > 0.0 ? 1.0 / b : 0.0; }
 // |w_{j+1}| from the exact sum of (q q) >> 16 at exponent e_w.
 __device__ inline double lz_beta(i128 sumsq, int e_w) { return sqrt(i128_to_f64(sumsq, 2 * e_w + 16)); }
 
+// Coefficient on q_k of one Gram-Schmidt pass from the exact dot acc = sum
+// (q_k q_w) >> 24: <w_k, w> / beta_k^2 in units of w's exponent ew (the total
+// rounded once, as a host conversion of it would be; IEEE divide and exact
+// scalings).
+__device__ inline double reorth_r(i128 acc, int ek, double bk, int ew) {
+    const double dotv = i128_to_f64(acc, ek + ew + 24);
+    return scale2(dotv / (bk * bk), ek - ew);
+}
+
+// Guard bits of a sum of nk terms in a Gram-Schmidt pass.
+__device__ inline int reorth_guard(int nk) {
+    int extra = 0;
+    while ((1 << (10 + extra)) < nk) ++extra;
+    return extra;
+}
+
+// Fraction bits that keep r within 62 - extra bits (r != 0).
+__device__ inline int reorth_bits(double r, int extra) {
+    return 62 - frexp_exp(r) - extra;
+}
+
+// The integer coefficient t of r and its right shift sh to the pass's common
+// F (the smallest reorth_bits of the nonzero r).
+__device__ inline void reorth_fix(double r, int extra, int F, int64_t* t, int* sh) {
+    *t = 0;
+    *sh = 0;
+    if (r == 0.0) return;
+    const int f = reorth_bits(r, extra);
+    if (f - F < 120) {
+        *t = (int64_t)llrint(scale2(r, f));
+        *sh = f - F;
+    }
+}
+
 __device__ inline void lz_after_matvec(LzState* lz, int j, i128 alpha_raw, uint64_t m_u, int s_u, int Fc) {
     const int eX = lz->e[j];
     const int e_u = eX - Fc + s_u;

@@ -42,6 +42,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "ed_grid.cuh"
 #include "ed_lanczos.hpp"
 #include "ed_lanczos_dev.cuh"
 #include "ed_matvec_tma.cuh"
@@ -50,20 +51,6 @@ namespace ed {
 using namespace dev;
 
 namespace {
-
-constexpr uint64_t kLimb = (1ULL << 42) - 1;
-
-__device__ __forceinline__ unsigned int ld_relaxed_gpu(const unsigned int* p) {
-    unsigned int v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned int v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // A word of host-mapped memory written by the host (system scope).
 __device__ __forceinline__ int ld_relaxed_sys(const int* p) {
@@ -79,56 +66,6 @@ __device__ __forceinline__ void mirror_slot(HostMirror* hm, const LzState* lz, i
     hm->beta[k] = lz->beta[k];
     __threadfence_system();
     *(volatile int*)&hm->done = k;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Thread 0: add a CTA's sum and max to an accumulator set.
-__device__ __forceinline__ void red_push(LzRedSet* r, i128 v, uint64_t m) {
-    const u128 uv = (u128)v;
-    atomicAdd(&r->l0, (unsigned long long)(uv & kLimb));
-    atomicAdd(&r->l1, (unsigned long long)((uv >> 42) & kLimb));
-    atomicAdd(&r->l2, (unsigned long long)(int64_t)(v >> 84));
-    atomicMax(&r->mx, (unsigned long long)m);
-}
-
-// Thread 0, after the barrier: the grid totals.
-__device__ __forceinline__ void red_pull(const LzRedSet* r, i128& v, uint64_t& m) {
-    const unsigned long long l0 = __ldcg(&r->l0), l1 = __ldcg(&r->l1), l2 = __ldcg(&r->l2);
-    m = __ldcg(&r->mx);
-    v = (i128)((u128)l0 + ((u128)l1 << 42) + ((u128)(i128)(int64_t)l2 << 84));
-}
-
-// Grid-wide barrier on a monotone arrival counter: the k-th barrier of the
-// launch completes when k * gridDim.x CTAs have arrived.  Writes and atomics
-// before it (by any thread of any CTA) are visible after it.  False when the
-// wait gave up; *give_up is then set for the whole CTA.
-__device__ __forceinline__ bool grid_sync(unsigned int* gbar, unsigned int& target, int* give_up, int* err,
-                                          const GridWait& lim) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        // release: this CTA's writes and atomics (ordered before this thread
-        // by the CTA barrier above) before the arrival
-        red_release_gpu_add(gbar, 1u);
-        const unsigned long long t0 = global_ns();
-        const unsigned int want = target + lim.extra;
-        long long it = 0;
-        while (ld_relaxed_gpu(gbar) < want) {
-            if (++it > lim.spin || global_ns() - t0 > lim.ns) {
-                atomicExch(err, 1);
-                *give_up = 1;
-                break;
-            }
-        }
-        fence_acq_rel_gpu();  // acquire: everything released before the last arrival
-    }
-    __syncthreads();
-    return *give_up == 0;
 }
 
 __device__ __forceinline__ unsigned long long* stamps_at(const LzFusedArgs& f, int j) {

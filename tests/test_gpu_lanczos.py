@@ -430,3 +430,43 @@ def test_ritz_sum_lengths(ed, qu, qd, steps):
     assert e1 == e2
     assert np.linalg.norm(v1 - v2) < 1e-14
     op.close()
+
+
+@pytest.mark.parametrize("case", ["tiny", "odd", "odd_long", "complex", "multi_class", "wide", "wider", "one_row", "reference"])
+def test_reorth_one_launch_matches_per_step(ed, monkeypatch, case):
+    """A reorthogonalised run in one cooperative launch gives the per-step
+    kernels' T, E0, Ritz vector and bookkeeping bit for bit: odd and even
+    sectors, complex and multi-class operators, the basis in shared memory or
+    not (long runs, wide ranges), a range wider than the block, one row, and
+    the stop test's launches of ten steps."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    N, qu, qd, t, steps, mode = 8, 4, 4, L.chain(8), 40, "fixed"
+    if case == "tiny":
+        N, qu, qd, t, steps = 4, 2, 2, L.chain(4), 8
+    elif case in ("odd", "odd_long"):
+        N, qu, qd, t = 7, 3, 2, L.chain(7, eps=list(philox_uniform(6, 7, 1.0)))
+        steps = 33 if case == "odd" else 400
+    elif case == "complex":
+        N, qu, qd, t = 12, 2, 3, L.kagome12(flux=0.4)
+    elif case == "multi_class":
+        N, qu, qd, t = 12, 3, 2, L.lieb12(list(philox_uniform(8, 12, 0.5) + 1.0))
+    elif case == "wide":
+        N, qu, qd, t, steps = 10, 5, 5, L.chain(10), 70
+    elif case == "wider":
+        N, qu, qd, t, steps = 11, 5, 5, L.chain(11), 25
+    elif case == "one_row":
+        N, qu, qd, t = 9, 0, 4, L.chain(9, eps=list(philox_uniform(2, 9, 1.0)))
+    else:
+        steps, mode = 200, "reference"
+    got = {}
+    for form in ("launch", "steps"):
+        monkeypatch.setenv("ED_LZ_FUSED", "0") if form == "steps" else monkeypatch.delenv("ED_LZ_FUSED", raising=False)
+        op = op_for(ed, N, qu, qd, t, t, 4.0)
+        lz = ed.Lanczos()
+        e0, v = lz.eigen(op, max_steps=steps, mode=mode, ritz="stored", reorth=True, seed=5)
+        r = lz.result
+        got[form] = (e0, lz.a, lz.b, r.steps, r.status, r.min_bits, r.converged, r.residual), v, r.launches
+        op.close()
+    assert got["launch"][0] == got["steps"][0]
+    assert np.array_equal(got["launch"][1], got["steps"][1])
+    assert got["launch"][2] < got["steps"][2]
