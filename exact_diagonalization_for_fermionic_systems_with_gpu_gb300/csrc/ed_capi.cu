@@ -266,6 +266,30 @@ static ed_status plan_striped(ed_op* op, bool forced, int64_t chunk_cap = 16384)
     return ED_OK;
 }
 
+// Plans and uploads the row-pair matvec where two rows fit shared memory;
+// leaves op->pair false otherwise.
+static ed_status plan_pair(ed_op* op) {
+    if (ed::pair_smem_bytes((op->dimDN + 7) / 8 * 8) == 0) return ED_OK;
+    ed::PairSchedule g;
+    std::string err;
+    if (!ed::build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err)) return ED_OK;
+    if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
+        upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
+        upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
+        return ED_ERR_ALLOC;
+    op->pair_args = {op->d_pairWords, op->d_pairSteps, op->d_pairNeg, g.groups, (int)g.blocks, (int)g.zbase, g.sign};
+    op->pair_smem = ed::pair_smem_bytes(g.zbase);
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
+    // two CTAs of 512 threads an SM where their rows fit, else one of 1,024
+    const bool two = op->pair_smem <= 110 * 1024;
+    op->pair_rows = 2 * op->pair_smem <= 110 * 1024 ? 2 : 1;
+    op->pair_threads = two ? 512 : 1024;
+    op->pair_grid = two ? 2 * sms : sms;
+    op->pair = true;
+    return ED_OK;
+}
+
 // The Lanczos workspace pointer rides on the op (opaque to the header).
 struct ed_op_ext : ed_op {
     OpExtra extra;
@@ -580,11 +604,20 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     // generic kernel (tests compare the two)
     const char* pick = std::getenv("ED_MATVEC");
     const std::string want = pick ? pick : "";
-    if (want != "generic" && want != "striped") op->tma_smem = ed::tma_plan(op, &a);
+    if (want != "generic" && want != "striped" && want != "pair") op->tma_smem = ed::tma_plan(op, &a);
+    // real single-class sectors whose tables leave no room for that plan but
+    // where two rows fit (3,000 to 14,000 down states): the row-pair kernel
+    if (op->tma_smem == 0 && (want.empty() || want == "pair") && !cplx && op->mv_fast) {
+        const ed_status pst = plan_pair(op);
+        if (pst != ED_OK) {
+            ed_op_destroy(op);
+            return pst;
+        }
+    }
     // sectors whose down rows exceed shared memory: the two-pass matvec over
     // a bandwidth-reducing order of the down index (ED_MATVEC=striped forces
     // it where it applies)
-    if (op->tma_smem == 0 && want != "generic" && !cplx && op->mv_fast && op->dimDN % 2 == 0) {
+    if (op->tma_smem == 0 && !op->pair && want != "generic" && !cplx && op->mv_fast && op->dimDN % 2 == 0) {
         const ed_status sst = plan_striped(op, want == "striped");
         if (sst != ED_OK) {
             ed_op_destroy(op);
@@ -628,6 +661,7 @@ ed_status ed_op_destroy(ed_op* op) {
     cudaFree(op->d_upSegE); cudaFree(op->d_upSegP); cudaFree(op->d_dnSegE); cudaFree(op->d_dnSegP);
     cudaFree(op->d_permDN); cudaFree(op->d_sched16); cudaFree(op->d_steps32); cudaFree(op->d_dDNqP);
     cudaFree(op->d_stDNp); cudaFree(op->d_sdn); cudaFree(op->d_negDN);
+    cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);
     cudaFree(op->d_err);
     cudaFree(op->d_dUPq); cudaFree(op->d_dDNq); cudaFree(op->d_stUP); cudaFree(op->d_stDN);
     cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_flag); cudaFree(op->d_io);

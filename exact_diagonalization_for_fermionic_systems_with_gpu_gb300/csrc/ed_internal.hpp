@@ -106,6 +106,18 @@ struct StripedArgs {
     int* err;
 };
 
+// Row-pair matvec (ed_matvec_pair.cu) for real single-class sectors whose
+// tables do not fit shared memory beside the rows but two rows do.
+struct PairArgs {
+    const uint16_t* words;   // PairSchedule
+    const uint8_t* steps;
+    const uint8_t* negcnt;
+    int groups;
+    int blocks;
+    int zbase;
+    int sign;                // +1 / -1: the sign of every entry; 0: mixed
+};
+
 }  // namespace ed
 
 struct ed_op {
@@ -161,6 +173,12 @@ struct ed_op {
     int64_t* d_dDNqP = nullptr;
     uint64_t* d_stDNp = nullptr;
     int64_t* d_sdn = nullptr;   // D down sums, allocated on first use
+    // row-pair matvec
+    bool pair = false;
+    ed::PairArgs pair_args{};
+    int pair_smem = 0, pair_rows = 1, pair_threads = 0, pair_grid = 0;  // bytes of a pair, pairs staged, launch
+    uint16_t* d_pairWords = nullptr;
+    uint8_t *d_pairSteps = nullptr, *d_pairNeg = nullptr;
     std::string last_error;
 };
 
@@ -186,6 +204,9 @@ int tma_grid(const ed_op* op);
 // w < 0: ED_ROW_COST_UP or kRowCostUp.
 void row_plan(const SpinTable& up, int G, std::vector<uint32_t>* start, std::vector<uint32_t>* list,
               std::vector<uint32_t>* queue, double w = -1.0);
+// Shared memory of a row pair of zbase + 8 slots (0: does not fit).
+int pair_smem_bytes(int64_t zbase);
+cudaError_t launch_matvec_pair(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
 cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
 cudaError_t launch_striped_down(const ed_op* op, const StripedArgs& g, cudaStream_t s);
 cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, int out, cudaStream_t s);

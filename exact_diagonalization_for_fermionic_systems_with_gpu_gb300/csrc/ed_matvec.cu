@@ -312,6 +312,7 @@ cudaError_t launch_matvec_f64(const ed_op* op, const int64_t* xq, const int* d_e
     // matvec's permutations in and out cost more than they save (the
     // Lanczos path, which permutes once per solve, uses it)
     if (op->tma_smem > 0) return launch_matvec_tma(op, a, 0, s);
+    if (op->pair) return launch_matvec_pair(op, a, 0, s);
     return op->cplx ? launch_mv<true, 0>(op, a, s) : launch_mv<false, 0>(op, a, s);
 }
 
@@ -331,6 +332,7 @@ cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, vo
         return e;
     }
     if (op->tma_smem > 0) return launch_matvec_tma(op, a, 1, s);
+    if (op->pair) return launch_matvec_pair(op, a, 1, s);
     return op->cplx ? launch_mv<true, 1>(op, a, s) : launch_mv<false, 1>(op, a, s);
 }
 

@@ -1,0 +1,307 @@
+// ed_matvec_pair.cu — one-launch matvec over pairs of up rows, for real
+// operators with one coefficient class per spin whose down rows are too long
+// for the table-resident row engine (14- to 16-site sectors: 3,000 to 14,000
+// down states).
+//
+// A CTA stages rows u and u + 1 of x interleaved in shared memory, 16 bytes a
+// column, so that one 16-byte load of a down hop serves both rows and one
+// decoded schedule entry four additions.  The schedule (ed::PairSchedule, read
+// from L1 / L2, eight steps in a 16-byte word) gives the eight lanes of every
+// quarter warp different bank groups in each step.  A lane computes two columns
+// of both rows: down sums from shared memory, then the up neighbours of each
+// row with 16-byte loads of its column pair (dim_dn even; two 8-byte loads
+// otherwise), the diagonal, one rounding, and the Lanczos partials.
+// The next pair's rows are prefetched into L2 meanwhile.
+//
+// Measured against the one-thread-per-element kernel it replaces there (Lanczos
+// matvec): 14-site chain 7+7 230 -> 186 us, 14-site 7+6 237 -> 154 us, 15-site
+// 7+8 1,470 -> 653 us, 16-site 8+8 6,300 -> 2,570 us.  242 instructions an output
+// at 40 % of the issue slots: bound by the latency of the up loads and the
+// schedule words (sixteen to thirty-two warps an SM at 64 registers) and by the
+// barriers at the ends of the staged rows.  Loading the words and the first up
+// loads ahead of the sums (74 to 90 registers, 24 or 20 warps) was slower.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "ed_device.cuh"
+#include "ed_internal.hpp"
+#include "ed_matvec_common.cuh"
+
+namespace ed {
+using namespace dev;
+
+namespace {
+
+constexpr int kPairUp = 256;  // up entries staged per row (the longest row has 255)
+constexpr int kPairMax = 2;   // row pairs staged at a time
+constexpr int kPairMaxSmem = 220 * 1024;
+
+struct Two {
+    int64_t a, b;  // rows u, u + 1
+};
+
+// 16 bytes of shared memory at a 32-bit address (volatile: ordered with the
+// barriers around the staged rows)
+__device__ __forceinline__ void lds2(uint32_t addr, int64_t& x, int64_t& y) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(addr));
+}
+
+// One step of both rows: slot word w (low 15 bits; sign in bit 15).
+template <bool SIGN>
+__device__ __forceinline__ void pair_step(uint32_t addr, uint32_t m, Two& acc) {
+    int64_t x, y;
+    lds2(addr, x, y);
+    if (SIGN) {
+        uint64_t mm;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(mm) : "r"(m));
+        x ^= (int64_t)mm;
+        y ^= (int64_t)mm;
+    }
+    acc.a += x;
+    acc.b += y;
+}
+
+template <bool SIGN>
+__device__ __forceinline__ void pair_lo(uint32_t xs, uint32_t w, Two& acc) {
+    uint32_t m = 0;
+    if (SIGN) asm("prmt.b32 %0, %1, 0, 0x9999;" : "=r"(m) : "r"(w));  // bit 15 replicated
+    pair_step<SIGN>(xs + ((w & 0x7FFFu) << 4), m, acc);
+}
+
+template <bool SIGN>
+__device__ __forceinline__ void pair_hi(uint32_t xs, uint32_t w, Two& acc) {
+    pair_step<SIGN>(xs + ((w >> 12) & 0x7FFF0u), (uint32_t)((int32_t)w >> 31), acc);
+}
+
+// n (0..8, the same for the warp) steps of a schedule word
+template <bool SIGN>
+__device__ __forceinline__ void pair_group(uint32_t xs, const uint4 w, int n, Two& acc) {
+    switch (n) {
+        case 8: pair_hi<SIGN>(xs, w.w, acc); [[fallthrough]];
+        case 7: pair_lo<SIGN>(xs, w.w, acc); [[fallthrough]];
+        case 6: pair_hi<SIGN>(xs, w.z, acc); [[fallthrough]];
+        case 5: pair_lo<SIGN>(xs, w.z, acc); [[fallthrough]];
+        case 4: pair_hi<SIGN>(xs, w.y, acc); [[fallthrough]];
+        case 3: pair_lo<SIGN>(xs, w.y, acc); [[fallthrough]];
+        case 2: pair_hi<SIGN>(xs, w.x, acc); [[fallthrough]];
+        case 1: pair_lo<SIGN>(xs, w.x, acc); [[fallthrough]];
+        default: break;
+    }
+}
+
+// What a unit needs of one staged row.
+struct PairRow {
+    uint64_t st;
+    int64_t du;
+    int len, npos;
+};
+
+}  // namespace
+
+// OUT = 0: FP64 y; OUT = 1: FX u with the Lanczos epilogue.  VEC: dim_dn even,
+// lane l has columns 2l, 2l + 1 of a 64-column block; otherwise l, l + 32.
+// MERGE: equal hopping coefficients, one product for the up and down sums.
+// P row pairs are staged at a time (more units per barrier for short rows).
+template <int OUT, bool VEC, bool SIGN, bool MERGE>
+__global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g, const int P) {
+    extern __shared__ __align__(128) unsigned char xs[];
+    __shared__ uint32_t uoff[2 * kPairMax][kPairUp];
+    __shared__ PairRow rows[2 * kPairMax];
+    const uint32_t dimUP = (uint32_t)a.dimUP, dimDN = (uint32_t)a.dimDN;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int64_t* __restrict__ xq = a.xq;
+    const uint4* __restrict__ words = reinterpret_cast<const uint4*>(g.words);
+    const uint32_t xs32 = (uint32_t)__cvta_generic_to_shared(xs), pstride = (uint32_t)(g.zbase + 8) * 16u;
+    int E_out = 0, s_u = 0;
+    if (OUT == 0) {
+        E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
+    } else {
+        const int b = a.bq_bits + bitlen_u64(*a.p_mx) - 62;
+        s_u = b > 0 ? b : 0;
+    }
+    const bool unitU = a.unitUP != 0 && a.nclsUP == 1, unitD = a.unitDN != 0 && a.nclsDN == 1;
+    const bool fold = OUT == 1 && MERGE && unitU && s_u > 0 && a.Fc >= s_u;
+    const bool y16 = OUT == 1 || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;  // y may start on any double
+    i128 dot = 0;
+    uint64_t mx = 0;
+    if (tid < 8 * P) *reinterpret_cast<longlong2*>(xs + (tid >> 3) * pstride + (g.zbase + (tid & 7)) * 16) = make_longlong2(0, 0);
+    const uint32_t nitems = (dimUP + 2 * P - 1) / (2 * P);
+    for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const uint32_t ubase = it * 2 * P;
+        const int nrow = (int)min((uint32_t)(2 * P), dimUP - ubase);  // an odd count ends on a pair of one row
+        const int np = (nrow + 1) / 2;
+        __syncthreads();  // the previous rows are no longer read
+        for (int r = 0; r < nrow; ++r) {
+            const uint32_t u = ubase + r, q0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - q0;
+            for (uint32_t k = tid; k < len; k += blockDim.x) uoff[r][k] = (__ldg(a.upEntC + q0 + k) & kColMask) * dimDN;
+            if (tid == r) rows[r] = {__ldg(a.stUP + u), __ldg(a.dUPq + u), (int)len, (int)__ldg(a.upNpos + u)};
+        }
+        for (int p = 0; p < np; ++p) {
+            const int64_t* r0 = xq + (size_t)(ubase + 2 * p) * dimDN;
+            const int64_t* r1 = 2 * p + 1 < nrow ? r0 + dimDN : r0;
+            longlong2* x2 = reinterpret_cast<longlong2*>(xs + p * pstride);
+            if (VEC) {
+#pragma unroll 2
+                for (uint32_t c = 2 * tid; c < dimDN; c += 2 * blockDim.x) {
+                    const longlong2 v0 = __ldg(reinterpret_cast<const longlong2*>(r0 + c));
+                    const longlong2 v1 = __ldg(reinterpret_cast<const longlong2*>(r1 + c));
+                    x2[pair_slot(c)] = make_longlong2(v0.x, v1.x);
+                    x2[pair_slot(c + 1)] = make_longlong2(v0.y, v1.y);
+                }
+            } else {
+#pragma unroll 4
+                for (uint32_t c = tid; c < dimDN; c += blockDim.x)
+                    x2[pair_slot(c)] = make_longlong2(__ldg(r0 + c), __ldg(r1 + c));
+            }
+        }
+        if (tid == 0 && it + gridDim.x < nitems) {
+            // an even row starts on a 16-byte boundary
+            const uint32_t un = (it + gridDim.x) * 2 * P;
+            const uint32_t bytes = (dimDN * min((uint32_t)(2 * P), dimUP - un) * 8u) & ~15u;
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(xq + (size_t)un * dimDN), "r"(bytes)
+                         : "memory");
+        }
+        __syncthreads();
+        for (int t = warp; t < np * g.blocks; t += nwarps) {
+            const int p = t >= g.blocks ? 1 : 0, b = t - p * g.blocks;
+            const uint32_t c0 = 64u * b + (VEC ? 2u * lane : (uint32_t)lane), c1 = VEC ? c0 + 1 : c0 + 32;
+            if (c0 >= dimDN) continue;
+            const bool v1 = VEC || c1 < dimDN;           // the second column exists
+            const bool has1 = 2 * p + 1 < nrow;          // the second row exists
+            const uint32_t u0 = ubase + 2 * p, xp = xs32 + p * pstride;
+            const uint32_t* const uo[2] = {uoff[2 * p], uoff[2 * p + 1]};
+            const int64_t* const xc = xq + c0;
+            auto get = [&](uint32_t off, int64_t& w0, int64_t& w1) {
+                if (VEC) {
+                    const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(xc + off));
+                    w0 = v.x;
+                    w1 = v.y;
+                } else {
+                    w0 = __ldcg(xc + off);
+                    w1 = v1 ? __ldcg(xc + off + 32) : 0;
+                }
+            };
+            // down sums of columns c0, c1 in both rows
+            Two dn[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4* sp = words + ((size_t)(2 * b + h) * g.groups) * 32 + lane;
+                int n = __ldg(g.steps + 2 * b + h);
+                const int64_t neg = SIGN && (h == 0 || v1) ? __ldg(g.negcnt + (h ? c1 : c0)) : 0;
+                dn[h] = Two{neg, neg};
+                for (; n > 8; n -= 8, sp += 32) pair_group<SIGN>(xp, __ldg(sp), 8, dn[h]);
+                pair_group<SIGN>(xp, __ldg(sp), n, dn[h]);
+                if (!SIGN && g.sign < 0) dn[h] = Two{-dn[h].a, -dn[h].b};
+            }
+            // up sums (added to the down sums where one product serves both)
+            Two up[2];
+            if (MERGE) {
+                up[0] = dn[0];
+                up[1] = dn[1];
+            } else {
+                up[0] = up[1] = Two{0, 0};
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if (r == 1 && !has1) break;
+                const int len = rows[2 * p + r].len, npos = rows[2 * p + r].npos;
+                int64_t s0 = 0, s1 = 0;
+                int k = 0;
+#pragma unroll 4
+                for (; k < npos; ++k) {
+                    int64_t w0, w1;
+                    get(uo[r][k], w0, w1);
+                    s0 += w0;
+                    s1 += w1;
+                }
+#pragma unroll 4
+                for (; k < len; ++k) {
+                    int64_t w0, w1;
+                    get(uo[r][k], w0, w1);
+                    s0 -= w0;
+                    s1 -= w1;
+                }
+                (r ? up[0].b : up[0].a) += s0;
+                (r ? up[1].b : up[1].a) += s1;
+            }
+            int64_t qo[2][2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h == 1 && !v1) break;
+                const uint32_t c = h ? c1 : c0;
+                int64_t xr[2];
+                lds2(xp + pair_slot(c) * 16u, xr[0], xr[1]);
+                const int64_t ddn = __ldg(a.dDNq + c);
+                const uint64_t std_ = __ldg(a.stDN + c) & a.mask;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const PairRow& R = rows[2 * p + (has1 ? r : 0)];
+                    const int64_t x = xr[r], us = r ? up[h].b : up[h].a, ds = r ? dn[h].b : dn[h].a;
+                    const int64_t dq = R.du + ddn + a.Uq * (int64_t)__popcll(R.st & std_);
+                    if (OUT == 1 && fold) {
+                        // (S 2^Fc + dq x) >> s_u with Fc >= s_u > 0: the hops' part is a multiple
+                        qo[r][h] = (us << (a.Fc - s_u)) + shr_round_i64(mul_wide(dq, x), s_u);
+                    } else {
+                        i128 ar = 0, ai = 0;
+                        if (MERGE) {
+                            apply_class<false>(ar, ai, us, 0, a.coefUP, 0, unitU, a.Fc);
+                        } else {
+                            if (R.len) apply_class<false>(ar, ai, us, 0, a.coefUP, 0, unitU, a.Fc);
+                            if (a.nclsDN) apply_class<false>(ar, ai, ds, 0, a.coefDN, 0, unitD, a.Fc);
+                        }
+                        ar += mul_wide(dq, x);
+                        qo[r][h] = OUT == 0 ? __double_as_longlong(i128_to_f64(ar, E_out)) : shr_round_i64(ar, s_u);
+                    }
+                    if (OUT == 1 && (r == 0 || has1)) {
+                        const int64_t q = qo[r][h];
+                        dot += mul_wide(x, q) >> 24;
+                        const uint64_t aq = (uint64_t)(q < 0 ? -q : q);
+                        mx = aq > mx ? aq : mx;
+                    }
+                }
+            }
+            int64_t* out = OUT == 0 ? reinterpret_cast<int64_t*>(a.y) : a.uq;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if (r == 1 && !has1) break;
+                int64_t* o = out + (size_t)(u0 + r) * dimDN + c0;
+                if (VEC && y16) {
+                    __stcs(reinterpret_cast<longlong2*>(o), make_longlong2(qo[r][0], qo[r][1]));
+                } else {
+                    o[0] = qo[r][0];
+                    if (v1) o[c1 - c0] = qo[r][1];
+                }
+            }
+        }
+    }
+    if (OUT == 1) mv_lanczos_epilogue(a, dot, mx, s_u);
+}
+
+int pair_smem_bytes(int64_t zbase) {
+    const int64_t bytes = (zbase + 8) * 16;
+    return bytes <= kPairMaxSmem ? (int)bytes : 0;
+}
+
+template <int OUT, bool VEC, bool MERGE>
+static cudaError_t launch_pair3(const ed_op* op, const MvArgs& a, cudaStream_t s) {
+    auto kern = op->pair_args.sign == 0 ? k_mv_pair<OUT, VEC, true, MERGE> : k_mv_pair<OUT, VEC, false, MERGE>;
+    const int smem = op->pair_smem * op->pair_rows;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kern<<<op->pair_grid, op->pair_threads, smem, s>>>(a, op->pair_args, op->pair_rows);
+    return cudaGetLastError();
+}
+
+template <int OUT, bool VEC>
+static cudaError_t launch_pair2(const ed_op* op, const MvArgs& a, cudaStream_t s) {
+    return a.mergeUD ? launch_pair3<OUT, VEC, true>(op, a, s) : launch_pair3<OUT, VEC, false>(op, a, s);
+}
+
+cudaError_t launch_matvec_pair(const ed_op* op, const MvArgs& a, int out, cudaStream_t s) {
+    if (op->dimDN % 2 == 0) return out == 0 ? launch_pair2<0, true>(op, a, s) : launch_pair2<1, true>(op, a, s);
+    return out == 0 ? launch_pair2<0, false>(op, a, s) : launch_pair2<1, false>(op, a, s);
+}
+
+}  // namespace ed

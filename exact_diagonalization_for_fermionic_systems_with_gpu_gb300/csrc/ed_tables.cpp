@@ -621,6 +621,73 @@ bool build_gather_schedule32(const SpinTable& t, const std::vector<uint32_t>& pe
     return true;
 }
 
+bool build_pair_schedule(const SpinTable& t, bool adjacent, PairSchedule* g, std::string* err) {
+    if (t.complex_coef || t.coef.size() > 1) {
+        if (err) *err = "gather schedule: needs a real single-class table";
+        return false;
+    }
+    g->blocks = (t.count + 63) / 64;
+    g->zbase = (t.count + 7) / 8 * 8;
+    if (g->zbase + 8 > (1 << 15)) {
+        if (err) *err = "gather schedule: too many states";
+        return false;
+    }
+    int64_t n_neg = 0;
+    for (int64_t c = 0; c < t.count; ++c)
+        for (int k = 0; k < t.len[c]; ++k) n_neg += t.ent[(size_t)k * t.count + c] & kSignBit ? 1 : 0;
+    g->sign = n_neg == 0 ? 1 : (n_neg == t.nnz ? -1 : 0);
+    g->steps.assign(2 * g->blocks, 0);
+    g->negcnt.assign(64 * g->blocks, 0);
+    // every quarter warp of a half block coloured by itself
+    std::vector<std::vector<uint16_t>> quarter(8 * g->blocks);  // [steps][8]
+    int smax = 1;
+    for (int64_t hb = 0; hb < 2 * g->blocks; ++hb)
+        for (int qw = 0; qw < 4; ++qw) {
+            std::vector<GroupEdge> edges;
+            for (int l8 = 0; l8 < 8; ++l8) {
+                const int lane = 8 * qw + l8;
+                const int64_t c = (hb / 2) * 64 + (adjacent ? 2 * lane + (hb & 1) : lane + 32 * (hb & 1));
+                if (c >= t.count) continue;
+                for (int k = 0; k < t.len[c]; ++k) {
+                    const uint32_t e = t.ent[(size_t)k * t.count + c];
+                    const uint32_t slot = pair_slot(e & kColMask), neg = g->sign == 0 && (e & kSignBit) ? 1u : 0u;
+                    edges.push_back({l8, (int)(slot & 7u), slot | neg << 15});
+                    g->negcnt[c] = (uint8_t)(g->negcnt[c] + neg);
+                }
+            }
+            int D = 0;
+            std::vector<int> pick, freeb;
+            if (!colour_group(edges, &D, &pick, &freeb, err, 8)) return false;
+            std::vector<uint16_t>& w = quarter[4 * hb + qw];
+            w.resize((size_t)D * 8);
+            for (int c = 0; c < D; ++c) {
+                // eight lanes on eight bank groups: a step with an idle lane has a free one
+                const uint16_t z = (uint16_t)(g->zbase + (freeb[c] ? __builtin_ctz((unsigned)freeb[c]) : 0));
+                for (int l8 = 0; l8 < 8; ++l8) {
+                    const int e = pick[(size_t)c * 16 + l8];
+                    w[(size_t)c * 8 + l8] = e >= 0 ? (uint16_t)edges[e].word : z;
+                }
+            }
+            g->steps[hb] = (uint8_t)std::max<int>(g->steps[hb], D);
+            smax = std::max(smax, D);
+        }
+    if (smax > 255) {
+        if (err) *err = "gather schedule: more than 255 steps";
+        return false;
+    }
+    g->groups = (smax + 7) / 8;
+    g->words.assign((size_t)(2 * g->blocks * g->groups * 256), (uint16_t)g->zbase);
+    for (int64_t hb = 0; hb < 2 * g->blocks; ++hb)
+        for (int qw = 0; qw < 4; ++qw) {
+            const std::vector<uint16_t>& w = quarter[4 * hb + qw];
+            for (size_t i = 0; i < w.size(); ++i) {
+                const size_t st = i / 8, lane = 8 * qw + i % 8;
+                g->words[(((size_t)hb * g->groups + st / 8) * 32 + lane) * 8 + st % 8] = w[i];
+            }
+        }
+    return true;
+}
+
 std::vector<uint32_t> unit_queue(const std::vector<uint32_t>& rq, int64_t dimDN, int G) {
     const size_t k = G > 0 ? rq.size() % (size_t)G : 0;
     // parts of a multiple of 32 columns, every one of them non-empty

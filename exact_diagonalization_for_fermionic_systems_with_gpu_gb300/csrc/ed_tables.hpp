@@ -171,6 +171,33 @@ bool window_schedule16(const GatherSchedule32& g, int64_t count, int64_t chunk, 
 // zero slot zbase (offset zbase, + sign).
 std::vector<uint16_t> lane_packed16(const std::vector<uint16_t>& s16, int64_t cpad, int64_t steps, int64_t zbase);
 
+// Gather schedule of the row-pair matvec (ed_matvec_pair.cu), real single-class
+// tables.  Shared memory holds two rows interleaved, 16 bytes a column, column
+// t at slot pair_slot(t); the eight lanes of a quarter warp read eight
+// different 16-byte bank groups (slot mod 8) in every step.  A 64-column block
+// is computed by one warp, two columns a lane: columns 2l and 2l + 1 when
+// `adjacent`, l and l + 32 otherwise; half block 2b + h holds the lanes' h-th
+// columns.  words: lane-packed [2 blocks][groups of 8 steps][32][8], slot |
+// sign << 15; idle lanes read one of eight zero slots from `zbase` at a bank
+// group no busy lane of the step uses.  steps: steps of each half block;
+// negcnt: negative entries of each column.
+struct PairSchedule {
+    int groups = 0;      // groups of eight steps
+    int64_t blocks = 0;  // 64-column blocks
+    int64_t zbase = 0;   // first zero slot; zbase + 8 slots in all
+    int sign = 1;        // +1 / -1: every entry has that sign (no sign bits, no counts); 0: mixed
+    std::vector<uint16_t> words;
+    std::vector<uint8_t> steps;
+    std::vector<uint8_t> negcnt;
+};
+
+// The low three bits take part of the higher ones: a bijection inside groups
+// of eight that spreads the hops of neighbouring columns over the bank groups
+// (16-site chain: 12.0 steps a half block, 13.6 with slot = column, 10.6 its
+// largest hop counts).
+constexpr uint32_t pair_slot(uint32_t t) { return t ^ (((t >> 3) ^ (t >> 6) ^ (t >> 9)) & 7u); }
+bool build_pair_schedule(const SpinTable& t, bool adjacent, PairSchedule* g, std::string* err);
+
 // Build both layouts for one spin from a term list.  Returns ED_OK or an
 // error (bad site, table overflow, complex term in a real operator when
 // allow_complex is false).

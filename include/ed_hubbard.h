@@ -134,7 +134,7 @@ int64_t ed_op_dim_dn(const ed_op* op);
 int ed_op_is_complex(const ed_op* op);
 
 /* The matvec kernel of the operator's Lanczos steps: ED_MV_GENERIC (one
- * thread per element), ED_MV_ROWS (rows staged in shared memory by bulk
+ * thread per element, or row pairs in shared memory), ED_MV_ROWS (rows staged in shared memory by bulk
  * copies) or ED_MV_TWO_PASS (down sums over a bandwidth-reduced down index,
  * then the up term over L2-resident column stripes); -1 for a null op.
  * Chosen at ed_op_create from the sector's shape (ED_MATVEC overrides). */
