@@ -495,7 +495,8 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
               upload(&op->d_dDNq, dq_d.data(), dq_d.size()) == cudaSuccess &&
               upload(&op->d_stUP, op->bup.state.data(), op->bup.state.size()) == cudaSuccess &&
               upload(&op->d_stDN, op->bdn.state.data(), op->bdn.state.size()) == cudaSuccess &&
-              cudaMalloc(&op->d_emax, sizeof(int)) == cudaSuccess && cudaMalloc(&op->d_flag, sizeof(int)) == cudaSuccess;
+              cudaMalloc(&op->d_emax, sizeof(int)) == cudaSuccess && cudaMalloc(&op->d_flag, sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&op->d_apply, sizeof(int) * (ed::kApplyPart + 1)) == cudaSuccess;
     // CSR copies (row-contiguous entries) for the shared-memory kernel
     auto csr = [](const ed::SpinTable& t, std::vector<uint32_t>* ptr, std::vector<uint32_t>* ent) {
         ptr->assign(t.count + 1, 0);
@@ -643,6 +644,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         op->mv.rowQueue = op->d_rowQueue;
         op->mv.unitQueue = op->d_unitQueue;
         op->mv.nunits = (uint32_t)uq.size();
+        op->apply_grid = ed::apply_grid(op);
     }
     *out = op;
     return ED_OK;
@@ -664,7 +666,7 @@ ed_status ed_op_destroy(ed_op* op) {
     cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);
     cudaFree(op->d_err);
     cudaFree(op->d_dUPq); cudaFree(op->d_dDNq); cudaFree(op->d_stUP); cudaFree(op->d_stDN);
-    cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_flag); cudaFree(op->d_io);
+    cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_flag); cudaFree(op->d_apply); cudaFree(op->d_io);
     if (op->h_stage) cudaFreeHost(op->h_stage);
     delete ox;
     return ED_OK;
@@ -705,9 +707,7 @@ ed_status ed_op_perform(ed_op* op, const double* x, double* y, int mem, void* st
         dx = op->d_io;
         dy = op->d_io + DW;
     }
-    if (ed::launch_emax(dx, DW, op->d_emax, op->d_flag, s) != cudaSuccess) return ED_ERR_CUDA;
-    if (ed::launch_to_fx(dx, DW, op->d_emax, op->d_xq, s) != cudaSuccess) return ED_ERR_CUDA;
-    cudaError_t e = ed::launch_matvec_f64(op, op->d_xq, op->d_emax, dy, s);
+    const cudaError_t e = ed::launch_apply(op, dx, dy, op->d_xq, op->d_emax, op->d_flag, op->d_apply, s);
     if (e != cudaSuccess) { op->last_error = cudaGetErrorString(e); return ED_ERR_CUDA; }
     if (mem == ED_MEM_HOST) {
         int flag = 0, err = 0;

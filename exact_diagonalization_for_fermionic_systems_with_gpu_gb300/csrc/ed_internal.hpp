@@ -87,6 +87,19 @@ struct MvArgs {
     int64_t coefDN[2 * kMaxCls];
 };
 
+// FP64 apply in one cooperative launch (k_apply): FX copy of x and the words
+// its grid shares.
+struct ApplyArgs {
+    const double* x;
+    int64_t n;            // stored values
+    int64_t* xq;
+    int* emax;            // out: largest biased exponent of x
+    int* flag;            // out: 1 when x holds a non-finite value
+    int* part;            // kApplyPart ints: each CTA's largest exponent
+    unsigned int* taken;  // the row queue's counter
+};
+constexpr int kApplyPart = 1024;
+
 // Two-pass (striped) matvec for sectors whose down rows exceed shared memory
 // (ed_matvec_striped.cu); the down index is in the op's permuted order.
 struct StripedArgs {
@@ -146,6 +159,7 @@ struct ed_op {
     int64_t* d_xq = nullptr;
     int* d_emax = nullptr;
     int* d_flag = nullptr;
+    int* d_apply = nullptr;     // kApplyPart ints and the queue counter
     double* h_stage = nullptr;  // pinned staging for host-pointer perform
     size_t h_stage_bytes = 0;
     double* d_io = nullptr;     // device x|y for host-pointer perform
@@ -156,6 +170,7 @@ struct ed_op {
     bool mv_fast = false;       // at most one coefficient class per spin
     int tma_smem = 0;           // >0: the shared-memory/TMA matvec is used
     int tma_grid = 0;
+    int apply_grid = 0;         // CTAs of the one-launch FP64 apply (0: its grid cannot be co-resident)
     // two-pass matvec (striped): down index permuted by perm (new -> old)
     bool striped = false;
     int st_grid = 0, st_win = 0, st_chunk = 0, st_zbase = 0;
@@ -187,7 +202,8 @@ namespace ed {
 // Launch-level API used by the C ABI and the Lanczos driver.
 cudaError_t launch_emax(const double* x, int64_t n, int* d_emax, int* d_flag, cudaStream_t s);
 cudaError_t launch_to_fx(const double* x, int64_t n, const int* d_emax, int64_t* xq, cudaStream_t s);
-// y = H x from the FX copy xq (exponent from d_emax), FP64 output.
+// y = H x from the FX copy xq (exponent from d_emax), FP64 output (operators
+// without the one-launch apply).
 cudaError_t launch_matvec_f64(const ed_op* op, const int64_t* xq, const int* d_emax, double* y,
                               cudaStream_t s);
 // u = H x in FX with the Lanczos-step epilogue (dot and max partials).
@@ -207,7 +223,14 @@ void row_plan(const SpinTable& up, int G, std::vector<uint32_t>* start, std::vec
 // Shared memory of a row pair of zbase + 8 slots (0: does not fit).
 int pair_smem_bytes(int64_t zbase);
 cudaError_t launch_matvec_pair(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
-cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
+cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, cudaStream_t s);
+// y = H x from FP64 x: the FX copy into xq (DW + 2 values), then the matvec.
+// words: kApplyPart + 1 ints of scratch.
+cudaError_t launch_apply(const ed_op* op, const double* x, double* y, int64_t* xq, int* d_emax, int* d_flag, int* words,
+                         cudaStream_t s);
+// CTAs of the one-launch apply of an operator with a row-engine plan (0: none).
+int apply_grid(const ed_op* op);
+cudaError_t launch_apply_rows(const ed_op* op, const MvArgs& a, const ApplyArgs& f, cudaStream_t s);
 cudaError_t launch_striped_down(const ed_op* op, const StripedArgs& g, cudaStream_t s);
 cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, int out, cudaStream_t s);
 cudaError_t launch_permute_f64(const ed_op* op, const double* in, double* out, int forward, cudaStream_t s);

@@ -311,9 +311,22 @@ cudaError_t launch_matvec_f64(const ed_op* op, const int64_t* xq, const int* d_e
     // the FP64 apply stays in table order: for one product the two-pass
     // matvec's permutations in and out cost more than they save (the
     // Lanczos path, which permutes once per solve, uses it)
-    if (op->tma_smem > 0) return launch_matvec_tma(op, a, 0, s);
     if (op->pair) return launch_matvec_pair(op, a, 0, s);
     return op->cplx ? launch_mv<true, 0>(op, a, s) : launch_mv<false, 0>(op, a, s);
+}
+
+cudaError_t launch_apply(const ed_op* op, const double* x, double* y, int64_t* xq, int* d_emax, int* d_flag, int* words,
+                         cudaStream_t s) {
+    const int64_t n = op->D * (op->cplx ? 2 : 1);
+    if (op->apply_grid > 0) {
+        MvArgs a = op->mv;
+        a.y = y;
+        const ApplyArgs f{x, n, xq, d_emax, d_flag, words, reinterpret_cast<unsigned int*>(words + kApplyPart)};
+        return launch_apply_rows(op, a, f, s);
+    }
+    cudaError_t e = launch_emax(x, n, d_emax, d_flag, s);
+    if (e == cudaSuccess) e = launch_to_fx(x, n, d_emax, xq, s);
+    return e == cudaSuccess ? launch_matvec_f64(op, xq, d_emax, y, s) : e;
 }
 
 cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, void* lz,
@@ -331,7 +344,7 @@ cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, vo
         if (e == cudaSuccess) e = launch_striped_up(op, a, g, 1, s);
         return e;
     }
-    if (op->tma_smem > 0) return launch_matvec_tma(op, a, 1, s);
+    if (op->tma_smem > 0) return launch_matvec_tma(op, a, s);
     if (op->pair) return launch_matvec_pair(op, a, 1, s);
     return op->cplx ? launch_mv<true, 1>(op, a, s) : launch_mv<false, 1>(op, a, s);
 }

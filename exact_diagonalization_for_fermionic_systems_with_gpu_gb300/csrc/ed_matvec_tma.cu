@@ -3,6 +3,7 @@
 // clusters up to ~14 sites, Kagome/Lieb 12).  The row engine lives in
 // ed_matvec_tma.cuh; this file adds the kernel around it, the shared-memory
 // plan and the launchers.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,7 +20,8 @@ using namespace dev;
 
 constexpr double kRowCostUp = 0.8;  // up-term share of a row's cost at the mean up-row length
 
-template <bool CPLX, int OUT, bool FAST, bool SCHED, bool SEG = false>
+// The Lanczos matvec: FX u with the step's partials.
+template <bool CPLX, bool FAST, bool SCHED, bool SEG = false>
 __global__ void __launch_bounds__(kTmaThreads, 2) k_matvec_tma(const MvArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ uint32_t uoff[kTmaUpStage];
@@ -41,25 +43,135 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_matvec_tma(const MvArgs a) {
     }
     __syncthreads();
 
-    int E_out = 0, s_u = 0;
-    if (OUT == 0) {
-        E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
-    } else {
-        const int b = a.bq_bits + bitlen_u64(*a.p_mx) - 62;
-        s_u = b > 0 ? b : 0;
-    }
+    const int b = a.bq_bits + bitlen_u64(*a.p_mx) - 62;
+    const int s_u = b > 0 ? b : 0;
     i128 dot = 0;
     uint64_t mx = 0;
     uint32_t rc = 0;
     if (!give_up) {
-        tma_rows<CPLX, OUT, FAST, false, SCHED, false, SEG>(a, S, a.xq, a.uq, a.y, rc, E_out, s_u, dot, mx);
+        tma_rows<CPLX, 1, FAST, false, SCHED, false, SEG>(a, S, a.xq, a.uq, nullptr, rc, 0, s_u, dot, mx);
     } else if (threadIdx.x == 0) {
         // the table copy (the wait that gave up, once more) and the first row
         // copy must land before the CTA exits (bounded waits)
         tma::mbar_wait(&S.bar[2], 0);
         if (has_row) tma::mbar_wait(&S.bar[0], 0);
     }
-    if (OUT == 1) mv_lanczos_epilogue(a, dot, mx, s_u);
+    mv_lanczos_epilogue(a, dot, mx, s_u);
+}
+
+// The FP64 apply in one cooperative launch: largest exponent of x, grid
+// barrier, FX copy of x, grid barrier, rows from the unit queue (as in the
+// persistent Lanczos kernel).  As five stream operations (two memsets, the
+// exponent pass, the conversion, the matvec) a Kagome12 apply spent 17 of its
+// 42 us outside the matvec, and an 8-site one 16 us on launches alone; here the
+// down tables land during the first pass, the last rows are split over the
+// CTAs, and nothing is cleared by the host.  The conversion reads x again from
+// L2.  The barriers are the runtime's (cooperative launch: every CTA is
+// resident), so a CTA whose table copy gave up still takes part in both.
+// Kagome12 42.0 -> 30.7 us, Kagome12 with flux 95 -> 84 us, 8-site ring 17.0 ->
+// 10.2 us (calls in a row, host and device).
+template <bool CPLX, bool FAST, bool SCHED, bool SEG = false>
+__global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const ApplyArgs f) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ uint32_t uoff[kTmaUpStage];
+    __shared__ uint32_t uent[kTmaUpStage];
+    __shared__ int give_up, s_emax, s_red[32];
+    __shared__ uint32_t s_next;
+    const TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    const int tid = threadIdx.x;
+    const int64_t gt = (int64_t)blockIdx.x * kTmaThreads + tid, GT = (int64_t)gridDim.x * kTmaThreads;
+    uint32_t u0 = 0;
+    const bool has_row = tma_first_row_dyn<!CPLX>(a, &u0);
+    if (tid == 0) {
+        tma_init(S);
+        tma_issue_tables(a, S);
+    }
+    if (SCHED) tma_zero_slots(a, S);
+    {
+        int e = 0;
+#pragma unroll 4
+        for (int64_t i = gt; i < f.n; i += GT) e = max(e, f64_biased_exp(__ldg(f.x + i)));
+        e = block_max_int(e, s_red);
+        if (tid == 0) {
+            f.part[blockIdx.x] = e;
+            if (blockIdx.x == 0) *f.taken = 0;
+        }
+    }
+    cooperative_groups::this_grid().sync();
+    {
+        int e = 0;
+        for (int b = tid; b < (int)gridDim.x; b += kTmaThreads) e = max(e, __ldcg(f.part + b));
+        e = block_max_int(e, s_red);
+        if (tid == 0) {
+            s_emax = e;
+            if (blockIdx.x == 0) {
+                *f.emax = e;
+                *f.flag = e == 2047 ? 1 : 0;
+            }
+        }
+        __syncthreads();
+    }
+    const int E = fx_exp_from_emax(s_emax);
+#pragma unroll 4
+    for (int64_t i = gt; i < f.n; i += GT) f.xq[i] = f64_to_fx(__ldg(f.x + i), E);
+    if (!tma::mbar_wait(&S.bar[2], 0)) {
+        if (tid == 0) {
+            atomicExch(a.err, 1);
+            tma::mbar_wait(&S.bar[2], 0);  // the table copy must land before the CTA exits (bounded)
+        }
+        give_up = 1;
+    }
+    cooperative_groups::this_grid().sync();
+    if (give_up) return;
+    tma::fence_proxy_async_global();  // xq was written by other CTAs; its rows are read by bulk copies
+    if (tid == 0 && has_row) {
+        tma::fence_proxy_async_smem();
+        tma_issue_row<CPLX>(a, S, f.xq, u0, 0);
+    }
+    uint32_t rc = 0;
+    i128 dot = 0;
+    uint64_t mx = 0;
+    tma_rows<CPLX, 0, FAST, true, SCHED, true, SEG, false, !CPLX>(a, S, f.xq, nullptr, a.y, rc, E - a.Fc, 0, dot, mx,
+                                                                  f.taken, &s_next);
+}
+
+static const void* apply_kernel(const ed_op* op) {
+    if (op->cplx)
+        return op->mv_fast ? (const void*)k_apply<true, true, false>
+               : op->mv.upSegE ? (const void*)k_apply<true, false, false, true>
+                               : (const void*)k_apply<true, false, false>;
+    if (!op->mv_fast)
+        return op->mv.upSegE ? (const void*)k_apply<false, false, false, true> : (const void*)k_apply<false, false, false>;
+    return op->mv.dnSched ? (const void*)k_apply<false, true, true> : (const void*)k_apply<false, true, false>;
+}
+
+int apply_grid(const ed_op* op) {
+    const void* fn = apply_kernel(op);
+    // the kernel's shared-memory limit at the device's largest (never lowered
+    // by a smaller operator), so that a call sets no attribute
+    int per_sm = 0, sms = 0, coop = 0, optin = 0;
+    cudaFuncAttributes fa;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, op->device) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, fn) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTmaThreads, op->tma_smem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, op->device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    // a CTA for every unit of work, as many as are resident together
+    const int64_t units = op->cplx ? op->dimUP : (int64_t)op->mv.nunits;
+    const int64_t g = std::min<int64_t>({(int64_t)per_sm * sms, op->tma_grid, std::max<int64_t>(units, 1), kApplyPart});
+    return coop ? (int)g : 0;
+}
+
+cudaError_t launch_apply_rows(const ed_op* op, const MvArgs& a, const ApplyArgs& f, cudaStream_t s) {
+    MvArgs av = a;
+    ApplyArgs fv = f;
+    void* args[] = {&av, &fv};
+    return cudaLaunchCooperativeKernel(apply_kernel(op), dim3((unsigned)op->apply_grid), dim3(kTmaThreads), args,
+                                       (size_t)op->tma_smem, s);
 }
 
 // Shared-memory plan: returns the dynamic bytes (0 when the sector does not
@@ -104,42 +216,29 @@ int tma_plan(const ed_op* op, MvArgs* a) {
     return (int)off;
 }
 
-template <bool CPLX, int OUT, bool FAST, bool SCHED, bool SEG = false>
-static cudaError_t launch_tma4(const ed_op* op, const MvArgs& a, cudaStream_t s) {
-    auto kern = k_matvec_tma<CPLX, OUT, FAST, SCHED, SEG>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->tma_smem);
-    if (e != cudaSuccess) return e;
-    kern<<<op->tma_grid, kTmaThreads, op->tma_smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <int OUT>
-static cudaError_t launch_tma_out(const ed_op* op, const MvArgs& a, cudaStream_t s) {
-    if (op->cplx) {
-        if (op->mv_fast) return launch_tma4<true, OUT, true, false>(op, a, s);
-        return a.upSegE ? launch_tma4<true, OUT, false, false, true>(op, a, s) : launch_tma4<true, OUT, false, false>(op, a, s);
-    }
+static const void* matvec_kernel(const ed_op* op) {
+    if (op->cplx)
+        return op->mv_fast ? (const void*)k_matvec_tma<true, true, false>
+               : op->mv.upSegE ? (const void*)k_matvec_tma<true, false, false, true>
+                               : (const void*)k_matvec_tma<true, false, false>;
     if (!op->mv_fast)
-        return a.upSegE ? launch_tma4<false, OUT, false, false, true>(op, a, s) : launch_tma4<false, OUT, false, false>(op, a, s);
-    return a.dnSched ? launch_tma4<false, OUT, true, true>(op, a, s) : launch_tma4<false, OUT, true, false>(op, a, s);
+        return op->mv.upSegE ? (const void*)k_matvec_tma<false, false, false, true>
+                             : (const void*)k_matvec_tma<false, false, false>;
+    return op->mv.dnSched ? (const void*)k_matvec_tma<false, true, true> : (const void*)k_matvec_tma<false, true, false>;
 }
 
-cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, int out, cudaStream_t s) {
-    return out == 0 ? launch_tma_out<0>(op, a, s) : launch_tma_out<1>(op, a, s);
+cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, cudaStream_t s) {
+    const void* fn = matvec_kernel(op);
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, op->tma_smem);
+    if (e != cudaSuccess) return e;
+    MvArgs av = a;
+    void* args[] = {&av};
+    return cudaLaunchKernel(fn, dim3((unsigned)op->tma_grid), dim3(kTmaThreads), args, (size_t)op->tma_smem, s);
 }
 
 int tma_grid(const ed_op* op) {
     int per_sm = 0;
-    const void* f;
-    if (op->cplx)
-        f = op->mv_fast ? (const void*)k_matvec_tma<true, 1, true, false>
-            : op->mv.upSegE ? (const void*)k_matvec_tma<true, 1, false, false, true>
-                            : (const void*)k_matvec_tma<true, 1, false, false>;
-    else if (!op->mv_fast)
-        f = op->mv.upSegE ? (const void*)k_matvec_tma<false, 1, false, false, true>
-                          : (const void*)k_matvec_tma<false, 1, false, false>;
-    else
-        f = op->mv.dnSched ? (const void*)k_matvec_tma<false, 1, true, true> : (const void*)k_matvec_tma<false, 1, true, false>;
+    const void* f = matvec_kernel(op);
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, op->tma_smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kTmaThreads, op->tma_smem) != cudaSuccess ||
         per_sm < 1)

@@ -8,7 +8,7 @@
 // cudaMalloc/cudaFree can cause.  For them ed_op_perform_noalloc takes its
 // scratch from the file-scope array below instead.
 //
-// Scratch: kNoAllocMaxElems int64 values (16 MiB) plus two ints, resident on
+// Scratch: kNoAllocMaxElems int64 values (16 MiB) plus the apply's shared words, resident on
 // a GPU from the first call on it until the process exits.  Under CUDA's
 // lazy module loading the array's module is loaded, and its 16 MiB reserved,
 // when the first call resolves the array's address: a caller whose allocator
@@ -32,7 +32,7 @@ constexpr int kMaxDevices = 64;
 // Device-side scratch.  In host code these names are only stand-ins: the
 // device addresses come from cudaGetSymbolAddress, once per device.
 static __device__ __align__(256) int64_t g_noalloc_xq[kNoAllocMaxElems + 2];  // + padding read by row copies
-static __device__ __align__(256) int g_noalloc_words[2];  // [0] max exponent, [1] non-finite flag
+static __device__ __align__(256) int g_noalloc_words[2 + ed::kApplyPart + 1];  // max exponent, non-finite flag, apply scratch
 
 struct Resolved {
     int64_t* xq = nullptr;
@@ -76,10 +76,8 @@ extern "C" ed_status ed_op_perform_noalloc(ed_op* op, const double* x, double* y
     const ed_status st = resolve(op->device, &r);
     if (st != ED_OK) return st;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    // launch_emax zeroes both words before the reduction, so nothing from the
-    // previous call leaks into this one
-    if (ed::launch_emax(x, n, r.words, r.words + 1, s) != cudaSuccess) return ED_ERR_CUDA;
-    if (ed::launch_to_fx(x, n, r.words, r.xq, s) != cudaSuccess) return ED_ERR_CUDA;
-    if (ed::launch_matvec_f64(op, r.xq, r.words, y, s) != cudaSuccess) return ED_ERR_CUDA;
+    // the apply writes both words itself, so nothing from the previous call
+    // leaks into this one
+    if (ed::launch_apply(op, x, y, r.xq, r.words, r.words + 1, r.words + 2, s) != cudaSuccess) return ED_ERR_CUDA;
     return ED_OK;
 }

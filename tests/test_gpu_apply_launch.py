@@ -1,0 +1,83 @@
+"""The one-launch FP64 apply (exponent pass, conversion and rows in one
+cooperative kernel) against the generic kernels' three launches, bit for bit:
+the same exact integer sums from the same fixed-point copy of x."""
+import numpy as np
+import pytest
+
+from conftest import philox_uniform
+
+pytestmark = pytest.mark.gpu
+
+
+def apply_cases():
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    r = list(philox_uniform(4, 12, 0.5) + 1.0)
+    return [
+        # units below and above the grid, odd rows, one row, every row-engine variant
+        ("ring4", 4, 2, 2, L.chain(4), 1.0),
+        ("ring8", 8, 4, 4, L.chain(8), 4.0),
+        ("ring7_odd", 7, 3, 2, L.chain(7), 2.0),
+        ("one_row", 9, 0, 4, L.chain(9), 2.0),
+        ("one_state", 6, 6, 6, L.chain(6), 2.0),
+        ("kagome12_66", 12, 6, 6, L.kagome12(), 8.0),
+        ("kagome12_84_odd", 12, 8, 4, L.kagome12(), 8.0),
+        ("no_schedule", 10, 5, 5, L.chain(10), 1.0),
+        ("lieb12_classes", 12, 5, 6, L.lieb12(r), 4.0),
+        ("kagome12_two_classes", 12, 4, 5, [(k, i, j, v * (1.0 if i % 2 else 0.5), p) for k, i, j, v, p in L.kagome12()], 2.0),
+        ("flux", 12, 4, 6, L.kagome12(flux=0.3, peierls=True), 4.0),
+        ("flux_one_class", 8, 3, 4, [("P", i, (i + 1) % 8, -1.0, 0.0) for i in range(8)], 4.0),
+    ]
+
+
+@pytest.mark.parametrize("case", apply_cases(), ids=lambda c: c[0])
+def test_one_launch_apply_matches_generic(ed, monkeypatch, case):
+    import torch
+    name, N, qu, qd, t, U = case
+    ops = {}
+    for kind in ("auto", "generic"):
+        if kind == "generic":
+            monkeypatch.setenv("ED_MATVEC", "generic")
+        elif name == "no_schedule":
+            monkeypatch.setenv("ED_NO_SCHED", "1")
+        ops[kind] = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), U)
+        monkeypatch.delenv("ED_MATVEC", raising=False)
+        monkeypatch.delenv("ED_NO_SCHED", raising=False)
+    n = ops["auto"].rows()
+    rng = np.random.default_rng(5)
+    dt = torch.complex128 if ops["auto"].is_complex else torch.float64
+    for scale in (1.0, 1e-200, 0.0, 3e150):  # a new exponent on every call
+        x = rng.standard_normal(n) + (1j * rng.standard_normal(n) if ops["auto"].is_complex else 0.0)
+        xd = torch.from_numpy(x * scale).to(dt).cuda()
+        ys = []
+        for op in ops.values():
+            y = torch.empty(n, dtype=dt, device="cuda")
+            op.Hubbard_mv(xd, y)
+            ys.append(y)
+        assert torch.equal(ys[0], ys[1]), scale
+    with pytest.raises(Exception):
+        bad = np.full(n, np.nan, dtype=np.complex128 if ops["auto"].is_complex else np.float64)
+        ops["auto"].matvec(bad)
+    good = ops["auto"].matvec(x)
+    assert np.array_equal(good, ops["generic"].matvec(x))
+
+
+def test_one_launch_apply_in_a_graph(ed):
+    """Captured once and replayed on new values of x, on a side stream."""
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    op = ed.Hubbard(ed.H_TBq(8, 4).extend(L.chain(8)), ed.H_TBq(8, 4).extend(L.chain(8)), 4.0)
+    x = torch.zeros(op.rows(), dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(x)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        op.Hubbard_mv(x, y)
+    s.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        op.Hubbard_mv(x, y)
+    for seed in range(3):
+        v = np.random.default_rng(seed).standard_normal(op.rows()) * 10.0 ** seed
+        x.copy_(torch.from_numpy(v))
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(y.cpu().numpy(), op.matvec(v))
