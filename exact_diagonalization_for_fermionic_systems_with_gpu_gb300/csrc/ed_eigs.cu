@@ -14,10 +14,14 @@
 // is done as a thick restart (Wu & Simon, SIAM J. Matrix Anal. Appl. 22
 // (2000) 602): the k Ritz vectors V Z[:, i] and the normalised residual become
 // the new first k + 1 basis vectors and the recurrence continues from there.
-// Every new vector is orthogonalised twice against the whole basis (classical
-// Gram-Schmidt, "twice is enough"), so the projected matrix T = V^T H V is
-// read off the Gram-Schmidt coefficients; its eigenpairs come from a cyclic
-// Jacobi solve on the host (T is ncv x ncv).  Convergence and the restart
+// Every new vector w = H v_j is orthogonalised twice ("twice is enough"): first
+// against the vectors it has more than rounding-level components on, v_j and
+// v_{j-1} (after a restart, for j = k, against all), then against the whole
+// basis.  The first pass over the other vectors would only subtract terms of
+// size eps |w|, which the second pass removes as well, so the basis is as
+// orthogonal as after two full passes for half the arithmetic.  The projected
+// matrix T = V^T H V is read off the Gram-Schmidt coefficients; its eigenpairs
+// come from a cyclic Jacobi solve on the host (T is ncv x ncv).  Convergence and the restart
 // size follow Spectra's rules (the ARPACK dsaup2 adjustment).  One cycle of
 // ncv - k steps is launched without a host synchronisation: the
 // coefficients are reduced on the device in a fixed order.
@@ -29,6 +33,7 @@
 #include <vector>
 
 #include "../../include/ed_hubbard.h"
+#include "ed_device.cuh"
 #include "ed_internal.hpp"
 
 namespace ed {
@@ -37,68 +42,169 @@ cudaError_t launch_random(double* f, int64_t n, uint64_t seed, cudaStream_t s);
 namespace {
 
 constexpr int kEgThreads = 256;
-constexpr int kEgChunks = 152 * 2;  // row chunks of a dot product (fixed: determinism)
-constexpr int kEgOut = 8;           // vectors formed per pass of the combination kernel
+constexpr int kEgWarps = kEgThreads / 32;
+constexpr int kEgDots = 16;  // dots whose partial sums a thread holds at a time
+constexpr int kEgBlocks = 152 * 4;
+constexpr int kEgOut = 8;    // vectors formed per pass of the combination kernel
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int w = kEgThreads / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+// The kernels below are bound by the FP64 pipe (1/64 of the FP32 rate: one
+// multiply-add holds a warp scheduler's pipe for 64 cycles), not by memory, so
+// they spend none of it on anything but the sums: scalars are computed by one
+// thread of one block, and the sixteen partial sums of a warp are reduced
+// together (16 additions a lane instead of 80).
+
+// 16 values per lane, summed over the 32 lanes: lane l gets the total of value
+// l >> 1.  Every step halves the values a lane keeps; fixed order.
+__device__ __forceinline__ double reduce16(double* s) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 8; h > 0; h >>= 1) {  // lanes differing in bit 2h
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double send = up ? s[i] : s[i + h], keep = up ? s[i + h] : s[i];
+            s[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+        }
+    }
+    return s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+}
+
+// A pair of elements 2i, 2i + 1 of a vector of n values (16-byte aligned; the
+// missing one of an odd n is 0).
+__device__ __forceinline__ double2 ld_pair(const double* __restrict__ v, int64_t i, int64_t n) {
+    if (2 * i + 1 < n) return *reinterpret_cast<const double2*>(v + 2 * i);
+    return make_double2(v[2 * i], 0.0);
+}
+
+__device__ __forceinline__ void st_pair(double* __restrict__ v, int64_t i, int64_t n, double2 x) {
+    if (2 * i + 1 < n) *reinterpret_cast<double2*>(v + 2 * i) = x;
+    else v[2 * i] = x.x;
+}
+
+// w <- w - sum_t loc_c[t] V_{loc0 + t} (t < nloc <= 2, written back), then
+// coef[k] = <V_k, w>, k0 <= k < k0 + nk, and tcol[k] = coef[k] + (loc_c where k
+// is a local vector, or with acc what tcol[k] was).  Block partials; the last
+// block sums them in index order.
+__global__ void __launch_bounds__(kEgThreads) k_eg_dots(const double* __restrict__ V, int64_t stride, int k0, int nk,
+                                                        double* __restrict__ w, int64_t n, int loc0, int nloc,
+                                                        const double* __restrict__ loc_c, double* __restrict__ part,
+                                                        unsigned int* counter, double* __restrict__ coef,
+                                                        double* __restrict__ tcol, int acc) {
+    __shared__ double sh[kEgWarps][kEgDots];
+    const int64_t np = (n + 1) >> 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double l0 = nloc > 0 ? __ldg(loc_c) : 0.0, l1 = nloc > 1 ? __ldg(loc_c + 1) : 0.0;
+    for (int g0 = 0; g0 < nk; g0 += kEgDots) {
+        const double* Vg = V + (size_t)(k0 + g0) * stride;
+        const int ng = min(kEgDots, nk - g0);
+        double s[kEgDots];
+#pragma unroll
+        for (int t = 0; t < kEgDots; ++t) s[t] = 0.0;
+        for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < np; i += (int64_t)gridDim.x * kEgThreads) {
+            double2 x = ld_pair(w, i, n);
+            if (g0 == 0 && nloc > 0) {
+                const double2 a = ld_pair(V + (size_t)loc0 * stride, i, n);
+                x.x = fma(-l0, a.x, x.x);
+                x.y = fma(-l0, a.y, x.y);
+                if (nloc > 1) {
+                    const double2 b = ld_pair(V + (size_t)(loc0 + 1) * stride, i, n);
+                    x.x = fma(-l1, b.x, x.x);
+                    x.y = fma(-l1, b.y, x.y);
+                }
+                st_pair(w, i, n, x);
+            }
+#pragma unroll
+            for (int t = 0; t < kEgDots; ++t)
+                if (t < ng) {
+                    const double2 v = ld_pair(Vg + (size_t)t * stride, i, n);
+                    s[t] = fma(v.x, x.x, s[t]);
+                    s[t] = fma(v.y, x.y, s[t]);
+                }
+        }
+        const double r = reduce16(s);
+        __syncthreads();  // the previous group's sums are read
+        if ((lane & 1) == 0) sh[warp][lane >> 1] = r;
         __syncthreads();
+        if (threadIdx.x < ng) {
+            double t = 0.0;
+#pragma unroll
+            for (int q = 0; q < kEgWarps; ++q) t += sh[q][threadIdx.x];
+            part[(size_t)(g0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+            __threadfence();
+        }
     }
-    const double r = sh[0];
     __syncthreads();
-    return r;
+    if (!dev::elect_last_block(counter)) return;
+    for (int k = warp; k < nk; k += kEgWarps) {
+        double t = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(part + (size_t)k * gridDim.x + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) {
+            const int kk = k0 + k;
+            coef[k] = t;
+            if (tcol) {
+                double base = acc ? tcol[kk] : 0.0;
+                if (nloc > 0 && kk == loc0) base = l0;
+                if (nloc > 1 && kk == loc0 + 1) base = l1;
+                tcol[kk] = base + t;
+            }
+        }
+    }
+    if (threadIdx.x == 0) *counter = 0;
 }
 
-// part[k * gridDim.x + chunk] = sum over the chunk's rows of V_k[i] * w[i]
-__global__ void __launch_bounds__(kEgThreads) k_mdot(const double* __restrict__ V, int64_t stride,
-                                                     const double* __restrict__ w, int64_t n, double* __restrict__ part) {
-    __shared__ double sh[kEgThreads];
-    const int k = blockIdx.y;
-    const double* v = V + (size_t)k * stride;
-    double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kEgThreads)
-        s = fma(v[i], w[i], s);
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[(size_t)k * gridDim.x + blockIdx.x] = s;
-}
-
-// coef[k] = sum_c part[k][c] (fixed order); tcol[k] = (acc ? tcol[k] : 0) + coef[k]
-__global__ void __launch_bounds__(kEgThreads) k_reduce(const double* __restrict__ part, int chunks,
-                                                       double* __restrict__ coef, double* __restrict__ tcol, int acc) {
-    __shared__ double sh[kEgThreads];
-    const int k = blockIdx.x;
-    double s = 0.0;
-    for (int c = threadIdx.x; c < chunks; c += kEgThreads) s += part[(size_t)k * chunks + c];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) {
-        coef[k] = s;
-        if (tcol) tcol[k] = (acc ? tcol[k] : 0.0) + s;
+// w <- w - sum_k coef[k] V_k, k < nk; with beta: beta[0] = |w| and *inv = 1 / |w|
+// (0 for a zero vector), block partials summed by the last block in index order.
+__global__ void __launch_bounds__(kEgThreads) k_eg_update(double* __restrict__ w, const double* __restrict__ V,
+                                                          int64_t stride, int nk, const double* __restrict__ coef,
+                                                          int64_t n, double* __restrict__ part, unsigned int* counter,
+                                                          double* __restrict__ beta, double* __restrict__ inv) {
+    __shared__ double sh[32];
+    const int64_t np = (n + 1) >> 1;
+    double ss = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < np; i += (int64_t)gridDim.x * kEgThreads) {
+        double2 x = ld_pair(w, i, n);
+#pragma unroll 4
+        for (int k = 0; k < nk; ++k) {
+            const double c = -__ldg(coef + k);
+            const double2 v = ld_pair(V + (size_t)k * stride, i, n);
+            x.x = fma(c, v.x, x.x);
+            x.y = fma(c, v.y, x.y);
+        }
+        if (nk > 0) st_pair(w, i, n, x);
+        if (beta) {
+            ss = fma(x.x, x.x, ss);
+            ss = fma(x.y, x.y, ss);
+        }
+    }
+    if (!beta) return;
+    ss = dev::block_sum_f64(ss, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = ss;
+    if (!dev::elect_last_block(counter)) return;
+    if (threadIdx.x < 32) {
+        double t = 0.0;
+        for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) t += __ldcg(part + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) {
+            const double b = sqrt(t);
+            *beta = b;
+            *inv = b > 0.0 ? 1.0 / b : 0.0;
+            *counter = 0;
+        }
     }
 }
 
-// w[i] -= sum_k coef[k] V_k[i]
-__global__ void __launch_bounds__(kEgThreads) k_maxpy(double* __restrict__ w, const double* __restrict__ V,
-                                                      int64_t stride, int nk, const double* __restrict__ coef,
-                                                      int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kEgThreads) {
-        double s = w[i];
-        for (int k = 0; k < nk; ++k) s = fma(-__ldg(coef + k), __ldg(V + (size_t)k * stride + i), s);
-        w[i] = s;
-    }
-}
-
-// v = w / beta, beta = sqrt(*ss) (v = 0 when beta = 0); beta_out = beta
+// v = w * (*inv)
 __global__ void __launch_bounds__(kEgThreads) k_scale(double* __restrict__ v, const double* __restrict__ w,
-                                                      const double* __restrict__ ss, int64_t n,
-                                                      double* __restrict__ beta_out) {
-    const double b = sqrt(*ss);
-    const double r = b > 0.0 ? 1.0 / b : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *beta_out = b;
-    for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kEgThreads)
-        v[i] = w[i] * r;
+                                                      const double* __restrict__ inv, int64_t n) {
+    const double r = __ldg(inv);
+    const int64_t np = (n + 1) >> 1;
+    for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < np; i += (int64_t)gridDim.x * kEgThreads) {
+        const double2 x = ld_pair(w, i, n);
+        st_pair(v, i, n, make_double2(x.x * r, x.y * r));
+    }
 }
 
 // out_t[i] = sum_k coef[t * nk + k] V_k[i] for t < nt
@@ -124,6 +230,13 @@ __global__ void __launch_bounds__(kEgThreads) k_combine(const double* __restrict
 int eg_grid(int64_t n) {
     const int64_t g = (n + kEgThreads - 1) / kEgThreads;
     return (int)std::max<int64_t>(1, std::min<int64_t>(g, 152 * 8));
+}
+
+// Blocks of the kernels that take pairs of elements (fixed by n: the sums'
+// order, and so every bit of the result, follows from it).
+int eg_pair_grid(int64_t n) {
+    const int64_t g = ((n + 1) / 2 + kEgThreads - 1) / kEgThreads;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(g, kEgBlocks));
 }
 
 }  // namespace
@@ -220,15 +333,17 @@ ed_status ed_eigs_lowest(ed_op* op, const ed_eigs_cfg* cfg, const double* start,
 
     double *V = nullptr, *Vn = nullptr, *w = nullptr, *part = nullptr, *coef = nullptr, *Tdev = nullptr,
            *beta = nullptr, *zc = nullptr;
+    unsigned int* counter = nullptr;
     auto release = [&]() {
         cudaFree(V); cudaFree(Vn); cudaFree(w); cudaFree(part); cudaFree(coef); cudaFree(Tdev); cudaFree(beta);
-        cudaFree(zc);
+        cudaFree(zc); cudaFree(counter);
     };
     if (cudaMalloc(&V, sizeof(double) * (size_t)(m + 1) * stride) != cudaSuccess ||
         cudaMalloc(&Vn, sizeof(double) * (size_t)(m + 1) * stride) != cudaSuccess ||
         cudaMalloc(&w, sizeof(double) * (size_t)stride) != cudaSuccess ||
-        cudaMalloc(&part, sizeof(double) * (size_t)(m + 1) * kEgChunks) != cudaSuccess ||
-        cudaMalloc(&coef, sizeof(double) * (m + 1)) != cudaSuccess ||
+        cudaMalloc(&part, sizeof(double) * (size_t)(m + 1) * kEgBlocks) != cudaSuccess ||
+        cudaMalloc(&coef, sizeof(double) * (m + 4)) != cudaSuccess ||
+        cudaMalloc(&counter, sizeof(unsigned int)) != cudaSuccess ||
         cudaMalloc(&Tdev, sizeof(double) * (size_t)m * m) != cudaSuccess ||
         cudaMalloc(&beta, sizeof(double) * (m + 1)) != cudaSuccess ||
         cudaMalloc(&zc, sizeof(double) * (size_t)m * (m + 1)) != cudaSuccess) {
@@ -252,14 +367,18 @@ ed_status ed_eigs_lowest(ed_op* op, const ed_eigs_cfg* cfg, const double* start,
         EG_CK(launch_random(w, n, cfg->seed, s));
         ++launches;
     }
-    auto norm_into = [&](double* dst, int bidx) -> cudaError_t {
-        k_mdot<<<dim3(kEgChunks, 1), kEgThreads, 0, s>>>(w, stride, w, n, part);
-        k_reduce<<<1, kEgThreads, 0, s>>>(part, kEgChunks, coef, nullptr, 0);
-        k_scale<<<g, kEgThreads, 0, s>>>(dst, w, coef, n, beta + bidx);
-        launches += 3;
+    EG_CK(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
+    const int gp = eg_pair_grid(n);
+    double* const inv = coef + m + 1;    // 1 / |w|
+    double* const local = coef + m + 2;  // coefficients on v_{j-1}, v_j of the first pass
+    // dst = w / |w| after w <- w - V[0..nk) coef, |w| to beta[bidx]
+    auto normalise = [&](double* dst, int nk, int bidx) -> cudaError_t {
+        k_eg_update<<<gp, kEgThreads, 0, s>>>(w, V, stride, nk, coef, n, part, counter, beta + bidx, inv);
+        k_scale<<<gp, kEgThreads, 0, s>>>(dst, w, inv, n);
+        launches += 2;
         return cudaGetLastError();
     };
-    EG_CK(norm_into(V, 0));
+    EG_CK(normalise(V, 0, 0));
 
     std::vector<double> T((size_t)m * m, 0.0), Tc((size_t)m * m), theta(m), Z((size_t)m * m), hb(m + 1);
     const double eps = std::numeric_limits<double>::epsilon();
@@ -273,15 +392,25 @@ ed_status ed_eigs_lowest(ed_op* op, const ed_eigs_cfg* cfg, const double* start,
         for (int j = k0; j < m; ++j) {
             const ed_status ps = ed_op_perform(op, V + (size_t)j * stride, w, ED_MEM_DEVICE, stream);
             if (ps != ED_OK) { release(); return ps; }
-            launches += 3;
+            ++launches;
             ++n_mv;
-            for (int pass = 0; pass < 2; ++pass) {
-                k_mdot<<<dim3(kEgChunks, j + 1), kEgThreads, 0, s>>>(V, stride, w, n, part);
-                k_reduce<<<j + 1, kEgThreads, 0, s>>>(part, kEgChunks, coef, Tdev + (size_t)j * m, pass);
-                k_maxpy<<<g, kEgThreads, 0, s>>>(w, V, stride, j + 1, coef, n);
-                launches += 3;
+            double* tcol = Tdev + (size_t)j * m;
+            // w = H v_j: the first pass against v_{j-1} and v_j, or against all
+            // in the step that follows a restart (T's arrow), the second against all
+            const bool full = j == k0 && j > 0;
+            const int nloc = full ? 0 : (j > 0 ? 2 : 1), loc0 = full ? 0 : j + 1 - nloc;
+            if (full) {
+                k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, 0, 0, nullptr, part, counter, coef, tcol, 0);
+                k_eg_update<<<gp, kEgThreads, 0, s>>>(w, V, stride, j + 1, coef, n, part, counter, nullptr, nullptr);
+                launches += 2;
+            } else {
+                k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, loc0, nloc, w, n, 0, 0, nullptr, part, counter, local, nullptr, 0);
+                ++launches;
             }
-            EG_CK(norm_into(V + (size_t)(j + 1) * stride, j + 1));
+            k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, loc0, nloc, local, part, counter, coef, tcol,
+                                                full ? 1 : 0);
+            ++launches;
+            EG_CK(normalise(V + (size_t)(j + 1) * stride, j + 1, j + 1));
         }
         EG_CK(cudaMemcpyAsync(Tc.data(), Tdev, sizeof(double) * (size_t)m * m, cudaMemcpyDeviceToHost, s));
         EG_CK(cudaMemcpyAsync(hb.data(), beta, sizeof(double) * (m + 1), cudaMemcpyDeviceToHost, s));

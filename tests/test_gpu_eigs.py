@@ -87,3 +87,23 @@ def test_eigs_on_degenerate_sectors(ed, orc):
     with pytest.raises(Exception):
         spectra.eigs_lowest(one, 1)
     one.close()
+
+
+@pytest.mark.parametrize("N,qu,qd,nev,ncv", [(7, 3, 2, 1, 3), (7, 3, 2, 3, 16), (7, 3, 4, 4, 17), (7, 2, 2, 2, 33), (9, 4, 3, 5, 24)])
+def test_eigs_dot_groups(ed, orc, N, qu, qd, nev, ncv):
+    """Subspaces below, at and above the sixteen dots a thread sums at a time,
+    on odd and even row counts (pairs with a missing element), with restarts:
+    eigenvalues against dense diagonalisation, eigenvectors orthonormal to the
+    rounding of sums of a thousand terms (1e-12)."""
+    from conftest import philox_uniform
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L, spectra
+    t = L.chain(N, periodic=False, eps=list(philox_uniform(40 + N, N, 1.5)))
+    op = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 2.0)
+    w, v, r = spectra.eigs_lowest(op, nev, ncv=ncv)
+    wd = np.linalg.eigvalsh(orc.hamiltonian(N, qu, qd, t, t, 2.0).toarray())
+    assert np.min(np.diff(wd[: nev + 1])) > 1e-6
+    assert np.max(np.abs(w - wd[:nev])) < 1e-10 * np.max(np.abs(wd[:nev]))
+    assert np.max(np.abs(v @ v.T - np.eye(nev))) < 1e-12
+    for k in range(nev):
+        assert np.linalg.norm(op.matvec(v[k]) - w[k] * v[k]) < 1e-8
+    op.close()
