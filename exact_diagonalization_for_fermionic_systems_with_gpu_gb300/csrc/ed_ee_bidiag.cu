@@ -45,8 +45,19 @@ struct EeJob {
     int64_t de;   // d at dd + de (n values), e at ee + de (n - 1 values)
 };
 
-// dynamic shared memory (doubles) of a CTA holding R rows of an n-column block
-size_t bd_smem_doubles(int R, int n) { return (size_t)R * n + 5 * (size_t)n + 2 + R + 2; }
+// Rows are summed in kBdGroups fixed groups combined in a binary tree, whatever
+// the cluster size, so that a block's result does not depend on how many CTAs
+// it got (and a state's not on the batch it came in).
+constexpr int kBdGroups = 32;
+constexpr int kBdChunk = 8;  // rows of an update unit
+
+int bd_group_rows(int m) { return (m + kBdGroups - 1) / kBdGroups; }
+
+// dynamic shared memory (doubles) of a CTA holding G groups of an m x n block
+size_t bd_smem_doubles(int m, int n, int G) {
+    const size_t R = (size_t)bd_group_rows(m) * G;
+    return R * n + (size_t)G * n + 5 * (size_t)n + 2 + R + 2;
+}
 
 // LAPACK dlarfg convention: H = I - tau v v^T, v_0 = 1, H [alpha; x] = [beta; 0]
 __device__ __forceinline__ void bd_reflector(double alpha, double xnorm2, double* beta, double* tau, double* scale) {
@@ -62,25 +73,40 @@ __device__ __forceinline__ void bd_reflector(double alpha, double xnorm2, double
     *scale = 1.0 / (alpha - b);
 }
 
+// part(g0) + ... + part(g0 + G - 1), neighbours first
+template <int G, typename F>
+__device__ __forceinline__ double tree_sum(int g0, const F& part) {
+    if constexpr (G == 1) return part(g0);
+    else return tree_sum<G / 2>(g0, part) + tree_sum<G / 2>(g0 + G / 2, part);
+}
+
+// The arithmetic (four multiply-adds an element and step) is bound by the FP64
+// pipe, which takes a warp instruction in 64 cycles on each of an SM's four
+// schedulers, so every phase deals equal units of (32 columns, a few rows) to
+// the 16 warps: with a thread per column, 5 warps of a 150-column step left
+// half the pipes idle, and a warp per row spent as much on its shuffle sums as
+// on the products.
+template <int CS>
 __global__ void __launch_bounds__(kBdThreads, 1) k_ee_bidiag(const EeJob* __restrict__ jobs,
                                                              const double* __restrict__ blocks,
                                                              double* __restrict__ dd, double* __restrict__ ee) {
     cg::cluster_group cl = cg::this_cluster();
-    const int CS = (int)cl.num_blocks();
+    constexpr int G = kBdGroups / CS;  // groups of this CTA
     const int rank = (int)cl.block_rank();
     const EeJob J = jobs[blockIdx.x / CS];
     const int m = J.m, n = J.n;
-    const int R = (m + CS - 1) / CS;
+    const int Rg = (m + kBdGroups - 1) / kBdGroups, R = Rg * G;
     const int r0 = min(m, rank * R), r1 = min(m, r0 + R);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     extern __shared__ double sm[];
     double* slab = sm;                    // own rows, row-major, stride n
-    double* part = slab + (size_t)R * n;  // [j] = sum over own rows i > k of A_ik A_ij, j >= k
+    double* pg = slab + (size_t)R * n;    // [g][j]: group g's part of the column sums
+    double* part = pg + (size_t)G * n;    // [j] = sum over own rows i > k of A_ik A_ij, j >= k
     double* rowk = part + n + 1;          // row k (columns >= k), written by its owner
-    double* wv = rowk + n;                // w_j of the left reflector
+    double* wv = rowk + n;                // tau w_j of the left reflector
     double* ubuf = wv + n;                // right reflector u_j (j > k), tau' at [n]
     double* uu = ubuf + n + 1;            // local copy of u
-    double* zz = uu + n;                  // v_i of the left reflector, then z_i of the right one
+    double* zz = uu + n;                  // v_i of the left reflector, then tau' z_i of the right one
     double* sc = zz + R;                  // tau, scale of the left reflector
     const double* src = blocks + J.off;
     for (int64_t idx = tid; idx < (int64_t)(r1 - r0) * n; idx += kBdThreads) {
@@ -88,25 +114,48 @@ __global__ void __launch_bounds__(kBdThreads, 1) k_ee_bidiag(const EeJob* __rest
         slab[(size_t)i * n + j] = src[(size_t)j * m + r0 + i];
     }
     __syncthreads();
+    // own rows ilo .. r1-1: A_ij -= z_i c_j for j >= j0
+    auto rank1 = [&](int ilo, int j0, const double* c) {
+        const int jb = (n - j0 + 31) / 32, nc = (r1 - ilo + kBdChunk - 1) / kBdChunk;
+        for (int u = warp; u < jb * nc; u += kBdWarps) {
+            const int q = u / jb, j = j0 + (u - q * jb) * 32 + lane;
+            if (j >= n) continue;
+            const double cj = -c[j];
+            const int i0 = ilo + q * kBdChunk, i1 = min(r1, i0 + kBdChunk);
+            double* a = slab + (size_t)(i0 - r0) * n + j;
+            for (int i = i0; i < i1; ++i, a += n) *a = fma(cj, zz[i - r0], *a);
+        }
+    };
     for (int k = 0; k < n; ++k) {
         const int owner = k / R;
         const int ilo = max(r0, k + 1);
-        // (1) partials over own rows below k; part[k] is the column's sigma'
-        for (int j = k + tid; j < n; j += kBdThreads) {
-            double w = 0.0;
-            for (int i = ilo; i < r1; ++i) w = fma(slab[(size_t)(i - r0) * n + k], slab[(size_t)(i - r0) * n + j], w);
-            part[j] = w;
+        // (1) partials over own rows below k, group by group; part[k] is the
+        // column's sigma'
+        {
+            const int jb = (n - k + 31) / 32;
+            for (int u = warp; u < jb * G; u += kBdWarps) {
+                const int g = u / jb, j = k + (u - g * jb) * 32 + lane;
+                if (j >= n) continue;
+                const int ib = max(ilo, r0 + g * Rg), ie = min(r1, r0 + (g + 1) * Rg);
+                const double* a = slab + (size_t)(ib - r0) * n;
+                double w = 0.0;
+                for (int i = ib; i < ie; ++i, a += n) w = fma(a[k], a[j], w);
+                pg[(size_t)g * n + j] = w;
+            }
+            __syncthreads();
+            for (int j = k + tid; j < n; j += kBdThreads)
+                part[j] = tree_sum<G>(0, [&](int g) { return pg[(size_t)g * n + j]; });
         }
         if (rank == owner)
             for (int j = k + tid; j < n; j += kBdThreads) rowk[j] = slab[(size_t)(k - r0) * n + j];
         cl.sync();  // A: partials and row k visible cluster-wide
         const double* rk = cl.map_shared_rank(rowk, owner);
-        // (2) one warp forms the left reflector (a fixed shuffle tree over the
-        // ranks, the same in every CTA)
+        // (2) one warp forms the left reflector (the same tree over the ranks in
+        // every CTA)
         if (warp == 0) {
             double sg = lane < CS ? cl.map_shared_rank(part, lane)[k] : 0.0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sg += __shfl_xor_sync(0xffffffffu, sg, o);
+            for (int o = 1; o < CS; o <<= 1) sg += __shfl_xor_sync(0xffffffffu, sg, o);
             if (lane == 0) {
                 double beta, tau, scale;
                 bd_reflector(rk[k], sg, &beta, &tau, &scale);
@@ -118,23 +167,15 @@ __global__ void __launch_bounds__(kBdThreads, 1) k_ee_bidiag(const EeJob* __rest
         __syncthreads();
         const double tau = sc[0], scale = sc[1];
         for (int j = k + 1 + tid; j < n; j += kBdThreads) {
-            double w = 0.0;
-#pragma unroll 4
-            for (int r = 0; r < CS; ++r) w += cl.map_shared_rank(part, r)[j];
-            wv[j] = fma(scale, w, rk[j]);
+            const double w = tree_sum<CS>(0, [&](int r) { return cl.map_shared_rank(part, r)[j]; });
+            wv[j] = tau * fma(scale, w, rk[j]);
         }
         const int il = max(r0, k);
         for (int i = il + tid; i < r1; i += kBdThreads)
             zz[i - r0] = (i == k) ? 1.0 : slab[(size_t)(i - r0) * n + k] * scale;
         __syncthreads();
         // (3) left update of own rows i >= k: A_ij -= tau v_i w_j
-        if (tau != 0.0) {
-            for (int j = k + 1 + tid; j < n; j += kBdThreads) {
-                const double tw = tau * wv[j];
-                for (int i = il; i < r1; ++i)
-                    slab[(size_t)(i - r0) * n + j] = fma(-tw, zz[i - r0], slab[(size_t)(i - r0) * n + j]);
-            }
-        }
+        if (tau != 0.0) rank1(il, k + 1, wv);
         __syncthreads();
         if (k + 1 >= n) break;
         // (4) one warp of the owner of row k forms the right reflector of A[k, k+1:]
@@ -154,58 +195,57 @@ __global__ void __launch_bounds__(kBdThreads, 1) k_ee_bidiag(const EeJob* __rest
             }
         }
         cl.sync();  // B: the right reflector visible cluster-wide
-        // (5) right update of own rows below k: z_i = A[i, k+1:] u, A -= tau' z u^T
+        // (5) right update of own rows below k: z_i = tau' A[i, k+1:] u, A -= z u^T
         const double* ur = cl.map_shared_rank(ubuf, owner);
         const double tau2 = ur[n];
         for (int j = k + 1 + tid; j < n; j += kBdThreads) uu[j] = ur[j];
         __syncthreads();
         if (tau2 != 0.0) {
-            for (int i = ilo + warp; i < r1; i += kBdWarps) {
-                const double* ai = slab + (size_t)(i - r0) * n;
+            // eight lanes a row, four rows a warp
+            const int sub = lane >> 3, l8 = lane & 7;
+            for (int i0 = ilo + 4 * warp; i0 < r1; i0 += 4 * kBdWarps) {
+                const int i = i0 + sub;
+                const double* ai = slab + (size_t)(min(i, r1 - 1) - r0) * n;
                 double z = 0.0;
-                for (int j = k + 1 + lane; j < n; j += 32) z = fma(ai[j], uu[j], z);
+                for (int j = k + 1 + l8; j < n; j += 8) z = fma(ai[j], uu[j], z);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-                if (lane == 0) zz[i - r0] = z;
+                for (int o = 1; o < 8; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                if (l8 == 0 && i < r1) zz[i - r0] = tau2 * z;
             }
             __syncthreads();
-            for (int j = k + 1 + tid; j < n; j += kBdThreads) {
-                const double tu = tau2 * uu[j];
-                for (int i = ilo; i < r1; ++i)
-                    slab[(size_t)(i - r0) * n + j] = fma(-tu, zz[i - r0], slab[(size_t)(i - r0) * n + j]);
-            }
+            rank1(ilo, k + 1, uu);
         }
         __syncthreads();
     }
     cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// Launch one cluster of cs CTAs per job; false when this device cannot run it.
-bool launch_bidiag(const std::vector<EeJob>& jobs, int cs, const double* blocks, double* dd, double* ee,
-                   cudaStream_t s, EeJob* djobs, size_t smem_bytes) {
+// Launch one cluster of CS CTAs per job; false when this device cannot run it.
+template <int CS>
+bool launch_bidiag(const std::vector<EeJob>& jobs, const double* blocks, double* dd, double* ee, cudaStream_t s,
+                   EeJob* djobs, size_t smem_bytes) {
     if (jobs.empty()) return true;
-    if (cudaFuncSetAttribute(k_ee_bidiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess)
-        return false;
-    if (cs > 8 && cudaFuncSetAttribute(k_ee_bidiag, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return false;
+    const auto fn = k_ee_bidiag<CS>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess) return false;
+    if (CS > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(jobs.size() * cs), 1, 1);
+    lc.gridDim = dim3((unsigned)(jobs.size() * CS), 1, 1);
     lc.blockDim = dim3(kBdThreads, 1, 1);
     lc.dynamicSmemBytes = smem_bytes;
     lc.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.x = CS;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, k_ee_bidiag, &lc) != cudaSuccess || nclusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &lc) != cudaSuccess || nclusters < 1) {
         cudaGetLastError();
         return false;
     }
-    if (cudaLaunchKernelEx(&lc, k_ee_bidiag, (const EeJob*)djobs, blocks, dd, ee) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&lc, fn, (const EeJob*)djobs, blocks, dd, ee) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -228,11 +268,33 @@ cudaStream_t bd_stream(int device, int i) {
     return st[device][i];
 }
 
+// Cluster size (log2) of an m x n block that is `share` times the largest one's
+// work when that gets `top` CTAs: in proportion to the work, and large enough
+// for the rows to fit the CTAs' shared memory (kBdSizes: it fits none).
+constexpr int kBdSizes = 5;  // cluster sizes 1, 2, 4, 8, 16
+
+static int bd_cluster(int m, int n, double share, int top, size_t cap) {
+    int g = 0;
+    while (g < kBdSizes - 1 && (double)(1 << g) < top * share) ++g;
+    while (g < kBdSizes && bd_smem_doubles(m, n, kBdGroups >> g) > cap) ++g;
+    return g;
+}
+
+// Time of a block on 2^g CTAs: 7.5 us of barriers and scalar code a step and
+// 2.4e9 multiply-adds/s a CTA (300 x 300 on 16, 8 and 4 CTAs: 3.32, 3.98, 5.83 ms).
+static double bd_seconds(int m, int n, int g) {
+    const double fma = 2.0 * n * n * ((double)m - n / 3.0);
+    return 7.5e-6 * n + fma / (2.4e9 * (1 << g));
+}
+
 // Singular values of the blocks that fit the cluster kernel: handled[k] = 1
 // and their values (descending) in sv_host[svo[k] ..).  The others are left
-// for the cuSOLVER path.  Cluster size per block in proportion to its work
-// (m n^2), the largest block on 16 CTAs, so that all clusters run in one
-// wave and finish together; one launch per cluster size, on its own stream.
+// for the cuSOLVER path.  Cluster size per block in proportion to its work.
+// The largest block's is the one with the smallest estimate: a state by itself
+// leaves SMs idle, so 16 CTAs end soonest ((7,5) of 12 sites: 3.3 ms, 5.8 ms
+// on 4), while the blocks of a batch fill the GPU and wider clusters only add
+// waiting (eight states: 14.7 ms on 16, 6.3 ms on 4).  One launch per cluster
+// size, on its own stream.
 ed_status ee_bidiag_blocks(int device, cudaStream_t s, const double* blocks, const std::vector<int64_t>& off,
                            const std::vector<int>& mm, const std::vector<int>& nn, const std::vector<int64_t>& svo,
                            std::vector<double>* sv_host, std::vector<char>* handled) {
@@ -244,21 +306,40 @@ ed_status ee_bidiag_blocks(int device, cudaStream_t s, const double* blocks, con
     const size_t cap = (size_t)max_smem / sizeof(double);
     double wmax = 0.0;
     for (size_t k = 0; k < off.size(); ++k) wmax = std::max(wmax, (double)mm[k] * nn[k] * nn[k]);
-    constexpr int kSizes = 5;  // cluster sizes 1, 2, 4, 8, 16
+    auto cluster = [&](size_t k, int top) {
+        return bd_cluster(mm[k], nn[k], (double)mm[k] * nn[k] * nn[k] / wmax, top, cap);
+    };
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    int top = 16;
+    double best = 1e300;
+    for (int t = 16; t >= 1; t /= 2) {
+        double longest = 0.0, area = 0.0;
+        for (size_t k = 0; k < off.size(); ++k) {
+            const int g = nn[k] > 0 ? cluster(k, t) : kBdSizes;
+            if (g >= kBdSizes) continue;
+            const double sec = bd_seconds(mm[k], nn[k], g);
+            longest = std::max(longest, sec);
+            area += sec * (1 << g);
+        }
+        const double est = std::max(longest, area / sms);
+        if (est < best) {
+            best = est;
+            top = t;
+        }
+    }
+    constexpr int kSizes = kBdSizes;
     std::vector<EeJob> group[kSizes];
-    size_t smem[kSizes] = {0, 0, 0, 0, 0};
+    size_t smem[kSizes] = {};
     std::vector<int> tag(off.size(), -1);
     for (size_t k = 0; k < off.size(); ++k) {
         const int m = mm[k], n = nn[k];
         if (n <= 0) { (*handled)[k] = 1; continue; }
-        const double want = 16.0 * (double)m * n * n / wmax;
-        int g = 0;
-        while (g < kSizes - 1 && (double)(1 << g) < want) ++g;
-        while (g < kSizes && bd_smem_doubles((m + (1 << g) - 1) >> g, n) > cap) ++g;
+        const int g = cluster(k, top);
         if (g >= kSizes) continue;  // too large for a cluster: cuSOLVER
         tag[k] = g;
         group[g].push_back(EeJob{off[k], m, n, svo[k]});
-        smem[g] = std::max(smem[g], bd_smem_doubles((m + (1 << g) - 1) >> g, n));
+        smem[g] = std::max(smem[g], bd_smem_doubles(m, n, kBdGroups >> g));
     }
     size_t njobs = 0;
     for (int g = 0; g < kSizes; ++g) njobs += group[g].size();
@@ -296,7 +377,15 @@ ed_status ee_bidiag_blocks(int device, cudaStream_t s, const double* blocks, con
             st = ED_ERR_CUDA;
             break;
         }
-        ok[g] = launch_bidiag(group[g], 1 << g, blocks, dd, ee, gs, djobs + first[g], smem[g] * sizeof(double));
+        const size_t bytes = smem[g] * sizeof(double);
+        EeJob* const dj = djobs + first[g];
+        switch (g) {
+            case 0: ok[g] = launch_bidiag<1>(group[g], blocks, dd, ee, gs, dj, bytes); break;
+            case 1: ok[g] = launch_bidiag<2>(group[g], blocks, dd, ee, gs, dj, bytes); break;
+            case 2: ok[g] = launch_bidiag<4>(group[g], blocks, dd, ee, gs, dj, bytes); break;
+            case 3: ok[g] = launch_bidiag<8>(group[g], blocks, dd, ee, gs, dj, bytes); break;
+            default: ok[g] = launch_bidiag<16>(group[g], blocks, dd, ee, gs, dj, bytes); break;
+        }
         cudaEventRecord(ev, gs);
         cudaStreamWaitEvent(s, ev, 0);
         done_ev.push_back(ev);

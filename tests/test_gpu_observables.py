@@ -356,3 +356,26 @@ def test_entropy_gesvd_pool_is_repeatable(ed, monkeypatch):
         assert ob.entanglement_entropy(op, psi, a_sites) == first
     assert abs(first[0] - ref[0]) < 1e-10 and abs(first[1] - ref[1]) < 1e-10 * max(1.0, ref[1])
     op.close()
+
+
+@pytest.mark.parametrize("N,qu,qd,a", [(12, 7, 5, 6), (12, 8, 4, 6), (11, 5, 4, 5), (9, 4, 4, 2), (8, 1, 7, 3), (6, 3, 3, 1)])
+def test_entropy_independent_of_cluster_size(ed, monkeypatch, N, qu, qd, a):
+    """The entropies of a state by itself (few wide clusters) and inside
+    batches of 3 and 9 (more, narrower ones) are the same bits, blocks of
+    fewer rows than row groups and of one column among them; and they agree
+    with gesvd's to the entropies' 1e-8."""
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L, observables as ob
+    t = L.chain(N, periodic=False)
+    op = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 1.0)
+    psi = torch.randn((9, op.rows()), dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    psi /= torch.linalg.vector_norm(psi, dim=1, keepdim=True)
+    nine = ob.entanglement_entropy_batch(op, psi, range(a))
+    three = ob.entanglement_entropy_batch(op, psi[:3], range(a))
+    one = [ob.entanglement_entropy(op, psi[b], range(a)) for b in range(3)]
+    for b in range(3):
+        assert one[b] == (three[0][b], three[1][b]) == (nine[0][b], nine[1][b])
+    monkeypatch.setenv("ED_EE_METHOD", "gesvd")
+    ref = ob.entanglement_entropy(op, psi[0], range(a))
+    assert abs(one[0][0] - ref[0]) < 1e-8 and abs(one[0][1] - ref[1]) < 1e-8
+    op.close()
