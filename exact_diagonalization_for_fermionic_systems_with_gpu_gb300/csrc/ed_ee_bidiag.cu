@@ -19,7 +19,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -404,27 +403,35 @@ ed_status ee_bidiag_blocks(int device, cudaStream_t s, const double* blocks, con
     for (size_t k = 0; k < off.size(); ++k)
         if (tag[k] >= 0 && ok[tag[k]]) todo.push_back((int)k);
     std::stable_sort(todo.begin(), todo.end(), [&](int a, int b) { return nn[a] > nn[b]; });
-    std::vector<char> fail(off.size(), 0);
+    std::vector<char> ok_sv(off.size(), 0);
     const int nth = std::max(1, std::min<int>((int)todo.size(), (int)std::thread::hardware_concurrency()));
-    std::vector<std::thread> th;
-    std::atomic<int> next(0);
-    auto work = [&]() {
-        for (;;) {
-            const int t = next.fetch_add(1);
-            if (t >= (int)todo.size()) return;
+    // dealt in turn, largest first; a thread sweeps several of its matrices at a time
+    auto work = [&](int t0) {
+        std::vector<int> mine, n;
+        std::vector<double*> d, e;
+        for (size_t t = t0; t < todo.size(); t += nth) {
             const int k = todo[t];
-            double* d = hd.data() + svo[k];
-            double* e = he.data() + svo[k];
-            if (!bidiag_singular_values(nn[k], d, e)) { fail[k] = 1; continue; }
-            std::sort(d, d + nn[k], [](double x, double y) { return x > y; });
-            std::copy(d, d + nn[k], sv_host->data() + svo[k]);
+            mine.push_back(k);
+            n.push_back(nn[k]);
+            d.push_back(hd.data() + svo[k]);
+            e.push_back(he.data() + svo[k]);
+        }
+        std::vector<char> good(mine.size(), 0);
+        bidiag_singular_values_many((int)mine.size(), n.data(), d.data(), e.data(), good.data());
+        for (size_t i = 0; i < mine.size(); ++i) {
+            const int k = mine[i];
+            ok_sv[k] = good[i];
+            if (!good[i]) continue;
+            std::sort(d[i], d[i] + n[i], [](double x, double y) { return x > y; });
+            std::copy(d[i], d[i] + n[i], sv_host->data() + svo[k]);
         }
     };
-    for (int i = 1; i < nth; ++i) th.emplace_back(work);
-    work();
+    std::vector<std::thread> th;
+    for (int i = 1; i < nth; ++i) th.emplace_back(work, i);
+    work(0);
     for (std::thread& t : th) t.join();
     for (int k : todo)
-        if (!fail[k]) (*handled)[k] = 1;
+        if (ok_sv[k]) (*handled)[k] = 1;
     return ED_OK;
 }
 

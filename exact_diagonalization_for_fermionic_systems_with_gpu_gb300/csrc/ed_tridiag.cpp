@@ -216,27 +216,39 @@ void tri_apply_z(const std::vector<TriRot>& rots, double* v) {
     }
 }
 
+// All times together: a row of V holds one component of the real and imaginary
+// parts at every time, so a rotation is read once and turns two contiguous rows
+// (vector instructions) instead of chaining through one vector per time.
 bool tridiag_expm_e0(int n, const double* a, const double* off, int n_times, const double* times, double* out) {
     std::vector<double> m;
     std::vector<TriRot> rots;
     if (!tridiag_eigen_rotations(n, a, off, &m, &rots)) return false;
-    std::vector<double> y(n, 0.0), re(n), im(n);
+    std::vector<double> y(n, 0.0);
     y[0] = 1.0;
     tri_apply_zt(rots, y.data());
-    for (int t = 0; t < n_times; ++t) {
-        for (int j = 0; j < n; ++j) {
+    const int cols = 2 * n_times;
+    std::vector<double> V((size_t)n * cols);
+    for (int j = 0; j < n; ++j)
+        for (int t = 0; t < n_times; ++t) {
             const double ph = m[j] * times[t];
-            re[j] = std::cos(ph) * y[j];
-            im[j] = -std::sin(ph) * y[j];
+            V[(size_t)j * cols + 2 * t] = std::cos(ph) * y[j];
+            V[(size_t)j * cols + 2 * t + 1] = -std::sin(ph) * y[j];
         }
-        tri_apply_z(rots, re.data());
-        tri_apply_z(rots, im.data());
-        double* o = out + (size_t)2 * n * t;
-        for (int k = 0; k < n; ++k) {
-            o[2 * k] = re[k];
-            o[2 * k + 1] = im[k];
+    for (auto it = rots.rbegin(); it != rots.rend(); ++it) {
+        const double c = it->c, s = it->s;
+        double* __restrict__ u = V.data() + (size_t)it->k * cols;
+        double* __restrict__ w = u + cols;
+        for (int q = 0; q < cols; ++q) {
+            const double x = u[q], z = w[q];
+            u[q] = c * x + s * z;
+            w[q] = -s * x + c * z;
         }
     }
+    for (int t = 0; t < n_times; ++t)
+        for (int k = 0; k < n; ++k) {
+            out[(size_t)2 * n * t + 2 * k] = V[(size_t)k * cols + 2 * t];
+            out[(size_t)2 * n * t + 2 * k + 1] = V[(size_t)k * cols + 2 * t + 1];
+        }
     return true;
 }
 
@@ -249,111 +261,176 @@ namespace ed {
 // which costs nothing at the eps |B| accuracy sought).
 inline double rot_norm(double a, double b) { return std::sqrt(a * a + b * b); }
 
-// Singular values of an upper bidiagonal B (d[0..n-1] diagonal, e[0..n-2]
-// superdiagonal; both overwritten, |values| left in d): the Golub-Kahan SVD
-// step with a Wilkinson shift from the trailing 2x2 of B^T B (Golub & Van
-// Loan, Matrix Computations, 4th ed., Algorithms 8.6.1-8.6.2).  A
+// One upper bidiagonal B (d[0..n-1] diagonal, e[0..n-2] superdiagonal; both
+// overwritten, |values| left in d) on its way to its singular values: the
+// Golub-Kahan SVD step with a Wilkinson shift from the trailing 2x2 of B^T B
+// (Golub & Van Loan, Matrix Computations, 4th ed., Algorithms 8.6.1-8.6.2).  A
 // superdiagonal entry deflates when |e_i| <= eps |B|; a diagonal entry with
 // |d_k| <= eps |B| is set to zero and its row is cleared by rotations from the
 // left, which moves the entry along the row until it leaves the block.
 // Absolute accuracy eps |B|, as LAPACK's gesvd gives after a Householder
-// bidiagonalisation.  False when 60 n sweeps did not converge.
-bool bidiag_singular_values(int n, double* d, double* e) {
-    if (n <= 0) return true;
-    const double eps = std::numeric_limits<double>::epsilon();
-    double bnorm = 0.0;
-    for (int i = 0; i < n; ++i) bnorm = std::max(bnorm, std::fabs(d[i]) + (i + 1 < n ? std::fabs(e[i]) : 0.0));
-    if (bnorm == 0.0) return true;
-    const double tol = eps * bnorm;
-    int q = n - 1;  // bottom of the active block
-    long long iters = 0;
-    const long long max_iters = 60LL * n;
-    while (q > 0) {
-        if (std::fabs(e[q - 1]) <= tol) {
-            e[q - 1] = 0.0;
-            --q;
-            continue;
-        }
-        int p = q - 1;
-        while (p > 0 && std::fabs(e[p - 1]) > tol) --p;
-        if (++iters > max_iters) return false;
-        // a (near-)zero diagonal entry in [p, q): clear its row
-        int z = -1;
-        for (int k = p; k < q; ++k)
-            if (std::fabs(d[k]) <= tol) { z = k; break; }
-        if (z >= 0) {
-            d[z] = 0.0;
-            double f = e[z];
-            e[z] = 0.0;
-            for (int j = z + 1; j <= q && f != 0.0; ++j) {
-                // rotate rows (z, j) so that the entry f in row z, column j
-                // goes to zero against d[j]
-                const double r = rot_norm(d[j], f);
-                const double ir = 1.0 / r;
-                const double c = d[j] * ir, s = f * ir;
-                d[j] = r;
-                if (j < q) {
-                    f = -s * e[j];
-                    e[j] = c * e[j];
-                }
-            }
-            continue;
-        }
-        if (std::fabs(d[q]) <= tol) {  // zero at the bottom: clear its column
-            d[q] = 0.0;
-            double f = e[q - 1];
-            e[q - 1] = 0.0;
-            for (int j = q - 1; j >= p && f != 0.0; --j) {
-                const double r = rot_norm(d[j], f);
-                const double ir = 1.0 / r;
-                const double c = d[j] * ir, s = f * ir;
-                d[j] = r;
-                if (j > p) {
-                    f = -s * e[j - 1];
-                    e[j - 1] = c * e[j - 1];
-                }
-            }
-            continue;
-        }
-        // Wilkinson shift: eigenvalue of the trailing 2x2 of B^T B nearer its last entry
-        const double dm = d[q - 1], em = e[q - 1], dq = d[q];
-        const double el = q - 1 > p ? e[q - 2] : 0.0;
-        const double t11 = dm * dm + el * el, t12 = dm * em, t22 = dq * dq + em * em;
-        const double h = 0.5 * (t11 - t22);
-        const double den = h + (h >= 0.0 ? 1.0 : -1.0) * rot_norm(h, t12);
-        const double mu = den != 0.0 ? t22 - t12 * t12 / den : t22;
-        double y = d[p] * d[p] - mu, zz = d[p] * e[p];
-        for (int k = p; k < q; ++k) {
-            // right rotation on columns (k, k+1): zero zz against y
-            double r = rot_norm(y, zz);
-            double ir = r != 0.0 ? 1.0 / r : 0.0;
-            double c = r != 0.0 ? y * ir : 1.0, s = -zz * ir;
-            if (k > p) e[k - 1] = r;
-            // [d_k e_k; 0 d_{k+1}] * [[c, s], [-s, c]] (the bulge below the diagonal)
-            const double dk = d[k], ek = e[k], dk1 = d[k + 1];
-            double a11 = c * dk - s * ek;
-            double a12 = s * dk + c * ek;
-            double a21 = -s * dk1;
-            double a22 = c * dk1;
-            // left rotation on rows (k, k+1): zero a21 against a11
-            r = rot_norm(a11, a21);
-            ir = r != 0.0 ? 1.0 / r : 0.0;
-            c = r != 0.0 ? a11 * ir : 1.0;
-            s = -a21 * ir;
-            d[k] = r;
-            // rows: [c -s; s c] * [[a11 a12 0], [a21 a22 e_{k+1}]]
-            e[k] = c * a12 - s * a22;
-            d[k + 1] = s * a12 + c * a22;
-            if (k + 1 < q) {
-                const double ek1 = e[k + 1];
-                y = e[k];
-                zz = -s * ek1;      // bulge at (k, k+2)
-                e[k + 1] = c * ek1;
-            }
-        }
+// bidiagonalisation.  60 n sweeps at most.
+struct BidiagLane {
+    double *d, *e;
+    int n, q, k;       // bottom of the active block; the sweep's next column
+    double tol, y, zz;  // the sweep's bulge
+    long long iters;
+
+    void start(int n_, double* d_, double* e_) {
+        d = d_;
+        e = e_;
+        n = n_;
+        q = n - 1;
+        k = q;
+        iters = 0;
+        double bnorm = 0.0;
+        for (int i = 0; i < n; ++i) bnorm = std::max(bnorm, std::fabs(d[i]) + (i + 1 < n ? std::fabs(e[i]) : 0.0));
+        tol = std::numeric_limits<double>::epsilon() * bnorm;
+        if (bnorm == 0.0) q = 0;
     }
-    for (int i = 0; i < n; ++i) d[i] = std::fabs(d[i]);
-    return true;
+
+    // Deflates until a sweep is due and starts it (1), or every value has
+    // settled (0), or the sweeps ran out (-1).
+    int prepare() {
+        while (q > 0) {
+            if (std::fabs(e[q - 1]) <= tol) {
+                e[q - 1] = 0.0;
+                --q;
+                continue;
+            }
+            int p = q - 1;
+            while (p > 0 && std::fabs(e[p - 1]) > tol) --p;
+            if (++iters > 60LL * n) return -1;
+            // a (near-)zero diagonal entry in [p, q): clear its row
+            int z = -1;
+            for (int i = p; i < q; ++i)
+                if (std::fabs(d[i]) <= tol) { z = i; break; }
+            if (z >= 0) {
+                d[z] = 0.0;
+                double f = e[z];
+                e[z] = 0.0;
+                for (int j = z + 1; j <= q && f != 0.0; ++j) {
+                    // rotate rows (z, j) so that the entry f in row z, column j
+                    // goes to zero against d[j]
+                    const double r = rot_norm(d[j], f);
+                    const double ir = 1.0 / r;
+                    const double c = d[j] * ir, s = f * ir;
+                    d[j] = r;
+                    if (j < q) {
+                        f = -s * e[j];
+                        e[j] = c * e[j];
+                    }
+                }
+                continue;
+            }
+            if (std::fabs(d[q]) <= tol) {  // zero at the bottom: clear its column
+                d[q] = 0.0;
+                double f = e[q - 1];
+                e[q - 1] = 0.0;
+                for (int j = q - 1; j >= p && f != 0.0; --j) {
+                    const double r = rot_norm(d[j], f);
+                    const double ir = 1.0 / r;
+                    const double c = d[j] * ir, s = f * ir;
+                    d[j] = r;
+                    if (j > p) {
+                        f = -s * e[j - 1];
+                        e[j - 1] = c * e[j - 1];
+                    }
+                }
+                continue;
+            }
+            // Wilkinson shift: eigenvalue of the trailing 2x2 of B^T B nearer its last entry
+            const double dm = d[q - 1], em = e[q - 1], dq = d[q];
+            const double el = q - 1 > p ? e[q - 2] : 0.0;
+            const double t11 = dm * dm + el * el, t12 = dm * em, t22 = dq * dq + em * em;
+            const double h = 0.5 * (t11 - t22);
+            const double den = h + (h >= 0.0 ? 1.0 : -1.0) * rot_norm(h, t12);
+            const double mu = den != 0.0 ? t22 - t12 * t12 / den : t22;
+            y = d[p] * d[p] - mu;
+            zz = d[p] * e[p];
+            first = p;
+            k = p;
+            return 1;
+        }
+        for (int i = 0; i < n; ++i) d[i] = std::fabs(d[i]);
+        return 0;
+    }
+
+    // Column k of the sweep.
+    void step() {
+        // right rotation on columns (k, k+1): zero zz against y
+        double r = rot_norm(y, zz);
+        double ir = r != 0.0 ? 1.0 / r : 0.0;
+        double c = r != 0.0 ? y * ir : 1.0, s = -zz * ir;
+        if (k > first) e[k - 1] = r;
+        // [d_k e_k; 0 d_{k+1}] * [[c, s], [-s, c]] (the bulge below the diagonal)
+        const double dk = d[k], ek = e[k], dk1 = d[k + 1];
+        const double a11 = c * dk - s * ek, a12 = s * dk + c * ek, a21 = -s * dk1, a22 = c * dk1;
+        // left rotation on rows (k, k+1): zero a21 against a11
+        r = rot_norm(a11, a21);
+        ir = r != 0.0 ? 1.0 / r : 0.0;
+        c = r != 0.0 ? a11 * ir : 1.0;
+        s = -a21 * ir;
+        d[k] = r;
+        // rows: [c -s; s c] * [[a11 a12 0], [a21 a22 e_{k+1}]]
+        e[k] = c * a12 - s * a22;
+        d[k + 1] = s * a12 + c * a22;
+        if (k + 1 < q) {
+            const double ek1 = e[k + 1];
+            y = e[k];
+            zz = -s * ek1;  // bulge at (k, k+2)
+            e[k + 1] = c * ek1;
+        }
+        ++k;
+    }
+
+    int first = 0;  // first column of the sweep
+};
+
+// A sweep is a chain of two square roots and two divisions a column, so the
+// core's dividers idle most of it; kBidiagLanes matrices are swept in turn,
+// column by column, and their chains overlap.  One loop body serves every lane
+// and any number of them: a matrix's values do not depend on its company.
+constexpr int kBidiagLanes = 4;
+
+void bidiag_singular_values_many(int count, const int* n, double* const* d, double* const* e, char* ok) {
+    BidiagLane lane[kBidiagLanes];
+    int item[kBidiagLanes], active = 0, next = 0;
+    for (;;) {
+        while (active < kBidiagLanes && next < count) {
+            if (n[next] <= 0) {
+                ok[next++] = 1;
+                continue;
+            }
+            lane[active].start(n[next], d[next], e[next]);
+            item[active++] = next++;
+        }
+        for (int w = 0; w < active;) {
+            // a lane between sweeps: its next one, or out
+            const int st = lane[w].k < lane[w].q ? 1 : lane[w].prepare();
+            if (st == 1) {
+                ++w;
+                continue;
+            }
+            ok[item[w]] = st == 0;
+            lane[w] = lane[--active];
+            item[w] = item[active];
+        }
+        if (active == 0) {
+            if (next >= count) return;
+            continue;
+        }
+        int len = lane[0].q - lane[0].k;
+        for (int w = 1; w < active; ++w) len = std::min(len, lane[w].q - lane[w].k);
+        for (int t = 0; t < len; ++t)
+            for (int w = 0; w < active; ++w) lane[w].step();
+    }
+}
+
+bool bidiag_singular_values(int n, double* d, double* e) {
+    char ok = 0;
+    bidiag_singular_values_many(1, &n, &d, &e, &ok);
+    return ok != 0;
 }
 
 }  // namespace ed

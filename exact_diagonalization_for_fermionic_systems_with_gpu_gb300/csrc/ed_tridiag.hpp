@@ -31,5 +31,8 @@ bool tridiag_expm_e0(int n, const double* a, const double* off, int n_times, con
 // Singular values of the upper bidiagonal (d, e) (both overwritten; the
 // values, unsorted and nonnegative, in d).  False when not converged.
 bool bidiag_singular_values(int n, double* d, double* e);
+// The same for `count` matrices, several at a time on the calling thread;
+// ok[i] as the return value above.
+void bidiag_singular_values_many(int count, const int* n, double* const* d, double* const* e, char* ok);
 
 }  // namespace ed
