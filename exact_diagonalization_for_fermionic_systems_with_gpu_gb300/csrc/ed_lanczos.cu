@@ -683,10 +683,11 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     // Steps run in the persistent kernel for real single-class operators
     // whose down table fits shared memory as a gather schedule, unless
     // reorthogonalisation or per-step timing asks for the per-step kernels.
-    // In the reference mode one launch runs every step while the host does
-    // the stop test every ten steps on the alpha and beta the kernel mirrors
-    // into mapped memory, and a host stop word ends the launch (a few steps
-    // after the test passes; T and the Ritz vector use the first n only).
+    // With a stop test (reference mode, or stop_beta) one launch runs every step
+    // while the host does the test every ten steps on the alpha and beta the
+    // kernel mirrors into mapped memory, and a host stop word ends the launch
+    // (a few steps after the test passes; T and the vectors use the first n
+    // only).
     // The tridiagonal eigensolve stays on the host: on this chip FP64 runs at
     // 1/64 of the FP32 rate, and one device thread's Sturm bisection of a
     // 300-step T takes milliseconds against ~0.1 ms on the host cores.  ED_LZ_FUSED=0 never uses it, ED_LZ_FUSED=1 also
@@ -707,10 +708,8 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     int j = 0;
     while (j < max_steps) {
         if (fused) {
-            const bool host_stop = cfg->mode == ED_LANCZOS_REFERENCE && stop_beta < 0.0 && j == 0;
-            const int j1 = (!host_stop && (cfg->mode == ED_LANCZOS_REFERENCE || stop_beta >= 0.0))
-                               ? std::min(max_steps, (j / 10 + 1) * 10)
-                               : max_steps;
+            const bool host_stop = cfg->mode == ED_LANCZOS_REFERENCE || stop_beta >= 0.0;
+            const int j1 = max_steps;
             LZ_CK(cudaMemsetAsync(w->gbar, 0, kFusedSync, s));
             if (host_stop) {
                 LZ_CK(ensure_mirror(w, max_steps));
@@ -749,18 +748,24 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
                 // the stop test at every tenth step as the kernel's mirror
                 // reaches it; the first test that passes stops the launch
                 int checked = 0;
-                bool ended = false;
+                bool ended = false, stopped = false;
                 for (;;) {
                     const int done = __atomic_load_n(&w->mirror_h->done, __ATOMIC_ACQUIRE);
-                    while (!converged && checked + 10 <= done && checked + 10 <= max_steps) {
+                    while (!stopped && checked + 10 <= done && checked + 10 <= max_steps) {
                         checked += 10;
-                        if (ref_test(checked, w->mirror_alpha, w->mirror_beta)) {
-                            converged = true;
+                        if (stop_beta >= 0.0) {
+                            for (int k = checked - 9; k <= checked; ++k)
+                                stopped = stopped || w->mirror_beta[k] == 0.0 ||  // breakdown
+                                          w->mirror_beta[k] < stop_beta * w->mirror_beta[0];
+                        } else {
+                            stopped = converged = ref_test(checked, w->mirror_alpha, w->mirror_beta);
+                        }
+                        if (stopped) {
                             n = checked;
                             __atomic_store_n(&w->mirror_h->stop, checked, __ATOMIC_RELEASE);
                         }
                     }
-                    if (converged || ended) break;
+                    if (stopped || ended) break;
                     const cudaError_t q = cudaStreamQuery(s);
                     if (q == cudaSuccess) {
                         ended = true;  // one more pass over the final count

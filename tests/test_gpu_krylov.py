@@ -177,3 +177,27 @@ def test_krylov_combine_time_groups(ed, orc, case, n_times):
     twice = ev.krylov_evolve(op, psi0, times, max_steps=37, out=got.copy())
     assert np.max(np.linalg.norm(twice - 2 * ref, axis=1)) < 2e-11 * nrm
     op.close()
+
+
+@pytest.mark.parametrize("steps", [1, 9, 10, 25])
+def test_krylov_one_launch_stops_like_per_step(ed, monkeypatch, steps):
+    """The Krylov run in one persistent launch with the stop test on the host
+    against the per-step kernels' test every ten steps: the same dimension and
+    the same bits, with and without a subspace that ends early (two sites: four
+    states; tol = 0 leaves only the breakdown)."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import evolution as ev, lattices as L
+    from conftest import philox_uniform
+    for N, q, tol in ((2, 1, 1e-10), (2, 1, 0.0), (7, 3, 1e-10), (7, 3, 0.9)):
+        t = L.chain(N, periodic=False, eps=list(philox_uniform(3, N, 1.0)))
+        op = ed.Hubbard(ed.H_TBq(N, q).extend(t), ed.H_TBq(N, q).extend(t), 2.0)
+        x = philox_uniform(23, 2 * op.rows())
+        psi0 = x[0::2] + 1j * x[1::2]
+        got = []
+        for form in ("1", "0"):
+            monkeypatch.setenv("ED_LZ_FUSED", form)
+            info = {}
+            got.append((ev.krylov_evolve(op, psi0, [0.2, 0.5], max_steps=steps, tol=tol, result=info), info["steps"]))
+        monkeypatch.delenv("ED_LZ_FUSED")
+        assert got[0][1] == got[1][1]
+        assert np.array_equal(got[0][0], got[1][0])
+        op.close()
