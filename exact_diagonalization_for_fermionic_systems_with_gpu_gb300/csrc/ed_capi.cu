@@ -556,6 +556,21 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         a.dnSegP = op->d_dnSegP;
         a.mergeMC = (a.nclsUP == a.nclsDN && tu.coef == td.coef) ? 1 : 0;
     }
+    // entries per (row, class) run of the two tables: below 2, a product per
+    // entry replaces the running class sums
+    {
+        int64_t runs = 0;
+        for (const ed::SpinTable* t : {&tu, &td})
+            for (int64_t r = 0; r < t->count; ++r) {
+                uint32_t last = ~0u;
+                for (int k = 0; k < t->len[r]; ++k) {
+                    const uint32_t c = (t->ent[(size_t)k * t->count + r] >> ed::kClassShift) & ed::kClassMask;
+                    runs += c != last;
+                    last = c;
+                }
+            }
+        a.perEntry = tu.nnz + td.nnz < 2 * runs ? 1 : 0;
+    }
     a.upPtr = op->d_upPtr;
     a.upEntC = op->d_upEntC;
     a.dnPtr = op->d_dnPtr;

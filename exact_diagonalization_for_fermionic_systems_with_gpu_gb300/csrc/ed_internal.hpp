@@ -81,6 +81,7 @@ struct MvArgs {
     const uint32_t* upSegP;
     const uint32_t* dnSegE;
     const uint32_t* dnSegP;
+    int perEntry;         // multi-class tables whose rows hold about one entry of a class: a product per entry
     int mergeMC;          // segmented tables with equal class lists: one product per class
     // coefficient classes, interleaved (re, im), scale 2^-Fc
     int64_t coefUP[2 * kMaxCls];

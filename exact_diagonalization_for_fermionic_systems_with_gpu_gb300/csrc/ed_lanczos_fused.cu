@@ -117,7 +117,10 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
     __shared__ SlotScalars sX, sP;  // slots j and j-1
     __shared__ int s_status, s_min_bits;
     __shared__ LzCoefs s_coef;
-    const TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    constexpr bool kGen = !FAST && !SEG;
+    __shared__ int64_t s_cls[kGen ? 4 * kMaxCls : 1];
+    TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    tma_stage_classes<kGen>(a, s_cls, S);
     LzState* lz = f.lz;
     const int tid = threadIdx.x;
     __shared__ uint32_t s_next;  // row-queue index taken by thread 0
@@ -741,7 +744,9 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_multi(const LzMultiArgs f
                 __syncthreads();
                 cur = b;
             }
-            const TmaSmem S = tma_view(s_args, sm, uoff, uent, &give_up);
+            TmaSmem S = tma_view(s_args, sm, uoff, uent, &give_up);
+            S.cup = s_args.coefUP;
+            S.cdn = s_args.coefDN;
             if (I.group != staged) {
                 if (tid == 0) {
                     tma::fence_proxy_async_smem();

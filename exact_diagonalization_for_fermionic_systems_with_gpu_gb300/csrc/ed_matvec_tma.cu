@@ -27,7 +27,10 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_matvec_tma(const MvArgs a) {
     __shared__ uint32_t uoff[kTmaUpStage];
     __shared__ uint32_t uent[kTmaUpStage];
     __shared__ int give_up;
-    const TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    constexpr bool kGen = !FAST && !SEG;
+    __shared__ int64_t s_cls[kGen ? 4 * kMaxCls : 1];
+    TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    tma_stage_classes<kGen>(a, s_cls, S);
     uint32_t u0 = 0;
     const bool has_row = tma_first_row(a, &u0);
     if (threadIdx.x == 0) {
@@ -77,7 +80,10 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const 
     __shared__ uint32_t uent[kTmaUpStage];
     __shared__ int give_up, s_emax, s_red[32];
     __shared__ uint32_t s_next;
-    const TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    constexpr bool kGen = !FAST && !SEG;
+    __shared__ int64_t s_cls[kGen ? 4 * kMaxCls : 1];
+    TmaSmem S = tma_view(a, sm, uoff, uent, &give_up);
+    tma_stage_classes<kGen>(a, s_cls, S);
     const int tid = threadIdx.x;
     const int64_t gt = (int64_t)blockIdx.x * kTmaThreads + tid, GT = (int64_t)gridDim.x * kTmaThreads;
     uint32_t u0 = 0;
@@ -211,7 +217,8 @@ int tma_plan(const ed_op* op, MvArgs* a) {
     off += up128(dimDN * 8);
     a->sm_stdn = (int)off;
     off += up128(dimDN * 8);
-    const int64_t static_bytes = 2 * kTmaUpStage * 4 + 64 + 24 * 64;  // uoff, uent, reduction scratch
+    // uoff, uent, reduction scratch; the general kernels' coefficient classes
+    const int64_t static_bytes = 2 * kTmaUpStage * 4 + 64 + 24 * 64 + (op->mv_fast || a->upSegE ? 0 : 4 * kMaxCls * 8);
     if (off + static_bytes > 227 * 1024) return 0;
     return (int)off;
 }

@@ -81,3 +81,45 @@ def test_one_launch_apply_in_a_graph(ed):
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(y.cpu().numpy(), op.matvec(v))
+
+
+@pytest.mark.parametrize("case", ["lieb_random", "kagome_random_flux", "kagome_random_odd", "few_classes", "one_up_hop"])
+def test_entry_products_match_generic(ed, monkeypatch, case):
+    """Tables with a coefficient per bond (a product per entry, in the apply,
+    the per-step, the persistent and the mixed batched kernels) and tables
+    whose rows hold several entries of a class (class sums), against the
+    generic kernel bit for bit."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    r = list(philox_uniform(14, 12, 0.5) + 1.0)
+    N, qu, qd, t = 12, 5, 4, L.lieb12(r)
+    if case == "kagome_random_flux":
+        qu, qd, t = 3, 4, L.kagome12(r, flux=0.4)
+    elif case == "kagome_random_odd":
+        qu, qd, t = 2, 8, L.kagome12(r)
+    elif case == "few_classes":  # five amplitudes on 24 bonds
+        t = [(k, i, j, v * (1.0 + 0.25 * (b % 5)), p) for b, (k, i, j, v, p) in enumerate(L.kagome12())]
+    elif case == "one_up_hop":
+        qu, qd = 12, 5
+    ops = {}
+    for kind in ("auto", "generic"):
+        if kind == "generic":
+            monkeypatch.setenv("ED_MATVEC", "generic")
+        ops[kind] = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 4.0)
+        monkeypatch.delenv("ED_MATVEC", raising=False)
+    n = ops["auto"].rows()
+    x = np.random.default_rng(8).standard_normal(n)
+    x = x + 1j * x[::-1] if ops["auto"].is_complex else x
+    assert np.array_equal(ops["auto"].matvec(x), ops["generic"].matvec(x))
+    runs = []
+    for kind, form in (("generic", "0"), ("auto", "0"), ("auto", "1")):
+        monkeypatch.setenv("ED_LZ_FUSED", form)
+        lz = ed.Lanczos()
+        e, v = lz.eigen(ops[kind], max_steps=25, mode="fixed", seed=6)
+        runs.append((e, lz.a, lz.b, v))
+    monkeypatch.delenv("ED_LZ_FUSED")
+    chain = ed.Hubbard(ed.H_TBq(8, 4).extend(L.chain(8)), ed.H_TBq(8, 4).extend(L.chain(8)), 1.0)
+    e, vs, al, be = ed.lanczos_multi([chain, ops["auto"]], 25, seed=5)  # run 1 from seed 6
+    runs.append((e[1], list(al[1]), list(be[1]), vs[1]))
+    for other in runs[1:]:
+        assert other[:3] == runs[0][:3]
+        assert np.array_equal(other[3], runs[0][3])
