@@ -680,9 +680,12 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
         return std::fabs(Bv[nn] * tri[nn]) < tolconv * anorm && std::fabs(tri[1]) > tolconv * anorm;
     };
 
-    // Steps run in the persistent kernel for real single-class operators
-    // whose down table fits shared memory as a gather schedule, unless
-    // reorthogonalisation or per-step timing asks for the per-step kernels.
+    // Steps run in the persistent kernel for every operator with a
+    // shared-memory plan, unless reorthogonalisation or per-step timing asks for
+    // the per-step kernels or ed_op_autotune chose them.  Us a step, per step and
+    // persistent: complex Kagome12 6+6 96 / 89, 4+4 45 / 36, 2+2 27 / 17;
+    // random-hopping Lieb12 6+6 68 / 57, 3+3 29 / 26; two classes on a 10-site
+    // ring 26 / 22; single-class operators gain most (Kagome12 49 / 38).
     // With a stop test (reference mode, or stop_beta) one launch runs every step
     // while the host does the test every ten steps on the alpha and beta the
     // kernel mirrors into mapped memory, and a host stop word ends the launch
@@ -690,15 +693,12 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     // only).
     // The tridiagonal eigensolve stays on the host: on this chip FP64 runs at
     // 1/64 of the FP32 rate, and one device thread's Sturm bisection of a
-    // 300-step T takes milliseconds against ~0.1 ms on the host cores.  ED_LZ_FUSED=0 never uses it, ED_LZ_FUSED=1 also
-    // for the other operators with a shared-memory plan (complex, several
-    // classes), where the per-step kernels measured faster.
+    // 300-step T takes milliseconds against ~0.1 ms on the host cores.
+    // ED_LZ_FUSED=0 never uses the persistent kernel, ED_LZ_FUSED=1 also where
+    // the autotuner chose the per-step ones.
     const char* fz = std::getenv("ED_LZ_FUSED");
     const bool force = fz && fz[0] == '1', never = fz && fz[0] == '0';
-    // ed_op_autotune's choice, when made, replaces the default rule
-    const bool rule = fz ? (force || op->mv.dnSched != nullptr)
-                         : (op->lz_mode == 2 || (op->lz_mode == 0 && op->mv.dnSched != nullptr));
-    bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && rule;
+    bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && (force || op->lz_mode != 1);
     // Reorthogonalised runs of small sectors: all steps in one cooperative
     // launch (ed_lanczos_reorth.cu).
     bool fused_reorth = cfg->reorth && !op->striped && !prof && !never && max_steps <= kReorthMaxSteps &&
