@@ -208,7 +208,8 @@ cudaError_t launch_to_fx(const double* x, int64_t n, const int* d_emax, int64_t*
 cudaError_t launch_matvec_f64(const ed_op* op, const int64_t* xq, const int* d_emax, double* y,
                               cudaStream_t s);
 // u = H x in FX with the Lanczos-step epilogue (dot and max partials).
-// d_mx: device pointer to max|xq| (the Krylov slot's m entry).
+// d_mx: device pointer to max|xq| (the Krylov slot's m entry).  step < 0: u
+// alone (a second pass).
 cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, void* lz,
                              const uint64_t* d_mx, int step, cudaStream_t s);
 int matvec_grid(const ed_op* op);
@@ -233,7 +234,7 @@ cudaError_t launch_apply(const ed_op* op, const double* x, double* y, int64_t* x
 int apply_grid(const ed_op* op);
 cudaError_t launch_apply_rows(const ed_op* op, const MvArgs& a, const ApplyArgs& f, cudaStream_t s);
 cudaError_t launch_striped_down(const ed_op* op, const StripedArgs& g, cudaStream_t s);
-cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, int out, cudaStream_t s);
+cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, cudaStream_t s);
 cudaError_t launch_permute_f64(const ed_op* op, const double* in, double* out, int forward, cudaStream_t s);
 cudaError_t launch_permute_i64(const ed_op* op, const int64_t* in, int64_t* out, int forward, cudaStream_t s);
 cudaError_t launch_to_fx_perm(const ed_op* op, const double* x, const int* d_emax, int64_t* xq, cudaStream_t s);

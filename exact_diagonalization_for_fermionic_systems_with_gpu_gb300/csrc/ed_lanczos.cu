@@ -324,16 +324,50 @@ __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__
     }
 }
 
-// Second-pass Ritz sum: acc (+)= (rt_k q_k >> rs_k) * 2^-F for the Lanczos
-// vector q_k just produced (first: acc is overwritten).
+// Second-pass Ritz sum, first term: acc = (rt_0 q_0 >> rs_0) * 2^-F.
 __global__ void __launch_bounds__(kLzThreads) k_ritz_acc(double* __restrict__ acc, const int64_t* __restrict__ q,
                                                          int64_t n, const int64_t* __restrict__ rt,
-                                                         const int* __restrict__ rs, int F, int k, int first) {
-    const int64_t c = rt[k];
-    const int r = rs[k];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double t = i128_to_f64(mul_wide(c, q[i]) >> r, -F);
-        acc[i] = first ? t : acc[i] + t;
+                                                         const int* __restrict__ rs, int F) {
+    const int64_t c = rt[0];
+    const int r = rs[0];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        acc[i] = i128_to_f64(mul_wide(c, q[i]) >> r, -F);
+}
+
+// A second-pass step: w_{k+1} = round((at0 u + at1 x + at2 p) / 2^Fa) with the
+// first pass's coefficients of step k, and acc += c_{k+1} w_{k+1} as in
+// k_ritz_acc.  The sums of w that the first pass took are known, and w is not
+// read back for the accumulation: 48 bytes an element in one kernel where the
+// axpy and k_ritz_acc moved 56 in two (Lieb18 4+9: 0.89 + 1.25 -> 1.64 ms, now
+// bound by the conversions to FP64).
+__global__ void __launch_bounds__(kLzThreads) k_lz_replay(const int64_t* __restrict__ uq, const int64_t* __restrict__ xq,
+                                                          const int64_t* __restrict__ pq, int64_t* __restrict__ wq,
+                                                          double* __restrict__ acc, int64_t n, const LzState* lz, int k,
+                                                          const int64_t* __restrict__ rt, const int* __restrict__ rs,
+                                                          int F) {
+    const int64_t a0 = lz->at_hist[3 * k], a1 = lz->at_hist[3 * k + 1], a2 = lz->at_hist[3 * k + 2];
+    const int Fa = lz->Fa_hist[k];
+    const int64_t c = rt[k + 1];
+    const int r = rs[k + 1];
+    auto step = [&](int64_t u, int64_t x, int64_t p) {
+        return shr_round_i64(mul_wide(a0, u) + mul_wide(a1, x) + mul_wide(a2, p), Fa);
+    };
+    const int64_t npair = n >> 1;
+    const longlong2* u2 = reinterpret_cast<const longlong2*>(uq);
+    const longlong2* x2 = reinterpret_cast<const longlong2*>(xq);
+    const longlong2* p2 = reinterpret_cast<const longlong2*>(pq);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npair; i += (int64_t)gridDim.x * blockDim.x) {
+        const longlong2 u = __ldg(u2 + i), x = __ldg(x2 + i), p = __ldg(p2 + i);
+        const double y0 = acc[2 * i], y1 = acc[2 * i + 1];  // a caller's vector: any 8-byte boundary
+        const longlong2 w = make_longlong2(step(u.x, x.x, p.x), step(u.y, x.y, p.y));
+        reinterpret_cast<longlong2*>(wq)[i] = w;
+        acc[2 * i] = y0 + i128_to_f64(mul_wide(c, w.x) >> r, -F);
+        acc[2 * i + 1] = y1 + i128_to_f64(mul_wide(c, w.y) >> r, -F);
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const int64_t w = step(uq[n - 1], xq[n - 1], pq[n - 1]);
+        wq[n - 1] = w;
+        acc[n - 1] += i128_to_f64(mul_wide(c, w) >> r, -F);
     }
 }
 
@@ -423,7 +457,7 @@ struct Workspace {
 
 void free_ws(Workspace* w) {
     cudaFree(w->basis); cudaFree(w->u); cudaFree(w->fbuf); cudaFree(w->lz);
-    cudaFree(w->h.e); cudaFree(w->h.m); cudaFree(w->h.beta); cudaFree(w->h.alpha);
+    cudaFree(w->h.e); cudaFree(w->h.m); cudaFree(w->h.beta); cudaFree(w->h.alpha); cudaFree(w->h.at_hist); cudaFree(w->h.Fa_hist);
     cudaFree(w->h.part_lo); cudaFree(w->h.part_hi); cudaFree(w->h.part_max); cudaFree(w->h.counter);
     cudaFree(w->emax); cudaFree(w->flag); 
     cudaFree(w->dot_lo); cudaFree(w->dot_hi); cudaFree(w->coef_rt); cudaFree(w->coef_rs); cudaFree(w->coef_F);
@@ -480,6 +514,8 @@ ed_status ensure_ws(ed_op* op, Workspace* w, size_t slots, int64_t DW, int max_s
     LZ_CK(cudaMalloc(&w->h.m, sizeof(uint64_t) * ns));
     LZ_CK(cudaMalloc(&w->h.beta, sizeof(double) * ns));
     LZ_CK(cudaMalloc(&w->h.alpha, sizeof(double) * ns));
+    LZ_CK(cudaMalloc(&w->h.at_hist, sizeof(int64_t) * 3 * ns));
+    LZ_CK(cudaMalloc(&w->h.Fa_hist, sizeof(int) * ns));
     LZ_CK(cudaMalloc(&w->h.part_lo, sizeof(uint64_t) * kLzMaxPartials));
     LZ_CK(cudaMalloc(&w->h.part_hi, sizeof(uint64_t) * kLzMaxPartials));
     LZ_CK(cudaMalloc(&w->h.part_max, sizeof(uint64_t) * kLzMaxPartials));
@@ -935,17 +971,15 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
         // the start vector in fbuf is consumed: fbuf can hold the sum
         double* out = evec_mem == ED_MEM_DEVICE ? evec : w->fbuf;
         const int g = lz_grid(DW);
-        k_ritz_acc<<<g, kLzThreads, 0, s>>>(out, slot(0), DW, w->coef_rt, w->coef_rs, F, 0, 1);
+        k_ritz_acc<<<g, kLzThreads, 0, s>>>(out, slot(0), DW, w->coef_rt, w->coef_rs, F);
         LZ_CK(cudaGetLastError());
         launches += 3;
         for (int k = 0; k + 1 < n; ++k) {
-            LZ_CK(launch_matvec_lz(op, slot(k), w->u, lz, w->fxbound, k, s));
+            LZ_CK(launch_matvec_lz(op, slot(k), w->u, lz, w->fxbound, -1, s));
             const int64_t* pk = k > 0 ? slot(k - 1) : slot(k);
-            k_lz_axpy<<<g, kLzThreads, 0, s>>>(w->u, slot(k), pk, slot(k + 1), DW, lz, k);
+            k_lz_replay<<<g, kLzThreads, 0, s>>>(w->u, slot(k), pk, slot(k + 1), out, DW, lz, k, w->coef_rt, w->coef_rs, F);
             LZ_CK(cudaGetLastError());
-            k_ritz_acc<<<g, kLzThreads, 0, s>>>(out, slot(k + 1), DW, w->coef_rt, w->coef_rs, F, k + 1, 0);
-            LZ_CK(cudaGetLastError());
-            launches += 3;
+            launches += 2;
         }
         k_inv_norm<<<g, kLzThreads, 0, s>>>(out, DW, w->ritz_part, w->ritz_ctr, w->inv_norm);
         LZ_CK(cudaGetLastError());

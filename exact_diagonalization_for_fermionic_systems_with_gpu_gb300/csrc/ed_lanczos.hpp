@@ -27,6 +27,8 @@ struct LzState {
     uint64_t* part_hi;
     uint64_t* part_max;
     unsigned int* counter;  // [4] last-block counters (matvec, axpy, start, misc)
+    int64_t* at_hist;  // [3 j + k]: step j's axpy coefficients, and their fraction bits,
+    int* Fa_hist;      // for the second pass, which repeats the steps without the sums
     // current step scalars
     int s_u;         // right shift applied to the exact matvec accumulator
     int e_u;         // exponent of u = H w_j

@@ -141,6 +141,17 @@ __device__ inline void reorth_fix(double r, int extra, int F, int64_t* t, int* s
     }
 }
 
+// Step j's coefficients into the run's state.
+__device__ inline void lz_store_coefs(LzState* lz, int j, const LzCoefs& c) {
+    lz->alpha[j] = c.alpha;
+    for (int k = 0; k < 3; ++k) {
+        lz->at[k] = lz->at_hist[3 * j + k] = c.at[k];
+        lz->sh[k] = 0;
+    }
+    lz->Fa = lz->Fa_hist[j] = c.Fa;
+    lz->e_w = c.e_w;
+}
+
 __device__ inline void lz_after_matvec(LzState* lz, int j, i128 alpha_raw, uint64_t m_u, int s_u, int Fc) {
     const int eX = lz->e[j];
     const int e_u = eX - Fc + s_u;
@@ -150,13 +161,7 @@ __device__ inline void lz_after_matvec(LzState* lz, int j, i128 alpha_raw, uint6
     const LzCoefs c = lz_coefs(j, alpha_raw, e_u, m_u, eX, lz->m[j], lz->beta[j], lz_inv(lz->beta[j]),
                                j > 0 ? lz->e[j - 1] : 0,
                                j > 0 ? lz->m[j - 1] : 0, j > 0 ? lz_inv(lz->beta[j - 1]) : 0.0, lz->status);
-    lz->alpha[j] = c.alpha;
-    for (int k = 0; k < 3; ++k) {
-        lz->at[k] = c.at[k];
-        lz->sh[k] = 0;
-    }
-    lz->Fa = c.Fa;
-    lz->e_w = c.e_w;
+    lz_store_coefs(lz, j, c);
 }
 
 __device__ inline void lz_after_axpy(LzState* lz, int j, i128 sumsq, uint64_t m_w) {

@@ -225,13 +225,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
                 lz->s_u = s_u;
                 lz->e_u = e_u;
                 lz->m_u = m;
-                lz->alpha[j] = s_coef.alpha;
-                for (int k = 0; k < 3; ++k) {
-                    lz->at[k] = s_coef.at[k];
-                    lz->sh[k] = 0;
-                }
-                lz->Fa = s_coef.Fa;
-                lz->e_w = s_coef.e_w;
+                lz_store_coefs(lz, j, s_coef);
             }
             if (stamp) st[4] = global_ns();
         }
@@ -566,13 +560,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_batch(const MvArgs a, con
                 lz->s_u = s_u;
                 lz->e_u = e_u;
                 lz->m_u = m;
-                lz->alpha[j] = s_coef[b].alpha;
-                for (int k = 0; k < 3; ++k) {
-                    lz->at[k] = s_coef[b].at[k];
-                    lz->sh[k] = 0;
-                }
-                lz->Fa = s_coef[b].Fa;
-                lz->e_w = s_coef[b].e_w;
+                lz_store_coefs(lz, j, s_coef[b]);
             }
         }
         __syncthreads();
@@ -808,13 +796,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_multi(const LzMultiArgs f
                 lz->s_u = s_u;
                 lz->e_u = e_u;
                 lz->m_u = m;
-                lz->alpha[j] = s_coef[b].alpha;
-                for (int k = 0; k < 3; ++k) {
-                    lz->at[k] = s_coef[b].at[k];
-                    lz->sh[k] = 0;
-                }
-                lz->Fa = s_coef[b].Fa;
-                lz->e_w = s_coef[b].e_w;
+                lz_store_coefs(lz, j, s_coef[b]);
             }
         }
         __syncthreads();

@@ -286,13 +286,7 @@ __global__ void __launch_bounds__(kRoThreads, 1) k_lz_reorth_run(const MvArgs a,
                 lz->s_u = s_u;
                 lz->e_u = e_u;
                 lz->m_u = m;
-                lz->alpha[j] = s_coef.alpha;
-                for (int k = 0; k < 3; ++k) {
-                    lz->at[k] = s_coef.at[k];
-                    lz->sh[k] = 0;
-                }
-                lz->Fa = s_coef.Fa;
-                lz->e_w = s_coef.e_w;
+                lz_store_coefs(lz, j, s_coef);
                 lz->e[j + 1] = s_coef.e_w;
             }
         }

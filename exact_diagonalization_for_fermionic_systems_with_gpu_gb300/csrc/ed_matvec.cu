@@ -341,7 +341,7 @@ cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, vo
         StripedArgs g;
         cudaError_t e = striped_args(const_cast<ed_op*>(op), xq, &g);
         if (e == cudaSuccess) e = launch_striped_down(op, g, s);
-        if (e == cudaSuccess) e = launch_striped_up(op, a, g, 1, s);
+        if (e == cudaSuccess) e = launch_striped_up(op, a, g, s);
         return e;
     }
     if (op->tma_smem > 0) return launch_matvec_tma(op, a, s);

@@ -51,7 +51,9 @@ __device__ __forceinline__ void load_x(const int64_t* __restrict__ xq, uint32_t 
 
 // Lanczos epilogue of a matvec launch: block sums of <x, u> and max|u|,
 // then the last block finishes the grid reduction and the step scalars.
+// Nothing in a second pass (step < 0), which knows them.
 __device__ __forceinline__ void mv_lanczos_epilogue(const MvArgs& a, i128 dot, uint64_t mx, int s_u) {
+    if (a.step < 0) return;
     __shared__ i128 s128[32];
     __shared__ uint64_t s64[32];
     LzState* lz = reinterpret_cast<LzState*>(a.lz);

@@ -23,8 +23,7 @@
 //   rows so that the stripe of x (dim_up x kStripe x 8 B) stays in L2 while
 //   every row's up neighbours gather from it; a warp computes one row of a
 //   stripe (two column pairs per lane, 16-byte loads), adds S_dn and the diagonal,
-//   rounds once, and writes u (FX, Lanczos) or y (FP64, permuted order; the
-//   operator apply keeps the table-order kernels).
+//   rounds once, and writes u (the operator apply keeps the table-order kernels).
 // HBM traffic per matvec: pass D reads x and writes S_dn, pass U reads x,
 // S_dn and writes the result: 5 x 8 B per element (vs 2 x 8 B ideal, and
 // ~14 x 8 B when every up neighbour row is re-read from HBM).
@@ -178,7 +177,9 @@ __global__ void __launch_bounds__(kDownThreads, 1) k_mv_down(const StripedArgs g
 // each 16-byte load instruction of the warp reads one contiguous 512-byte
 // segment; the second pair is absent past the end of the row.  Row offsets
 // are 32-bit element offsets (a vector has < 2^32 elements).
-template <int OUT>
+// SUMS: the Lanczos partials too (a second pass has no use for them; Lieb18 4+9
+// 1.29 ms with, 1.11 ms without).
+template <bool SUMS>
 __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const StripedArgs g) {
     const int64_t dimUP = g.dimUP, dimDN = g.dimDN;
     const uint32_t dn32 = (uint32_t)dimDN;
@@ -187,13 +188,8 @@ __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const S
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nwarps = (int64_t)gridDim.x * (kUpThreads / 32);
     const int64_t* __restrict__ xq = g.xq;
-    int E_out = 0, s_u = 0;
-    if (OUT == 0) {
-        E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
-    } else {
-        const int b = a.bq_bits + bitlen_u64(*a.p_mx) - 62;
-        s_u = b > 0 ? b : 0;
-    }
+    const int sb = a.bq_bits + bitlen_u64(*a.p_mx) - 62;
+    const int s_u = sb > 0 ? sb : 0;
     const bool merge = a.mergeUD != 0;
     const bool unitU = a.unitUP != 0 && a.nclsUP == 1;
     const bool unitD = a.unitDN != 0 && a.nclsDN == 1;
@@ -258,7 +254,6 @@ __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const S
         for (int h = 0; h < 2; ++h) {
             if (h == 1 && !two) break;
             int64_t oq[2];
-            double of[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int q = 2 * h + e;
@@ -274,24 +269,17 @@ __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const S
                 const uint32_t cq = c + 64u * h + e;
                 const int64_t dq = du + __ldg(g.dDNq + cq) + a.Uq * (int64_t)__popcll(stu & __ldg(g.stDN + cq) & a.mask);
                 ar += mul_wide(dq, xv);
-                if (OUT == 0) {
-                    of[e] = i128_to_f64(ar, E_out);
-                } else {
-                    oq[e] = shr_round_i64(ar, s_u);
+                oq[e] = shr_round_i64(ar, s_u);
+                if (SUMS) {
                     dot += mul_wide(xv, oq[e]) >> 24;
                     const uint64_t aq = (uint64_t)(oq[e] < 0 ? -oq[e] : oq[e]);
                     mx = aq > mx ? aq : mx;
                 }
             }
-            if (OUT == 0) {
-                // the FP64 result overwrites S_dn in place (permuted order)
-                *reinterpret_cast<double2*>(g.sdn + rowu + 64u * h) = make_double2(of[0], of[1]);
-            } else {
-                __stcs(reinterpret_cast<longlong2*>(a.uq + rowu + 64u * h), make_longlong2(oq[0], oq[1]));
-            }
+            __stcs(reinterpret_cast<longlong2*>(a.uq + rowu + 64u * h), make_longlong2(oq[0], oq[1]));
         }
     }
-    if (OUT == 1) mv_lanczos_epilogue(a, dot, mx, s_u);
+    if (SUMS) mv_lanczos_epilogue(a, dot, mx, s_u);
 }
 
 // ---------------------------------------------------- down-index permutes --
@@ -334,9 +322,9 @@ cudaError_t launch_striped_down(const ed_op* op, const StripedArgs& g, cudaStrea
     return cudaGetLastError();
 }
 
-cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, int out, cudaStream_t s) {
-    if (out == 0) k_mv_up<0><<<op->st_grid, kUpThreads, 0, s>>>(a, g);
-    else k_mv_up<1><<<op->st_grid, kUpThreads, 0, s>>>(a, g);
+cudaError_t launch_striped_up(const ed_op* op, const MvArgs& a, const StripedArgs& g, cudaStream_t s) {
+    if (a.step >= 0) k_mv_up<true><<<op->st_grid, kUpThreads, 0, s>>>(a, g);
+    else k_mv_up<false><<<op->st_grid, kUpThreads, 0, s>>>(a, g);
     return cudaGetLastError();
 }
 
