@@ -114,6 +114,8 @@ struct SpinEntry {
     ed::SpinTable table;
     int sched_state = 0;  // 0 not built, 1 built, -1 the table takes no schedule
     ed::GatherSchedule sched;
+    int pair_state = 0;   // the same of the row-pair schedule
+    ed::PairSchedule pair;
 };
 
 std::mutex g_spin_mu;
@@ -179,28 +181,36 @@ ed_status build_spin_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bo
     return ED_OK;
 }
 
-// The row engine's gather schedule of a table built through the cache.
-bool gather_schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx, const ed::SpinTable& td,
-                            ed::GatherSchedule* gs, std::string* err) {
+// A schedule of a table built through the cache, kept in its entry.
+template <typename S, typename F>
+bool schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx, int SpinEntry::*state,
+                     S SpinEntry::*kept, S* out, const F& build) {
     const SpinKey k = spin_key(b.n_sites, b.n_part, cplx, t, nt);
     {
         std::lock_guard<std::mutex> g(g_spin_mu);
         for (SpinEntry& e : g_spin_cache)
-            if (e.key == k && e.sched_state != 0) {
-                if (e.sched_state < 0) return false;
-                *gs = e.sched;
+            if (e.key == k && e.*state != 0) {
+                if (e.*state < 0) return false;
+                *out = e.*kept;
                 return true;
             }
     }
-    const bool ok = ed::build_gather_schedule(td, gs, err);
+    const bool ok = build();
     std::lock_guard<std::mutex> g(g_spin_mu);
     for (SpinEntry& e : g_spin_cache)
         if (e.key == k) {
-            e.sched_state = ok ? 1 : -1;
-            if (ok) e.sched = *gs;
+            e.*state = ok ? 1 : -1;
+            if (ok) e.*kept = *out;
             break;
         }
     return ok;
+}
+
+// The row engine's gather schedule.
+bool gather_schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx, const ed::SpinTable& td,
+                            ed::GatherSchedule* gs, std::string* err) {
+    return schedule_cached(b, t, nt, cplx, &SpinEntry::sched_state, &SpinEntry::sched, gs,
+                           [&] { return ed::build_gather_schedule(td, gs, err); });
 }
 
 }  // namespace
@@ -268,11 +278,13 @@ static ed_status plan_striped(ed_op* op, bool forced, int64_t chunk_cap = 16384)
 
 // Plans and uploads the row-pair matvec where two rows fit shared memory;
 // leaves op->pair false otherwise.
-static ed_status plan_pair(ed_op* op) {
+static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
     if (ed::pair_smem_bytes((op->dimDN + 7) / 8 * 8) == 0) return ED_OK;
     ed::PairSchedule g;
     std::string err;
-    if (!ed::build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err)) return ED_OK;
+    if (!schedule_cached(op->bdn, dn_terms, n_dn_terms, false, &SpinEntry::pair_state, &SpinEntry::pair, &g,
+                         [&] { return ed::build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err); }))
+        return ED_OK;
     if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
         upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
         upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
@@ -495,8 +507,12 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
               upload(&op->d_dDNq, dq_d.data(), dq_d.size()) == cudaSuccess &&
               upload(&op->d_stUP, op->bup.state.data(), op->bup.state.size()) == cudaSuccess &&
               upload(&op->d_stDN, op->bdn.state.data(), op->bdn.state.size()) == cudaSuccess &&
-              cudaMalloc(&op->d_emax, sizeof(int)) == cudaSuccess && cudaMalloc(&op->d_flag, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&op->d_apply, sizeof(int) * (ed::kApplyPart + 1)) == cudaSuccess;
+              cudaMalloc(&op->d_emax, sizeof(int) * (4 + ed::kApplyPart + 1)) == cudaSuccess &&
+              cudaMemset(op->d_emax, 0, 4 * sizeof(int)) == cudaSuccess;
+    // one allocation for the small words
+    op->d_flag = op->d_emax + 1;
+    op->d_err = op->d_emax + 2;
+    op->d_apply = op->d_emax + 4;
     // CSR copies (row-contiguous entries) for the shared-memory kernel
     auto csr = [](const ed::SpinTable& t, std::vector<uint32_t>* ptr, std::vector<uint32_t>* ent) {
         ptr->assign(t.count + 1, 0);
@@ -513,8 +529,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     ok = ok && upload(&op->d_upPtr, up_ptr.data(), up_ptr.size()) == cudaSuccess &&
          upload(&op->d_upEntC, up_ent.data(), up_ent.size()) == cudaSuccess &&
          upload(&op->d_dnPtr, dn_ptr.data(), dn_ptr.size()) == cudaSuccess &&
-         upload(&op->d_dnEntC, dn_ent.data(), dn_ent.size()) == cudaSuccess &&
-         cudaMalloc(&op->d_err, sizeof(int)) == cudaSuccess && cudaMemset(op->d_err, 0, sizeof(int)) == cudaSuccess;
+         upload(&op->d_dnEntC, dn_ent.data(), dn_ent.size()) == cudaSuccess;
     if (!ok) { ed_op_destroy(op); return ED_ERR_ALLOC; }
     // class segments for multi-class tables with at most kSegCls classes
     auto segments = [](const ed::SpinTable& t, std::vector<uint32_t>* se, std::vector<uint32_t>* sp) {
@@ -555,6 +570,44 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         a.dnSegE = op->d_dnSegE;
         a.dnSegP = op->d_dnSegP;
         a.mergeMC = (a.nclsUP == a.nclsDN && tu.coef == td.coef) ? 1 : 0;
+        if (cplx) {
+            // the complex row engine's schedule; without one the operator takes
+            // the general path
+            ed::ClassSchedule cs;
+            std::string cerr;
+            if (ed::build_class_schedule(td, &cs, &cerr)) {
+                // one upload: words (64 bytes a step of a block), counts, steps
+                std::vector<uint32_t> all(cs.words.size() / 2 + cs.negcnt.size() + cs.steps4.size());
+                std::memcpy(all.data(), cs.words.data(), cs.words.size() * 2);
+                std::copy(cs.negcnt.begin(), cs.negcnt.end(), all.begin() + cs.words.size() / 2);
+                std::copy(cs.steps4.begin(), cs.steps4.end(), all.begin() + cs.words.size() / 2 + cs.negcnt.size());
+                if (upload(&op->d_clsSched, all.data(), all.size()) != cudaSuccess) {
+                    ed_op_destroy(op);
+                    return ED_ERR_ALLOC;
+                }
+                a.clsSched = reinterpret_cast<const uint16_t*>(op->d_clsSched);
+                a.clsNeg = op->d_clsSched + cs.words.size() / 2;
+                a.clsSteps = a.clsNeg + cs.negcnt.size();
+                a.schedSteps = cs.steps;
+                a.dimDNp = (int)cs.cpad;
+            } else {
+                a.upSegE = a.upSegP = a.dnSegE = a.dnSegP = nullptr;
+            }
+            auto partners = [](const int64_t* coef, int n, int8_t* part) {
+                for (int c = 0; c < ed::kSegCls; ++c) part[c] = (int8_t)c;
+                for (int c = 0; c < n; ++c) {
+                    if (part[c] != c || coef[2 * c + 1] == 0) continue;
+                    for (int q = c + 1; q < n; ++q)
+                        if (part[q] == q && coef[2 * q] == coef[2 * c] && coef[2 * q + 1] == -coef[2 * c + 1]) {
+                            part[c] = (int8_t)q;
+                            part[q] = -1;
+                            break;
+                        }
+                }
+            };
+            partners(a.coefUP, a.nclsUP, a.partUP);
+            partners(a.coefDN, a.nclsDN, a.partDN);
+        }
     }
     // entries per (row, class) run of the two tables: below 2, a product per
     // entry replaces the running class sums
@@ -580,8 +633,6 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     // single class); ED_NO_SCHED=1 keeps the CSR gathers
     a.dnSched = nullptr;
     a.dnSteps = nullptr;
-    a.schedSteps = 0;
-    a.dimDNp = 0;
     if (!cplx && td.coef.size() <= 1 && !std::getenv("ED_NO_SCHED")) {
         ed::GatherSchedule gs;
         std::string serr;
@@ -624,7 +675,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     // real single-class sectors whose tables leave no room for that plan but
     // where two rows fit (3,000 to 14,000 down states): the row-pair kernel
     if (op->tma_smem == 0 && (want.empty() || want == "pair") && !cplx && op->mv_fast) {
-        const ed_status pst = plan_pair(op);
+        const ed_status pst = plan_pair(op, desc->dn_terms, desc->n_dn_terms);
         if (pst != ED_OK) {
             ed_op_destroy(op);
             return pst;
@@ -678,10 +729,10 @@ ed_status ed_op_destroy(ed_op* op) {
     cudaFree(op->d_upSegE); cudaFree(op->d_upSegP); cudaFree(op->d_dnSegE); cudaFree(op->d_dnSegP);
     cudaFree(op->d_permDN); cudaFree(op->d_sched16); cudaFree(op->d_steps32); cudaFree(op->d_dDNqP);
     cudaFree(op->d_stDNp); cudaFree(op->d_sdn); cudaFree(op->d_negDN);
+    cudaFree(op->d_clsSched);
     cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);
-    cudaFree(op->d_err);
     cudaFree(op->d_dUPq); cudaFree(op->d_dDNq); cudaFree(op->d_stUP); cudaFree(op->d_stDN);
-    cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_flag); cudaFree(op->d_apply); cudaFree(op->d_io);
+    cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_io);
     if (op->h_stage) cudaFreeHost(op->h_stage);
     delete ox;
     return ED_OK;

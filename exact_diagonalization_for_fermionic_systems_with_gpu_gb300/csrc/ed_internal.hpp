@@ -81,6 +81,14 @@ struct MvArgs {
     const uint32_t* upSegP;
     const uint32_t* dnSegE;
     const uint32_t* dnSegP;
+    // class schedule of the down term (complex operators with class segments;
+    // null otherwise), ed::ClassSchedule
+    const uint16_t* clsSched;
+    const uint32_t* clsSteps;
+    const uint32_t* clsNeg;
+    // partner[c] > c: class partner[c] has the conjugate coefficient of class c;
+    // partner[c] == c: none has; -1: c is another one's partner
+    int8_t partUP[kSegCls], partDN[kSegCls];
     int perEntry;         // multi-class tables whose rows hold about one entry of a class: a product per entry
     int mergeMC;          // segmented tables with equal class lists: one product per class
     // coefficient classes, interleaved (re, im), scale 2^-Fc
@@ -153,14 +161,15 @@ struct ed_op {
     uint8_t* d_dnSteps = nullptr;
     uint32_t *d_rowStart = nullptr, *d_rowList = nullptr, *d_rowQueue = nullptr, *d_unitQueue = nullptr;
     uint32_t *d_upSegE = nullptr, *d_upSegP = nullptr, *d_dnSegE = nullptr, *d_dnSegP = nullptr;
-    int* d_err = nullptr;
+    uint32_t* d_clsSched = nullptr;  // the class schedule's three tables
+    int* d_err = nullptr;       // (in d_emax's allocation)
     int64_t *d_dUPq = nullptr, *d_dDNq = nullptr;
     uint64_t *d_stUP = nullptr, *d_stDN = nullptr;
     // perform-path workspace (grow-only)
     int64_t* d_xq = nullptr;
     int* d_emax = nullptr;
-    int* d_flag = nullptr;
-    int* d_apply = nullptr;     // kApplyPart ints and the queue counter
+    int* d_flag = nullptr;      // (in d_emax's allocation)
+    int* d_apply = nullptr;     // kApplyPart ints and the queue counter (in d_emax's allocation)
     double* h_stage = nullptr;  // pinned staging for host-pointer perform
     size_t h_stage_bytes = 0;
     double* d_io = nullptr;     // device x|y for host-pointer perform

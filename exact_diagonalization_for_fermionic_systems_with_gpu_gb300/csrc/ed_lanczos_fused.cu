@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
         s_min_bits = lz->min_bits;
         if (f.mirror && blockIdx.x == 0 && j == 0) mirror_slot(f.mirror, lz, 0);
     }
-    if (SCHED) tma_zero_slots(a, S);
+    if (SCHED || (CPLX && SEG)) tma_zero_slots(a, S);
     __syncthreads();
     if (!tma::mbar_wait(&S.bar[2], 0)) {
         if (tid == 0) atomicExch(a.err, 1);
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_multi(const LzMultiArgs f
                     tma::fence_proxy_async_smem();
                     tma_issue_tables(s_args, S);
                 }
-                if (I.kind == kKindRealSched) tma_zero_slots(s_args, S);
+                if (I.kind == kKindRealSched || I.kind == kKindCplxSeg) tma_zero_slots(s_args, S);
                 if (!tma::mbar_wait(&S.bar[2], tc & 1)) {
                     if (tid == 0) atomicExch(s_args.err, 1);
                     give_up = 1;

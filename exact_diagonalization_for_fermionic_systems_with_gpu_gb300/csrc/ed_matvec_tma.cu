@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_matvec_tma(const MvArgs a) {
         tma_issue_tables(a, S);
         if (has_row) tma_issue_row<CPLX>(a, S, a.xq, u0, 0);
     }
-    if (SCHED) tma_zero_slots(a, S);
+    if (SCHED || (CPLX && SEG)) tma_zero_slots(a, S);
     __syncthreads();
     if (!tma::mbar_wait(&S.bar[2], 0)) {
         if (threadIdx.x == 0) atomicExch(a.err, 1);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const 
         tma_init(S);
         tma_issue_tables(a, S);
     }
-    if (SCHED) tma_zero_slots(a, S);
+    if (SCHED || (CPLX && SEG)) tma_zero_slots(a, S);
     {
         int e = 0;
 #pragma unroll 4
@@ -186,6 +186,7 @@ int tma_plan(const ed_op* op, MvArgs* a) {
     const int W = op->cplx ? 2 : 1;
     const int64_t dimDN = op->dimDN;
     // an odd real row is copied with one element before or after it
+    // (a complex row has its zero slot there)
     const int64_t row_bytes = ((dimDN * W + 2) & ~(int64_t)1) * 8;
     // the gather schedule serves the single-class real kernel only
     if (op->cplx || !op->mv_fast) {
@@ -205,6 +206,13 @@ int tma_plan(const ed_op* op, MvArgs* a) {
         off += up128((int64_t)a->schedSteps * a->dimDNp * 2);
         a->sm_steps = (int)off;
         off += up128(a->dimDNp / 32);
+    } else if (a->clsSched) {
+        a->sm_sched = (int)off;
+        off += up128((int64_t)a->schedSteps * a->dimDNp * 2);
+        a->sm_steps = (int)off;
+        off += up128(a->dimDNp / 32 * 4);
+        a->sm_dnnpos = (int)off;
+        off += up128((int64_t)a->dimDNp * 4);
     } else {
         a->sm_dnptr = (int)off;
         off += up128((dimDN + 1) * 4);

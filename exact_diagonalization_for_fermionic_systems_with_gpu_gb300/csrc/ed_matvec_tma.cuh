@@ -94,8 +94,8 @@ struct TmaSmem {
     uint8_t* dnpos;
     int64_t* ddq;
     uint64_t* dst;
-    uint16_t* sched;  // gather schedule (when a.dnSched)
-    uint8_t* steps;
+    uint16_t* sched;  // gather schedule (a.dnSched) or class schedule (a.clsSched, its
+    uint8_t* steps;   // step words here, its negative counts at dnpos)
     uint32_t* uoff;
     uint32_t* uent;
     int* give_up;
@@ -160,6 +160,18 @@ __device__ __forceinline__ void tma_issue_tables(const MvArgs& a, const TmaSmem&
         tma::bulk_g2s(S.dst, a.stDN, b_dq, &S.bar[2]);
         return;
     }
+    if (a.clsSched) {
+        const uint32_t b_sc = tma::round16((uint32_t)a.schedSteps * (uint32_t)a.dimDNp * 2u),
+                       b_stp = tma::round16((uint32_t)a.dimDNp / 32u * 4u), b_neg = tma::round16((uint32_t)a.dimDNp * 4u),
+                       b_dq = tma::round16(dimDN * 8u);
+        tma::expect_tx(&S.bar[2], b_sc + b_stp + b_neg + 2 * b_dq);
+        tma::bulk_g2s(S.sched, a.clsSched, b_sc, &S.bar[2]);
+        tma::bulk_g2s(S.steps, a.clsSteps, b_stp, &S.bar[2]);
+        tma::bulk_g2s(S.dnpos, a.clsNeg, b_neg, &S.bar[2]);
+        tma::bulk_g2s(S.ddq, a.dDNq, b_dq, &S.bar[2]);
+        tma::bulk_g2s(S.dst, a.stDN, b_dq, &S.bar[2]);
+        return;
+    }
     const uint32_t b_ptr = tma::round16((dimDN + 1) * 4u), b_ent = tma::round16(a.dnNnz * 4u),
                    b_pos = tma::round16(dimDN), b_dq = tma::round16(dimDN * 8u), b_st = b_dq;
     tma::expect_tx(&S.bar[2], b_ptr + b_ent + b_pos + b_dq + b_st);
@@ -171,8 +183,16 @@ __device__ __forceinline__ void tma_issue_tables(const MvArgs& a, const TmaSmem&
 }
 
 // The 16 zeros of both row buffers that idle lanes of the gather schedule
-// read (the bulk copies only ever write [0, dimDN)).
+// read (the bulk copies only ever write [0, dimDN)), or the zero slot after a
+// complex row.
 __device__ __forceinline__ void tma_zero_slots(const MvArgs& a, const TmaSmem& S) {
+    if (a.clsSched) {
+        if (threadIdx.x < 2) {
+            S.row0[2 * a.dimDN + threadIdx.x] = 0;
+            S.row1[2 * a.dimDN + threadIdx.x] = 0;
+        }
+        return;
+    }
     if (threadIdx.x < 17) {  // 16 zeros after [x | -x] at either row offset
         S.row0[2 * a.schedNeg + threadIdx.x] = 0;
         S.row1[2 * a.schedNeg + threadIdx.x] = 0;
@@ -238,6 +258,44 @@ __device__ __forceinline__ void row_elem(const int64_t* xrow, uint32_t col, int6
         r = xrow[col];
         i = 0;
     }
+}
+
+// The classes' complex sums (sr, si) times their coefficients, added to
+// (ar, ai).  A class and the one with the conjugate coefficient share four
+// products where each alone takes four: with c, S1 and c*, S2,
+//   Re = Re c Re(S1 + S2) - Im c Im(S1 - S2), Im = Re c Im(S1 + S2) + Im c Re(S1 - S2)
+struct ClassSum {
+    int64_t r, i;
+};
+
+__device__ __forceinline__ void class_products(i128& ar, i128& ai, const ClassSum s0, const ClassSum s1,
+                                               const ClassSum s2, const ClassSum s3, const int64_t* __restrict__ coef,
+                                               const int8_t* __restrict__ part, int n) {
+    auto four = [&](ClassSum p, ClassSum q, int c) {
+        const int64_t cr = coef[2 * c], ci = coef[2 * c + 1];
+        mac_wide(ar, p.r, cr);
+        mac_wide(ai, p.i, cr);
+        if (ci != 0) {
+            mac_wide(ar, -q.i, ci);
+            mac_wide(ai, q.r, ci);
+        }
+    };
+    auto one = [&](const ClassSum& s, int c) {
+        if (c < n && part[c] == c) four(s, s, c);
+    };
+    auto two = [&](const ClassSum& s, const ClassSum& t, int c, int q) {
+        if (c < n && part[c] == q) four({s.r + t.r, s.i + t.i}, {s.r - t.r, s.i - t.i}, c);
+    };
+    one(s0, 0);
+    two(s0, s1, 0, 1);
+    two(s0, s2, 0, 2);
+    two(s0, s3, 0, 3);
+    one(s1, 1);
+    two(s1, s2, 1, 2);
+    two(s1, s3, 1, 3);
+    one(s2, 2);
+    two(s2, s3, 2, 3);
+    one(s3, 3);
 }
 
 // First row of this CTA (rowList[rowStart[b]]); false when it has none.
@@ -433,6 +491,62 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
                         apply_class<CPLX>(ar1, ai1, dr1, di1, a.coefDN, 0, unitD, a.Fc);
                     }
                 }
+            } else if (SEG && CPLX) {
+                // at most kSegCls classes, one sum for each, products at the end.
+                // Up entries (the same for every lane) are loaded four at a time
+                // and added by class; the down schedule's steps go class by
+                // class.  Against a loop per signed class segment, whose trip
+                // counts follow the warp's longest lane (25 steps for 13 hops;
+                // 18.5 here) and put each load behind the last: complex
+                // Kagome12 apply 84 -> 74 us, persistent step 89 -> 75 us.
+                const uint32_t d = d0;
+                // (named sums: an array would be indexed by the class, in local
+                // memory)
+                ClassSum s0{0, 0}, s1{0, 0}, s2{0, 0}, s3{0, 0};
+                for (uint32_t k = 0; k < lenU; k += 4) {
+                    int64_t vr[4], vi[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) up_load<CPLX, COH>(xq, S.uoff[min(k + t, lenU - 1)] + d, vr[t], vi[t]);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        if (k + t >= lenU) break;
+                        const uint32_t e = S.uent[k + t], cl = (e >> kClassShift) & 3u;
+                        const int64_t r = apply_sign(vr[t], e), i = apply_sign(vi[t], e);
+                        if (cl & 2u) {
+                            if (cl & 1u) { s3.r += r; s3.i += i; } else { s2.r += r; s2.i += i; }
+                        } else {
+                            if (cl & 1u) { s1.r += r; s1.i += i; } else { s0.r += r; s0.i += i; }
+                        }
+                    }
+                }
+                if (!a.mergeMC) {
+                    class_products(ar0, ai0, s0, s1, s2, s3, a.coefUP, a.partUP, a.nclsUP);
+                    s0 = s1 = s2 = s3 = ClassSum{0, 0};
+                }
+                const uint32_t dp = (uint32_t)a.dimDNp;
+                const uint32_t ns = reinterpret_cast<const uint32_t*>(S.steps)[d >> 5];
+                const uint32_t ng = reinterpret_cast<const uint32_t*>(S.dnpos)[d];
+                const uint16_t* sc = S.sched + d;
+                // v ^ m with m = 0 or -1; the -m parts, the class's negative
+                // entries of the column, are added once
+                auto steps = [&](ClassSum& sum, int n, int neg) {
+                    int64_t r = neg, i = neg;
+#pragma unroll 2
+                    for (int t = 0; t < n; ++t, sc += dp) {
+                        const uint32_t w = *sc;
+                        const longlong2 v = *reinterpret_cast<const longlong2*>(xrow + 2 * (w & 0x7FFFu));
+                        const int64_t m = -(int64_t)(w >> 15);
+                        r += v.x ^ m;
+                        i += v.y ^ m;
+                    }
+                    sum.r += r;
+                    sum.i += i;
+                };
+                steps(s0, ns & 0xFFu, ng & 0xFFu);
+                steps(s1, (ns >> 8) & 0xFFu, (ng >> 8) & 0xFFu);
+                steps(s2, (ns >> 16) & 0xFFu, (ng >> 16) & 0xFFu);
+                steps(s3, ns >> 24, ng >> 24);
+                class_products(ar0, ai0, s0, s1, s2, s3, a.coefDN, a.partDN, a.nclsDN);
             } else if (SEG) {
                 // at most kSegCls classes: class by class over segments taken
                 // from the rows' class-end bytes (+ entries first), the same
@@ -510,13 +624,13 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
                     const uint32_t cl = (e >> kClassShift) & kClassMask;
                     r = apply_sign(r, e);
                     const int64_t cr = coef[2 * cl];
-                    ar += mul_wide(r, cr);
+                    mac_wide(ar, r, cr);
                     if (CPLX) {
                         i = apply_sign(i, e);
                         const int64_t ci = coef[2 * cl + 1];
-                        ai += mul_wide(i, cr);
-                        ar -= mul_wide(i, ci);
-                        ai += mul_wide(r, ci);
+                        mac_wide(ai, i, cr);
+                        mac_wide(ar, -i, ci);
+                        mac_wide(ai, r, ci);
                     }
                 };
                 for (uint32_t k = 0; k < lenU; k += kN) {

@@ -688,6 +688,48 @@ bool build_pair_schedule(const SpinTable& t, bool adjacent, PairSchedule* g, std
     return true;
 }
 
+bool build_class_schedule(const SpinTable& t, ClassSchedule* g, std::string* err) {
+    constexpr int kC = 4;
+    if (t.coef.size() > kC || t.count >= (1 << 15)) {
+        if (err) *err = "class schedule: more than four classes or too many states";
+        return false;
+    }
+    const int64_t cpad = (t.count + 31) / 32 * 32, nb = cpad / 32;
+    g->cpad = cpad;
+    g->steps4.assign(nb, 0);
+    g->negcnt.assign(cpad, 0);
+    // a block's steps of a class: the most entries of it any of its columns has
+    std::vector<uint32_t> count4(cpad, 0);  // byte c: entries of class c (a row has at most 255)
+    int smax = 1;
+    for (int64_t b = 0; b < nb; ++b) {
+        int most[kC] = {0};
+        for (int64_t d = 32 * b; d < std::min<int64_t>(32 * b + 32, t.count); ++d) {
+            for (int k = 0; k < t.len[d]; ++k) {
+                const uint32_t e = t.ent[(size_t)k * t.count + d], one = 1u << (8 * ((e >> kClassShift) & kClassMask));
+                count4[d] += one;
+                if (e & kSignBit) g->negcnt[d] += one;
+            }
+            for (int c = 0; c < kC; ++c) most[c] = std::max<int>(most[c], (count4[d] >> (8 * c)) & 0xFF);
+        }
+        for (int c = 0; c < kC; ++c) g->steps4[b] |= (uint32_t)most[c] << (8 * c);
+        smax = std::max(smax, most[0] + most[1] + most[2] + most[3]);
+    }
+    g->steps = smax;
+    g->words.assign((size_t)smax * cpad, (uint16_t)t.count);
+    for (int64_t d = 0; d < t.count; ++d) {
+        const uint32_t ns = g->steps4[d / 32];
+        int base = 0, k = 0;  // entries are ordered by class
+        for (int c = 0; c < kC; ++c) {
+            for (int q = 0; q < (int)((count4[d] >> (8 * c)) & 0xFF); ++q, ++k) {
+                const uint32_t e = t.ent[(size_t)k * t.count + d];
+                g->words[(size_t)(base + q) * cpad + d] = (uint16_t)((e & kColMask) | (e & kSignBit) >> 16);
+            }
+            base += (ns >> (8 * c)) & 0xFF;
+        }
+    }
+    return true;
+}
+
 std::vector<uint32_t> unit_queue(const std::vector<uint32_t>& rq, int64_t dimDN, int G) {
     const size_t k = G > 0 ? rq.size() % (size_t)G : 0;
     // parts of a multiple of 32 columns, every one of them non-empty

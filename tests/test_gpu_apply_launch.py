@@ -123,3 +123,51 @@ def test_entry_products_match_generic(ed, monkeypatch, case):
     for other in runs[1:]:
         assert other[:3] == runs[0][:3]
         assert np.array_equal(other[3], runs[0][3])
+
+
+@pytest.mark.parametrize("case", ["pairs", "pairs_odd", "real_class", "imaginary", "unequal_spins", "no_down_hops", "one_row"])
+def test_complex_class_sums_match_generic(ed, monkeypatch, case):
+    """Complex operators of at most four classes (class sums, conjugate classes
+    sharing their products) in the apply, per-step, persistent and batched
+    kernels against the generic kernel bit for bit."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    import math
+    ring = lambda n, v, ph: [("P", i, (i + 1) % n, v, ph) for i in range(n)]  # noqa: E731
+    N, qu, qd, U = 9, 4, 3, 2.0
+    tu = td = ring(9, -1.0, 0.3) + [("P", i, (i + 2) % 9, 0.5, 0.6) for i in range(9)]
+    if case == "pairs_odd":
+        N, qu, qd = 7, 3, 2
+        tu = td = ring(7, -1.0, 0.3) + [("P", i, (i + 2) % 7, 0.5, 0.6) for i in range(7)]
+    elif case == "real_class":
+        tu = td = ring(9, -1.0, 0.3) + [("P", 0, 4, 0.7, 0.0)]
+    elif case == "imaginary":
+        tu = td = ring(9, 1.0, math.pi / 2) + [("P", 0, 4, 0.7, 0.2)]
+    elif case == "unequal_spins":
+        td = ring(9, -0.25, 0.1)
+    elif case == "no_down_hops":
+        td = [("N", i, 0, 0.1 * i, 0.0) for i in range(9)]
+    elif case == "one_row":
+        qu = 9
+    ops = {}
+    for kind in ("auto", "generic"):
+        if kind == "generic":
+            monkeypatch.setenv("ED_MATVEC", "generic")
+        ops[kind] = ed.Hubbard(ed.H_TBq(N, qu).extend(tu), ed.H_TBq(N, qd).extend(td), U)
+        monkeypatch.delenv("ED_MATVEC", raising=False)
+    n = ops["auto"].rows()
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    assert np.array_equal(ops["auto"].matvec(x), ops["generic"].matvec(x))
+    runs = []
+    for kind, form in (("generic", "0"), ("auto", "0"), ("auto", "1")):
+        monkeypatch.setenv("ED_LZ_FUSED", form)
+        lz = ed.Lanczos()
+        e, v = lz.eigen(ops[kind], max_steps=20, mode="fixed", seed=6)
+        runs.append((e, lz.a, lz.b, v))
+    monkeypatch.delenv("ED_LZ_FUSED")
+    chain = ed.Hubbard(ed.H_TBq(8, 4).extend(L.chain(8)), ed.H_TBq(8, 4).extend(L.chain(8)), 1.0)
+    e, vs, al, be = ed.lanczos_multi([chain, ops["auto"]], 20, seed=5)  # run 1 from seed 6
+    runs.append((e[1], list(al[1]), list(be[1]), vs[1]))
+    for other in runs[1:]:
+        assert other[:3] == runs[0][:3]
+        assert np.array_equal(other[3], runs[0][3])
