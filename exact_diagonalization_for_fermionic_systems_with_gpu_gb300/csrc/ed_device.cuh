@@ -181,6 +181,12 @@ __device__ __forceinline__ int64_t shr_round_i64(i128 v, int s) {
     return (int64_t)((v + ((i128)1 << (s - 1))) >> s);
 }
 
+// round((s 2^Fc + d) / 2^su) for Fc >= su > 0: the first part is a multiple of
+// the divisor, so only d is rounded (no 128-bit shift and addition of s).
+__device__ __forceinline__ int64_t fold_round(int64_t s, i128 d, int Fc, int su) {
+    return (s << (Fc - su)) + shr_round_i64(d, su);
+}
+
 __device__ __forceinline__ int bitlen_u64(uint64_t v) { return v ? 64 - __clzll((long long)v) : 0; }
 
 // ---------------------------------------------------------- warp / block ops --

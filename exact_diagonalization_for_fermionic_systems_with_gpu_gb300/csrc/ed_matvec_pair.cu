@@ -241,8 +241,7 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
                     const int64_t x = xr[r], us = r ? up[h].b : up[h].a, ds = r ? dn[h].b : dn[h].a;
                     const int64_t dq = R.du + ddn + a.Uq * (int64_t)__popcll(R.st & std_);
                     if (OUT == 1 && fold) {
-                        // (S 2^Fc + dq x) >> s_u with Fc >= s_u > 0: the hops' part is a multiple
-                        qo[r][h] = (us << (a.Fc - s_u)) + shr_round_i64(mul_wide(dq, x), s_u);
+                        qo[r][h] = fold_round(us, mul_wide(dq, x), a.Fc, s_u);
                     } else {
                         i128 ar = 0, ai = 0;
                         if (MERGE) {

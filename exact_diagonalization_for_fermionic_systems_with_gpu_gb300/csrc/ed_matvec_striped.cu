@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const S
     const bool merge = a.mergeUD != 0;
     const bool unitU = a.unitUP != 0 && a.nclsUP == 1;
     const bool unitD = a.unitDN != 0 && a.nclsDN == 1;
+    const bool fold = merge && unitU && s_u > 0 && a.Fc >= s_u;  // see fold_round
     i128 dot = 0;
     uint64_t mx = 0;
     for (int64_t it = (int64_t)blockIdx.x * (kUpThreads / 32) + warp; it < nitems; it += nwarps) {
@@ -259,17 +260,20 @@ __global__ void __launch_bounds__(kUpThreads, 1) k_mv_up(const MvArgs a, const S
                 const int q = 2 * h + e;
                 const int64_t dn_sum = e ? dsv[h].y : dsv[h].x;
                 const int64_t xv = e ? xs[h].y : xs[h].x;
-                i128 ar = 0, ai = 0;
-                if (merge) {
-                    apply_class<false>(ar, ai, sp[q] + dn_sum, 0, a.coefUP, 0, unitU, a.Fc);
-                } else {
-                    if (len) apply_class<false>(ar, ai, sp[q], 0, a.coefUP, 0, unitU, a.Fc);
-                    if (a.nclsDN) apply_class<false>(ar, ai, dn_sum, 0, a.coefDN, 0, unitD, a.Fc);
-                }
                 const uint32_t cq = c + 64u * h + e;
                 const int64_t dq = du + __ldg(g.dDNq + cq) + a.Uq * (int64_t)__popcll(stu & __ldg(g.stDN + cq) & a.mask);
-                ar += mul_wide(dq, xv);
-                oq[e] = shr_round_i64(ar, s_u);
+                if (fold) {
+                    oq[e] = fold_round(sp[q] + dn_sum, mul_wide(dq, xv), a.Fc, s_u);
+                } else {
+                    i128 ar = mul_wide(dq, xv), ai = 0;
+                    if (merge) {
+                        apply_class<false>(ar, ai, sp[q] + dn_sum, 0, a.coefUP, 0, unitU, a.Fc);
+                    } else {
+                        if (len) apply_class<false>(ar, ai, sp[q], 0, a.coefUP, 0, unitU, a.Fc);
+                        if (a.nclsDN) apply_class<false>(ar, ai, dn_sum, 0, a.coefDN, 0, unitD, a.Fc);
+                    }
+                    oq[e] = shr_round_i64(ar, s_u);
+                }
                 if (SUMS) {
                     dot += mul_wide(xv, oq[e]) >> 24;
                     const uint64_t aq = (uint64_t)(oq[e] < 0 ? -oq[e] : oq[e]);
