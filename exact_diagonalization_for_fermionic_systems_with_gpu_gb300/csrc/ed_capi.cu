@@ -293,9 +293,12 @@ static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
     op->pair_smem = ed::pair_smem_bytes(g.zbase);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
-    // two CTAs of 512 threads an SM where their rows fit, else one of 1,024
+    // two CTAs of 512 threads an SM where their rows fit, else one of 1,024.
+    // Staging two pairs a CTA (fewer barriers) cost more than it saved: the
+    // schedule words then miss the L1 that the shared memory leaves (14-site 7+7
+    // 188 against 164 us); 384, 448 or 640 threads, or three or four smaller
+    // CTAs, were slower or the same
     const bool two = op->pair_smem <= 110 * 1024;
-    op->pair_rows = 2 * op->pair_smem <= 110 * 1024 ? 2 : 1;
     op->pair_threads = two ? 512 : 1024;
     op->pair_grid = two ? 2 * sms : sms;
     op->pair = true;

@@ -201,7 +201,7 @@ struct ed_op {
     // row-pair matvec
     bool pair = false;
     ed::PairArgs pair_args{};
-    int pair_smem = 0, pair_rows = 1, pair_threads = 0, pair_grid = 0;  // bytes of a pair, pairs staged, launch
+    int pair_smem = 0, pair_threads = 0, pair_grid = 0;
     uint16_t* d_pairWords = nullptr;
     uint8_t *d_pairSteps = nullptr, *d_pairNeg = nullptr;
     std::string last_error;

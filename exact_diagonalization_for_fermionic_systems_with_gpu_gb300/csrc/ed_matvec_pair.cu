@@ -14,11 +14,11 @@
 // The next pair's rows are prefetched into L2 meanwhile.
 //
 // Measured against the one-thread-per-element kernel it replaces there (Lanczos
-// matvec): 14-site chain 7+7 230 -> 186 us, 14-site 7+6 237 -> 154 us, 15-site
-// 7+8 1,470 -> 653 us, 16-site 8+8 6,300 -> 2,570 us.  242 instructions an output
-// at 40 % of the issue slots: bound by the latency of the up loads and the
-// schedule words (sixteen to thirty-two warps an SM at 64 registers) and by the
-// barriers at the ends of the staged rows.  Loading the words and the first up
+// matvec): 14-site chain 7+7 230 -> 164 us, 14-site 7+6 237 -> 144 us, 15-site
+// 7+8 1,470 -> 609 us, 16-site 8+8 6,300 -> 2,530 us.  242 instructions an output
+// at 44 % of the issue slots: bound by the latency of the up loads and the
+// schedule words (32 warps an SM at 64 registers) and by the barriers at the
+// ends of the staged rows.  Loading the words and the first up
 // loads ahead of the sums (74 to 90 registers, 24 or 20 warps) was slower.
 #include <cuda_runtime.h>
 
@@ -35,7 +35,6 @@ using namespace dev;
 namespace {
 
 constexpr int kPairUp = 256;  // up entries staged per row (the longest row has 255)
-constexpr int kPairMax = 2;   // row pairs staged at a time
 constexpr int kPairMaxSmem = 220 * 1024;
 
 struct Two {
@@ -103,17 +102,17 @@ struct PairRow {
 // OUT = 0: FP64 y; OUT = 1: FX u with the Lanczos epilogue.  VEC: dim_dn even,
 // lane l has columns 2l, 2l + 1 of a 64-column block; otherwise l, l + 32.
 // MERGE: equal hopping coefficients, one product for the up and down sums.
-// P row pairs are staged at a time (more units per barrier for short rows).
 template <int OUT, bool VEC, bool SIGN, bool MERGE>
-__global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g, const int P) {
+__global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g) {
     extern __shared__ __align__(128) unsigned char xs[];
-    __shared__ uint32_t uoff[2 * kPairMax][kPairUp];
-    __shared__ PairRow rows[2 * kPairMax];
+    __shared__ uint32_t uoff[2][kPairUp];
+    __shared__ PairRow rows[2];
     const uint32_t dimUP = (uint32_t)a.dimUP, dimDN = (uint32_t)a.dimDN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int64_t* __restrict__ xq = a.xq;
     const uint4* __restrict__ words = reinterpret_cast<const uint4*>(g.words);
-    const uint32_t xs32 = (uint32_t)__cvta_generic_to_shared(xs), pstride = (uint32_t)(g.zbase + 8) * 16u;
+    const uint32_t xs32 = (uint32_t)__cvta_generic_to_shared(xs);
+    longlong2* const x2 = reinterpret_cast<longlong2*>(xs);
     int E_out = 0, s_u = 0;
     if (OUT == 0) {
         E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
@@ -126,52 +125,44 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
     const bool y16 = OUT == 1 || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;  // y may start on any double
     i128 dot = 0;
     uint64_t mx = 0;
-    if (tid < 8 * P) *reinterpret_cast<longlong2*>(xs + (tid >> 3) * pstride + (g.zbase + (tid & 7)) * 16) = make_longlong2(0, 0);
-    const uint32_t nitems = (dimUP + 2 * P - 1) / (2 * P);
-    for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
-        const uint32_t ubase = it * 2 * P;
-        const int nrow = (int)min((uint32_t)(2 * P), dimUP - ubase);  // an odd count ends on a pair of one row
-        const int np = (nrow + 1) / 2;
+    if (tid < 8) x2[g.zbase + tid] = make_longlong2(0, 0);
+    const uint32_t npairs = (dimUP + 1) / 2;
+    for (uint32_t it = blockIdx.x; it < npairs; it += gridDim.x) {
+        const uint32_t u0 = 2 * it;
+        const int nrow = u0 + 1 < dimUP ? 2 : 1;  // an odd count ends on a pair of one row
+        const bool has1 = nrow == 2;
         __syncthreads();  // the previous rows are no longer read
         for (int r = 0; r < nrow; ++r) {
-            const uint32_t u = ubase + r, q0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - q0;
+            const uint32_t u = u0 + r, q0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - q0;
             for (uint32_t k = tid; k < len; k += blockDim.x) uoff[r][k] = (__ldg(a.upEntC + q0 + k) & kColMask) * dimDN;
             if (tid == r) rows[r] = {__ldg(a.stUP + u), __ldg(a.dUPq + u), (int)len, (int)__ldg(a.upNpos + u)};
         }
-        for (int p = 0; p < np; ++p) {
-            const int64_t* r0 = xq + (size_t)(ubase + 2 * p) * dimDN;
-            const int64_t* r1 = 2 * p + 1 < nrow ? r0 + dimDN : r0;
-            longlong2* x2 = reinterpret_cast<longlong2*>(xs + p * pstride);
-            if (VEC) {
+        const int64_t* const r0 = xq + (size_t)u0 * dimDN;
+        const int64_t* const r1 = has1 ? r0 + dimDN : r0;
+        if (VEC) {
 #pragma unroll 2
-                for (uint32_t c = 2 * tid; c < dimDN; c += 2 * blockDim.x) {
-                    const longlong2 v0 = __ldg(reinterpret_cast<const longlong2*>(r0 + c));
-                    const longlong2 v1 = __ldg(reinterpret_cast<const longlong2*>(r1 + c));
-                    x2[pair_slot(c)] = make_longlong2(v0.x, v1.x);
-                    x2[pair_slot(c + 1)] = make_longlong2(v0.y, v1.y);
-                }
-            } else {
-#pragma unroll 4
-                for (uint32_t c = tid; c < dimDN; c += blockDim.x)
-                    x2[pair_slot(c)] = make_longlong2(__ldg(r0 + c), __ldg(r1 + c));
+            for (uint32_t c = 2 * tid; c < dimDN; c += 2 * blockDim.x) {
+                const longlong2 v0 = __ldg(reinterpret_cast<const longlong2*>(r0 + c));
+                const longlong2 v1 = __ldg(reinterpret_cast<const longlong2*>(r1 + c));
+                x2[pair_slot(c)] = make_longlong2(v0.x, v1.x);
+                x2[pair_slot(c + 1)] = make_longlong2(v0.y, v1.y);
             }
+        } else {
+#pragma unroll 4
+            for (uint32_t c = tid; c < dimDN; c += blockDim.x) x2[pair_slot(c)] = make_longlong2(__ldg(r0 + c), __ldg(r1 + c));
         }
-        if (tid == 0 && it + gridDim.x < nitems) {
+        if (tid == 0 && it + gridDim.x < npairs) {
             // an even row starts on a 16-byte boundary
-            const uint32_t un = (it + gridDim.x) * 2 * P;
-            const uint32_t bytes = (dimDN * min((uint32_t)(2 * P), dimUP - un) * 8u) & ~15u;
+            const uint32_t un = 2 * (it + gridDim.x);
+            const uint32_t bytes = (dimDN * (un + 1 < dimUP ? 2u : 1u) * 8u) & ~15u;
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(xq + (size_t)un * dimDN), "r"(bytes)
                          : "memory");
         }
         __syncthreads();
-        for (int t = warp; t < np * g.blocks; t += nwarps) {
-            const int p = t >= g.blocks ? 1 : 0, b = t - p * g.blocks;
+        for (int b = warp; b < g.blocks; b += nwarps) {
             const uint32_t c0 = 64u * b + (VEC ? 2u * lane : (uint32_t)lane), c1 = VEC ? c0 + 1 : c0 + 32;
             if (c0 >= dimDN) continue;
-            const bool v1 = VEC || c1 < dimDN;           // the second column exists
-            const bool has1 = 2 * p + 1 < nrow;          // the second row exists
-            const uint32_t u0 = ubase + 2 * p, xp = xs32 + p * pstride;
-            const uint32_t* const uo[2] = {uoff[2 * p], uoff[2 * p + 1]};
+            const bool v1 = VEC || c1 < dimDN;  // the second column exists
             const int64_t* const xc = xq + c0;
             auto get = [&](uint32_t off, int64_t& w0, int64_t& w1) {
                 if (VEC) {
@@ -191,8 +182,8 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
                 int n = __ldg(g.steps + 2 * b + h);
                 const int64_t neg = SIGN && (h == 0 || v1) ? __ldg(g.negcnt + (h ? c1 : c0)) : 0;
                 dn[h] = Two{neg, neg};
-                for (; n > 8; n -= 8, sp += 32) pair_group<SIGN>(xp, __ldg(sp), 8, dn[h]);
-                pair_group<SIGN>(xp, __ldg(sp), n, dn[h]);
+                for (; n > 8; n -= 8, sp += 32) pair_group<SIGN>(xs32, __ldg(sp), 8, dn[h]);
+                pair_group<SIGN>(xs32, __ldg(sp), n, dn[h]);
                 if (!SIGN && g.sign < 0) dn[h] = Two{-dn[h].a, -dn[h].b};
             }
             // up sums (added to the down sums where one product serves both)
@@ -206,20 +197,20 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 if (r == 1 && !has1) break;
-                const int len = rows[2 * p + r].len, npos = rows[2 * p + r].npos;
+                const int len = rows[r].len, npos = rows[r].npos;
                 int64_t s0 = 0, s1 = 0;
                 int k = 0;
 #pragma unroll 4
                 for (; k < npos; ++k) {
                     int64_t w0, w1;
-                    get(uo[r][k], w0, w1);
+                    get(uoff[r][k], w0, w1);
                     s0 += w0;
                     s1 += w1;
                 }
 #pragma unroll 4
                 for (; k < len; ++k) {
                     int64_t w0, w1;
-                    get(uo[r][k], w0, w1);
+                    get(uoff[r][k], w0, w1);
                     s0 -= w0;
                     s1 -= w1;
                 }
@@ -232,12 +223,12 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
                 if (h == 1 && !v1) break;
                 const uint32_t c = h ? c1 : c0;
                 int64_t xr[2];
-                lds2(xp + pair_slot(c) * 16u, xr[0], xr[1]);
+                lds2(xs32 + pair_slot(c) * 16u, xr[0], xr[1]);
                 const int64_t ddn = __ldg(a.dDNq + c);
                 const uint64_t std_ = __ldg(a.stDN + c) & a.mask;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const PairRow& R = rows[2 * p + (has1 ? r : 0)];
+                    const PairRow& R = rows[has1 ? r : 0];
                     const int64_t x = xr[r], us = r ? up[h].b : up[h].a, ds = r ? dn[h].b : dn[h].a;
                     const int64_t dq = R.du + ddn + a.Uq * (int64_t)__popcll(R.st & std_);
                     if (OUT == 1 && fold) {
@@ -286,10 +277,9 @@ int pair_smem_bytes(int64_t zbase) {
 template <int OUT, bool VEC, bool MERGE>
 static cudaError_t launch_pair3(const ed_op* op, const MvArgs& a, cudaStream_t s) {
     auto kern = op->pair_args.sign == 0 ? k_mv_pair<OUT, VEC, true, MERGE> : k_mv_pair<OUT, VEC, false, MERGE>;
-    const int smem = op->pair_smem * op->pair_rows;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->pair_smem);
     if (e != cudaSuccess) return e;
-    kern<<<op->pair_grid, op->pair_threads, smem, s>>>(a, op->pair_args, op->pair_rows);
+    kern<<<op->pair_grid, op->pair_threads, op->pair_smem, s>>>(a, op->pair_args);
     return cudaGetLastError();
 }
 
