@@ -293,14 +293,12 @@ static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
     op->pair_smem = ed::pair_smem_bytes(g.zbase);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
-    // two CTAs of 512 threads an SM where their rows fit, else one of 1,024.
-    // Staging two pairs a CTA (fewer barriers) cost more than it saved: the
-    // schedule words then miss the L1 that the shared memory leaves (14-site 7+7
-    // 188 against 164 us); 384, 448 or 640 threads, or three or four smaller
-    // CTAs, were slower or the same
-    const bool two = op->pair_smem <= 110 * 1024;
-    op->pair_threads = two ? 512 : 1024;
-    op->pair_grid = two ? 2 * sms : sms;
+    // one CTA of 1,024 threads an SM; two row pairs in shared memory where they
+    // fit (dim_dn up to 7,032: 14- and 15-site sectors), the second staged while
+    // the first is summed
+    op->pair_nbuf = 2 * op->pair_smem <= ed::kPairMaxSmem ? 2 : 1;
+    op->pair_threads = 1024;
+    op->pair_grid = sms;
     op->pair = true;
     return ED_OK;
 }

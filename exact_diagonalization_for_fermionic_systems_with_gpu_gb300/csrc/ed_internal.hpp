@@ -201,7 +201,7 @@ struct ed_op {
     // row-pair matvec
     bool pair = false;
     ed::PairArgs pair_args{};
-    int pair_smem = 0, pair_threads = 0, pair_grid = 0;
+    int pair_smem = 0, pair_nbuf = 1, pair_threads = 0, pair_grid = 0;  // bytes of a row pair, pairs staged, launch
     uint16_t* d_pairWords = nullptr;
     uint8_t *d_pairSteps = nullptr, *d_pairNeg = nullptr;
     std::string last_error;
@@ -232,6 +232,7 @@ int tma_grid(const ed_op* op);
 void row_plan(const SpinTable& up, int G, std::vector<uint32_t>* start, std::vector<uint32_t>* list,
               std::vector<uint32_t>* queue, double w = -1.0);
 // Shared memory of a row pair of zbase + 8 slots (0: does not fit).
+constexpr int kPairMaxSmem = 220 * 1024;
 int pair_smem_bytes(int64_t zbase);
 cudaError_t launch_matvec_pair(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
 cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, cudaStream_t s);

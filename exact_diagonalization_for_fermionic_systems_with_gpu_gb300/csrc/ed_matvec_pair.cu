@@ -11,15 +11,24 @@
 // of both rows: down sums from shared memory, then the up neighbours of each
 // row with 16-byte loads of its column pair (dim_dn even; two 8-byte loads
 // otherwise), the diagonal, one rounding, and the Lanczos partials.
-// The next pair's rows are prefetched into L2 meanwhile.
+// Where two pairs fit in shared memory the last warp stages the next one with
+// 8-byte asynchronous copies (each row is contiguous, the pair is not) while the
+// other 31 compute, with a full and an empty barrier a buffer: units of 64 columns
+// go round the computing warps across pairs, so that no warp waits at the end of
+// a pair for the slowest (54 units on 16 warps: four rounds for 3.4).  Longer rows
+// are staged by all threads between two barriers; the next pair is prefetched into
+// L2 meanwhile.
 //
 // Measured against the one-thread-per-element kernel it replaces there (Lanczos
-// matvec): 14-site chain 7+7 230 -> 164 us, 14-site 7+6 237 -> 144 us, 15-site
-// 7+8 1,470 -> 609 us, 16-site 8+8 6,300 -> 2,530 us.  242 instructions an output
-// at 44 % of the issue slots: bound by the latency of the up loads and the
-// schedule words (32 warps an SM at 64 registers) and by the barriers at the
-// ends of the staged rows.  Loading the words and the first up
-// loads ahead of the sums (74 to 90 registers, 24 or 20 warps) was slower.
+// matvec): 14-site chain 7+7 230 -> 142 us, 14-site 7+6 237 -> 134 us, 15-site
+// 7+8 1,470 -> 516 us, 16-site 8+8 6,300 -> 2,515 us (with one pair a CTA, two CTAs
+// of 512 threads and barriers around each pair: 160, 144, 606 and 2,530 us).
+// About 240 instructions an output at half of the issue slots (16 sites: 40 %):
+// bound by the latency of the up loads and the schedule words (32 warps an SM at
+// 64 registers).  Loading the words and the first up loads ahead of the sums (74 to
+// 90 registers, 24 or 20 warps), prefetching the up neighbours of a warp's next
+// unit into L2 (16-site 2,530 -> 2,650 us) and batching the up loads' remainders
+// were slower or the same.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +37,7 @@
 #include "ed_device.cuh"
 #include "ed_internal.hpp"
 #include "ed_matvec_common.cuh"
+#include "ed_matvec_tma.cuh"
 
 namespace ed {
 using namespace dev;
@@ -35,7 +45,6 @@ using namespace dev;
 namespace {
 
 constexpr int kPairUp = 256;  // up entries staged per row (the longest row has 255)
-constexpr int kPairMaxSmem = 220 * 1024;
 
 struct Two {
     int64_t a, b;  // rows u, u + 1
@@ -45,6 +54,14 @@ struct Two {
 // barriers around the staged rows)
 __device__ __forceinline__ void lds2(uint32_t addr, int64_t& x, int64_t& y) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(addr));
+}
+
+__device__ __forceinline__ void cp_async8(uint32_t dst, const int64_t* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tma::smem_u32(bar)) : "memory");
 }
 
 // One step of both rows: slot word w (low 15 bits; sign in bit 15).
@@ -102,17 +119,20 @@ struct PairRow {
 // OUT = 0: FP64 y; OUT = 1: FX u with the Lanczos epilogue.  VEC: dim_dn even,
 // lane l has columns 2l, 2l + 1 of a 64-column block; otherwise l, l + 32.
 // MERGE: equal hopping coefficients, one product for the up and down sums.
+// nbuf: row pairs in shared memory (2: the last warp stages, 1: all do).
 template <int OUT, bool VEC, bool SIGN, bool MERGE>
-__global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g) {
+__global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g, const int nbuf) {
     extern __shared__ __align__(128) unsigned char xs[];
-    __shared__ uint32_t uoff[2][kPairUp];
-    __shared__ PairRow rows[2];
+    __shared__ uint32_t uoff_s[2][2][kPairUp];
+    __shared__ PairRow rows_s[2][2];
+    __shared__ uint64_t full[2], empty[2];
     const uint32_t dimUP = (uint32_t)a.dimUP, dimDN = (uint32_t)a.dimDN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int nc = nbuf == 1 ? nwarps : nwarps - 1;  // computing warps
     const int64_t* __restrict__ xq = a.xq;
     const uint4* __restrict__ words = reinterpret_cast<const uint4*>(g.words);
-    const uint32_t xs32 = (uint32_t)__cvta_generic_to_shared(xs);
-    longlong2* const x2 = reinterpret_cast<longlong2*>(xs);
+    const uint32_t xs_base = (uint32_t)__cvta_generic_to_shared(xs);
+    const uint32_t pair_bytes = (uint32_t)(g.zbase + 8) * 16u;
     int E_out = 0, s_u = 0;
     if (OUT == 0) {
         E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
@@ -125,41 +145,77 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
     const bool y16 = OUT == 1 || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;  // y may start on any double
     i128 dot = 0;
     uint64_t mx = 0;
-    if (tid < 8) x2[g.zbase + tid] = make_longlong2(0, 0);
+    if (tid < 8 * nbuf)
+        *reinterpret_cast<longlong2*>(xs + (tid >> 3) * pair_bytes + (g.zbase + (tid & 7)) * 16) = make_longlong2(0, 0);
+    if (tid == 0) {
+        for (int k = 0; k < 2; ++k) {
+            tma::mbar_init(&full[k], 64);
+            tma::mbar_init(&empty[k], nc);
+        }
+        tma::fence_mbar_init();
+    }
+    __syncthreads();
     const uint32_t npairs = (dimUP + 1) / 2;
-    for (uint32_t it = blockIdx.x; it < npairs; it += gridDim.x) {
+    int buf = 0;
+    uint32_t parity = 0;  // of the buffer's current use
+    // row pair `it` into buffer k: thread i of n
+    auto stage = [&](uint32_t it, int k, uint32_t i0, uint32_t n) {
         const uint32_t u0 = 2 * it;
         const int nrow = u0 + 1 < dimUP ? 2 : 1;  // an odd count ends on a pair of one row
-        const bool has1 = nrow == 2;
-        __syncthreads();  // the previous rows are no longer read
         for (int r = 0; r < nrow; ++r) {
             const uint32_t u = u0 + r, q0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - q0;
-            for (uint32_t k = tid; k < len; k += blockDim.x) uoff[r][k] = (__ldg(a.upEntC + q0 + k) & kColMask) * dimDN;
-            if (tid == r) rows[r] = {__ldg(a.stUP + u), __ldg(a.dUPq + u), (int)len, (int)__ldg(a.upNpos + u)};
+            for (uint32_t i = i0; i < len; i += n) uoff_s[k][r][i] = (__ldg(a.upEntC + q0 + i) & kColMask) * dimDN;
+            if (i0 == r) rows_s[k][r] = {__ldg(a.stUP + u), __ldg(a.dUPq + u), (int)len, (int)__ldg(a.upNpos + u)};
         }
         const int64_t* const r0 = xq + (size_t)u0 * dimDN;
-        const int64_t* const r1 = has1 ? r0 + dimDN : r0;
-        if (VEC) {
-#pragma unroll 2
-            for (uint32_t c = 2 * tid; c < dimDN; c += 2 * blockDim.x) {
-                const longlong2 v0 = __ldg(reinterpret_cast<const longlong2*>(r0 + c));
-                const longlong2 v1 = __ldg(reinterpret_cast<const longlong2*>(r1 + c));
-                x2[pair_slot(c)] = make_longlong2(v0.x, v1.x);
-                x2[pair_slot(c + 1)] = make_longlong2(v0.y, v1.y);
-            }
-        } else {
+        const int64_t* const r1 = nrow == 2 ? r0 + dimDN : r0;
+        const uint32_t xb = xs_base + k * pair_bytes;
 #pragma unroll 4
-            for (uint32_t c = tid; c < dimDN; c += blockDim.x) x2[pair_slot(c)] = make_longlong2(__ldg(r0 + c), __ldg(r1 + c));
+        for (uint32_t c = i0; c < dimDN; c += n) {
+            const uint32_t d = xb + pair_slot(c) * 16u;
+            cp_async8(d, r0 + c);
+            cp_async8(d + 8, r1 + c);
         }
-        if (tid == 0 && it + gridDim.x < npairs) {
-            // an even row starts on a 16-byte boundary
-            const uint32_t un = 2 * (it + gridDim.x);
-            const uint32_t bytes = (dimDN * (un + 1 < dimUP ? 2u : 1u) * 8u) & ~15u;
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(xq + (size_t)un * dimDN), "r"(bytes)
-                         : "memory");
+    };
+    if (warp == nc) {
+        for (uint32_t it = blockIdx.x; it < npairs; it += gridDim.x) {
+            if (!tma::mbar_wait(&empty[buf], parity ^ 1)) {  // at once in the buffer's first use
+                if (lane == 0) atomicExch(a.err, 1);
+                break;
+            }
+            stage(it, buf, lane, 32);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tma::smem_u32(&full[buf])) : "memory");
+            mbar_arrive(&full[buf]);
+            buf ^= 1;
+            if (buf == 0) parity ^= 1;
         }
-        __syncthreads();
-        for (int b = warp; b < g.blocks; b += nwarps) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    uint32_t b0 = warp;  // this warp's first unit of the item: units go round the computing warps across items
+    for (uint32_t it = warp == nc ? npairs : blockIdx.x; it < npairs; it += gridDim.x) {
+        const uint32_t u0 = 2 * it;
+        const bool has1 = u0 + 1 < dimUP;
+        const uint32_t xs32 = xs_base + buf * pair_bytes;
+        const uint32_t(*uoff)[kPairUp] = uoff_s[buf];
+        const PairRow* const rows = rows_s[buf];
+        if (nbuf == 1) {
+            __syncthreads();  // the previous rows are no longer read
+            stage(it, 0, tid, blockDim.x);
+            if (tid == 0 && it + gridDim.x < npairs) {
+                // an even row starts on a 16-byte boundary
+                const uint32_t un = 2 * (it + gridDim.x);
+                const uint32_t bytes = (dimDN * (un + 1 < dimUP ? 2u : 1u) * 8u) & ~15u;
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(xq + (size_t)un * dimDN), "r"(bytes)
+                             : "memory");
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+        } else if (!tma::mbar_wait(&full[buf], parity)) {
+            if (lane == 0) atomicExch(a.err, 1);
+            break;
+        }
+        int b = b0;
+        for (; b < g.blocks; b += nc) {
             const uint32_t c0 = 64u * b + (VEC ? 2u * lane : (uint32_t)lane), c1 = VEC ? c0 + 1 : c0 + 32;
             if (c0 >= dimDN) continue;
             const bool v1 = VEC || c1 < dimDN;  // the second column exists
@@ -265,6 +321,13 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
                 }
             }
         }
+        if (nbuf == 2) {
+            b0 = b - g.blocks;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[buf]);
+            buf ^= 1;
+            if (buf == 0) parity ^= 1;
+        }
     }
     if (OUT == 1) mv_lanczos_epilogue(a, dot, mx, s_u);
 }
@@ -277,9 +340,9 @@ int pair_smem_bytes(int64_t zbase) {
 template <int OUT, bool VEC, bool MERGE>
 static cudaError_t launch_pair3(const ed_op* op, const MvArgs& a, cudaStream_t s) {
     auto kern = op->pair_args.sign == 0 ? k_mv_pair<OUT, VEC, true, MERGE> : k_mv_pair<OUT, VEC, false, MERGE>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->pair_smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->pair_nbuf * op->pair_smem);
     if (e != cudaSuccess) return e;
-    kern<<<op->pair_grid, op->pair_threads, op->pair_smem, s>>>(a, op->pair_args);
+    kern<<<op->pair_grid, op->pair_threads, op->pair_nbuf * op->pair_smem, s>>>(a, op->pair_args, op->pair_nbuf);
     return cudaGetLastError();
 }
 

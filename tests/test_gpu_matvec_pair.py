@@ -62,3 +62,32 @@ def test_pair_matvec_matches_generic(ed, monkeypatch, case):
         op.close()
     assert runs["pair"][0] == runs["generic"][0]
     assert np.array_equal(runs["pair"][1], runs["generic"][1])
+
+
+# several row pairs a block: fewer 64-column units than computing warps, a
+# remainder of units carried from pair to pair, and rows too long for two
+# pairs in shared memory (even and odd)
+@pytest.mark.parametrize("N,qu,qd", [(12, 6, 2), (13, 6, 4), (14, 6, 7), (15, 4, 6), (16, 4, 8), (23, 3, 4)])
+def test_pair_matvec_many_pairs_a_block(ed, monkeypatch, N, qu, qd):
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    terms = L.chain(N, periodic=N % 2 == 1)
+    ops = {}
+    for kind in ("pair", "generic"):
+        monkeypatch.setenv("ED_MATVEC", kind)
+        ops[kind] = ed.Hubbard(ed.H_TBq(N, qu).extend(terms), ed.H_TBq(N, qd).extend(terms), 2.0)
+    n = ops["pair"].rows()
+    x = torch.from_numpy(np.random.default_rng(6).standard_normal(n)).cuda()
+    ys, runs = {}, {}
+    for k, op in ops.items():
+        y = torch.empty(n, dtype=torch.float64, device="cuda")
+        op.Hubbard_mv(x, y)
+        ys[k] = y
+        lz = ed.Lanczos()
+        e, v = lz.eigen(op, max_steps=5, mode="fixed", seed=2)
+        runs[k] = (e, lz.a, lz.b, lz.result.min_bits, lz.result.status), v
+    assert torch.equal(ys["pair"], ys["generic"])
+    assert runs["pair"][0] == runs["generic"][0]
+    assert np.array_equal(runs["pair"][1], runs["generic"][1])
+    for op in ops.values():
+        op.close()
