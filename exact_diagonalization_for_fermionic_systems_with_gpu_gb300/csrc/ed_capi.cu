@@ -276,6 +276,22 @@ static ed_status plan_striped(ed_op* op, bool forced, int64_t chunk_cap = 16384)
     return ED_OK;
 }
 
+// Real single-class sectors: the row-pair kernel where the row engine's tables
+// leave it no shared memory (from about 3,000 down states), and for vectors that
+// are large enough to pay for its launches where they do.  A Lanczos step (100
+// steps, open chains), row engine -> pairs, with two row CTAs an SM: 14-site 7+4
+// (3.4 M elements) 88 -> 95 us, 15-site 5+4 (4.1 M) 104 -> 98, 16-site 6+3 (4.5 M)
+// 152 -> 139, 15-site 7+4 (8.8 M) 214 -> 186; with one, whose 16 warps leave the
+// loads' latency open: 13-site 4+6 (1.2 M) 47 -> 47, 15 sites in a 3 x 5 torus 4+4
+// (1.9 M) 86 -> 71, 14-site 4+5 (2.0 M) 64 -> 63, 13-site 5+6 (2.2 M) 76 -> 63,
+// 13-site 6+6 (2.9 M) 102 -> 74, 16-site 8+4 (23 M) 894 -> 413.
+static bool prefer_pair(const ed_op* op) {
+    if (op->tma_smem == 0) return true;
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
+    return op->D >= (op->tma_grid >= 2 * sms ? 4000000 : 1500000);
+}
+
 // Plans and uploads the row-pair matvec where two rows fit shared memory;
 // leaves op->pair false otherwise.
 static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
@@ -673,9 +689,8 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     const char* pick = std::getenv("ED_MATVEC");
     const std::string want = pick ? pick : "";
     if (want != "generic" && want != "striped" && want != "pair") op->tma_smem = ed::tma_plan(op, &a);
-    // real single-class sectors whose tables leave no room for that plan but
-    // where two rows fit (3,000 to 14,000 down states): the row-pair kernel
-    if (op->tma_smem == 0 && (want.empty() || want == "pair") && !cplx && op->mv_fast) {
+    if (op->tma_smem > 0) op->tma_grid = ed::tma_grid(op);
+    if (!cplx && op->mv_fast && (want.empty() || want == "pair") && prefer_pair(op)) {
         const ed_status pst = plan_pair(op, desc->dn_terms, desc->n_dn_terms);
         if (pst != ED_OK) {
             ed_op_destroy(op);
@@ -693,7 +708,6 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         }
     }
     if (op->tma_smem > 0) {
-        op->tma_grid = ed::tma_grid(op);
         std::vector<uint32_t> rs, rl, rq;
         ed::row_plan(op->tup, op->tma_grid, &rs, &rl, &rq);
         const std::vector<uint32_t> uq = ed::unit_queue(rq, op->dimDN, op->tma_grid);
@@ -711,7 +725,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         op->mv.rowQueue = op->d_rowQueue;
         op->mv.unitQueue = op->d_unitQueue;
         op->mv.nunits = (uint32_t)uq.size();
-        op->apply_grid = ed::apply_grid(op);
+        op->apply_grid = op->pair ? 0 : ed::apply_grid(op);
     }
     *out = op;
     return ED_OK;

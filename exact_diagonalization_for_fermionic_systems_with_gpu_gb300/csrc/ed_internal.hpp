@@ -185,8 +185,9 @@ struct ed_op {
     bool striped = false;
     int st_grid = 0, st_win = 0, st_chunk = 0, st_zbase = 0;
     int st_s8 = 0;              // groups of eight steps of pass D's schedule (lane-packed layout)
-    // tuning (ed_op_autotune): Lanczos kernels 0 by the default rule, 1 per
-    // step, 2 persistent; weight of the persistent kernel's row queue
+    // tuning (ed_op_autotune): Lanczos kernels 0 by the default rule (persistent
+    // where the row engine serves the sector and no row pairs do), 1 per step,
+    // 2 persistent; weight of the persistent kernel's row queue
     int lz_mode = 0;
     int lz_grid = 0;            // persistent kernel's CTAs (0: tma_grid, two per SM)
     double row_cost = -1.0;

@@ -734,7 +734,10 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     // the autotuner chose the per-step ones.
     const char* fz = std::getenv("ED_LZ_FUSED");
     const bool force = fz && fz[0] == '1', never = fz && fz[0] == '0';
-    bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && (force || op->lz_mode != 1);
+    // Sectors with a row-pair matvec take it, a launch a step, unless a tuned
+    // plan chose the persistent kernel.
+    const bool pick = op->lz_mode == 2 || (op->lz_mode == 0 && !op->pair);
+    bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && (force || pick);
     // Reorthogonalised runs of small sectors: all steps in one cooperative
     // launch (ed_lanczos_reorth.cu).
     bool fused_reorth = cfg->reorth && !op->striped && !prof && !never && max_steps <= kReorthMaxSteps &&

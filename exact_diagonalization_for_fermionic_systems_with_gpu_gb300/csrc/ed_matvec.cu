@@ -344,8 +344,8 @@ cudaError_t launch_matvec_lz(const ed_op* op, const int64_t* xq, int64_t* uq, vo
         if (e == cudaSuccess) e = launch_striped_up(op, a, g, s);
         return e;
     }
-    if (op->tma_smem > 0) return launch_matvec_tma(op, a, s);
     if (op->pair) return launch_matvec_pair(op, a, 1, s);
+    if (op->tma_smem > 0) return launch_matvec_tma(op, a, s);
     return op->cplx ? launch_mv<true, 1>(op, a, s) : launch_mv<false, 1>(op, a, s);
 }
 

@@ -1,7 +1,7 @@
 // ed_matvec_pair.cu — one-launch matvec over pairs of up rows, for real
 // operators with one coefficient class per spin whose down rows are too long
 // for the table-resident row engine (14- to 16-site sectors: 3,000 to 14,000
-// down states).
+// down states), or whose vectors are large (prefer_pair has the sizes).
 //
 // A CTA stages rows u and u + 1 of x interleaved in shared memory, 16 bytes a
 // column, so that one 16-byte load of a down hop serves both rows and one

@@ -91,3 +91,37 @@ def test_pair_matvec_many_pairs_a_block(ed, monkeypatch, N, qu, qd):
     assert np.array_equal(runs["pair"][1], runs["generic"][1])
     for op in ops.values():
         op.close()
+
+
+# sectors that have row-engine tables too: the row-pair kernel by size; the
+# persistent row kernel (forced) and the generic one give the same bits
+@pytest.mark.parametrize("N,qu,qd", [(13, 5, 6), (13, 6, 7), (14, 5, 5), (15, 5, 4), (16, 6, 3)])
+def test_pair_chosen_by_size(ed, monkeypatch, N, qu, qd):
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    terms = L.chain(N, eps=list(philox_uniform(5, N, 2.0)))
+    up, dn = ed.H_TBq(N, qu).extend(terms), ed.H_TBq(N, qd).extend(terms)
+    op = ed.Hubbard(up, dn, 2.0)
+    monkeypatch.setenv("ED_MATVEC", "generic")
+    ref = ed.Hubbard(up, dn, 2.0)
+    monkeypatch.delenv("ED_MATVEC")
+    assert op.matvec_kind == "rows" and ref.matvec_kind == "generic"
+    x = torch.from_numpy(np.random.default_rng(7).standard_normal(op.rows())).cuda()
+    ys = [torch.empty_like(x) for _ in range(2)]
+    op.Hubbard_mv(x, ys[0])
+    ref.Hubbard_mv(x, ys[1])
+    assert torch.equal(ys[0], ys[1])
+    runs = []
+    for o, fused in ((op, None), (op, "1"), (ref, None)):  # two launches a step; one; two
+        if fused:
+            monkeypatch.setenv("ED_LZ_FUSED", fused)
+        lz = ed.Lanczos()
+        e, v = lz.eigen(o, max_steps=6, mode="fixed", seed=3)
+        monkeypatch.delenv("ED_LZ_FUSED", raising=False)
+        assert lz.result.launches >= 12 if fused is None else lz.result.launches < 12
+        runs.append(((e, lz.a, lz.b, lz.result.min_bits, lz.result.status), v))
+    for r in runs[1:]:
+        assert r[0] == runs[0][0]
+        assert np.array_equal(r[1], runs[0][1])
+    op.close()
+    ref.close()
