@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const 
     const int tid = threadIdx.x;
     const int64_t gt = (int64_t)blockIdx.x * kTmaThreads + tid, GT = (int64_t)gridDim.x * kTmaThreads;
     uint32_t u0 = 0;
-    const bool has_row = tma_first_row_dyn<!CPLX>(a, &u0);
+    const bool has_row = tma_first_row_dyn<true>(a, &u0);
     if (tid == 0) {
         tma_init(S);
         tma_issue_tables(a, S);
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const 
     uint32_t rc = 0;
     i128 dot = 0;
     uint64_t mx = 0;
-    tma_rows<CPLX, 0, FAST, true, SCHED, true, SEG, false, !CPLX>(a, S, f.xq, nullptr, a.y, rc, E - a.Fc, 0, dot, mx,
+    tma_rows<CPLX, 0, FAST, true, SCHED, true, SEG, false, true>(a, S, f.xq, nullptr, a.y, rc, E - a.Fc, 0, dot, mx,
                                                                   f.taken, &s_next);
 }
 
@@ -167,7 +167,7 @@ int apply_grid(const ed_op* op) {
         return 0;
     }
     // a CTA for every unit of work, as many as are resident together
-    const int64_t units = op->cplx ? op->dimUP : (int64_t)op->mv.nunits;
+    const int64_t units = op->mv.nunits;
     const int64_t g = std::min<int64_t>({(int64_t)per_sm * sms, op->tma_grid, std::max<int64_t>(units, 1), kApplyPart});
     return coop ? (int)g : 0;
 }

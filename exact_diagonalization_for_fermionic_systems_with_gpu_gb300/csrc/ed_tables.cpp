@@ -732,11 +732,18 @@ bool build_class_schedule(const SpinTable& t, ClassSchedule* g, std::string* err
 
 std::vector<uint32_t> unit_queue(const std::vector<uint32_t>& rq, int64_t dimDN, int G) {
     const size_t k = G > 0 ? rq.size() % (size_t)G : 0;
-    // parts of a multiple of 32 columns, every one of them non-empty
+    // Up to four parts of a multiple of 32 columns, every one of them non-empty,
+    // while every CTA takes at most one (a part costs a row's fixed latency, so two
+    // parts in turn take longer than one row: 11-site 5+5, 158 rows over 304 CTAs,
+    // in four 19.0, whole 16.9 us a step; 12-site 5+5 28.0 -> 26.0; 10-site 6+3
+    // 17.1 -> 13.5) and the part keeps 224 columns (11-site 4+4, 26 rows of 330,
+    // in four 15.5, whole 14.4; 12-site 6+6, 12 rows of 924, in four 28.4, whole
+    // 28.6, on Kagome 33.8 and 34.8).
+    constexpr int64_t kMinPart = 224;
     int lg = 2;
     while (lg > 0) {
         const int64_t P = (int64_t)1 << lg, ch = ((dimDN + P - 1) / P + 31) / 32 * 32;
-        if ((P - 1) * ch < dimDN) break;
+        if ((P - 1) * ch < dimDN && dimDN >= P * kMinPart && (int64_t)(k << lg) <= G) break;
         --lg;
     }
     if (k == 0 || lg == 0) return rq;

@@ -139,7 +139,8 @@ bool build_gather_schedule32(const SpinTable& t, const std::vector<uint32_t>& pe
 
 // The persistent Lanczos kernel's unit queue from a row queue rq for G CTAs:
 // the rows past the last full wave (rq.size() mod G of them, the cheapest)
-// each split into up to four column ranges.  An entry is a row, or
+// each split into up to four column ranges where there are CTAs for them and the
+// ranges stay wide.  An entry is a row, or
 // row | part << 24 | log2(P) << 28 for part `part` of P: columns
 // [part ch, min(dimDN, (part + 1) ch)) with ch = ceil(ceil(dimDN / P) / 32) 32,
 // every part non-empty (P = 1, no split, when dimDN is too narrow).  At most

@@ -171,3 +171,39 @@ def test_complex_class_sums_match_generic(ed, monkeypatch, case):
     for other in runs[1:]:
         assert other[:3] == runs[0][:3]
         assert np.array_equal(other[3], runs[0][3])
+
+
+# the last rows of the unit queue split into two or four column ranges, and
+# whole where their ranges would be narrow or more than the grid: apply and
+# persistent Lanczos against the generic kernel
+@pytest.mark.parametrize("N,qu,qd,flux", [(12, 2, 6, 0.3), (12, 2, 4, 0.3), (12, 6, 6, 0.3), (12, 4, 6, 0.3), (8, 4, 4, 0.2),
+                                          (12, 2, 6, 0.0), (13, 2, 4, 0.0), (11, 4, 4, 0.0), (10, 6, 3, 0.0)])
+def test_split_rows_match_generic(ed, monkeypatch, N, qu, qd, flux):
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    if flux and N == 12:
+        t = L.kagome12(flux=flux, peierls=True)
+    else:
+        t = [("P" if flux else "H", i, (i + 1) % N, -1.0, flux) for i in range(N)]
+    up, dn = ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t)
+    ops = [ed.Hubbard(up, dn, 4.0)]
+    monkeypatch.setenv("ED_MATVEC", "generic")
+    ops.append(ed.Hubbard(up, dn, 4.0))
+    monkeypatch.delenv("ED_MATVEC")
+    assert [op.matvec_kind for op in ops] == ["rows", "generic"]
+    n = ops[0].rows()
+    dt = torch.complex128 if flux else torch.float64
+    x = torch.from_numpy(np.random.default_rng(8).standard_normal(n)).to(dt).cuda()
+    x *= (1.0 - 2.0j) if flux else 1.0
+    ys, runs = [], []
+    for op in ops:
+        y = torch.empty_like(x)
+        op.Hubbard_mv(x, y)
+        ys.append(y)
+        lz = ed.Lanczos()
+        e, v = lz.eigen(op, max_steps=12, mode="fixed", seed=2)
+        runs.append(((e, lz.a, lz.b, lz.result.min_bits, lz.result.status), v))
+        op.close()
+    assert torch.equal(ys[0], ys[1])
+    assert runs[0][0] == runs[1][0]
+    assert np.array_equal(runs[0][1], runs[1][1])
