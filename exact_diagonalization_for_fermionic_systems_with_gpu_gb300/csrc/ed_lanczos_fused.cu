@@ -209,24 +209,25 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
         // step's last barrier (the load's latency hides behind the axpy)
         int host_stop = 0;
         if (f.mirror && blockIdx.x == 0 && tid == 0) host_stop = ld_relaxed_sys(&f.mirror->stop);
-        if (tid == 0) {
+        if (tid < 32) {
             if (stamp) st[3] = global_ns();
             i128 s;
             uint64_t m;
             red_pull(&f.red[rM % 4], s, m);
-            if (blockIdx.x == 0) {
-                if (rM >= 2) f.red[(rM - 2) % 4] = LzRedSet{0, 0, 0, 0};
-                // the other queue counter was last taken from in step j-1 and
-                // is next taken from in step j+1, after the next barrier
-                f.taken[(j + 1) & 1] = 0;
-            }
             const int e_u = sX.e - a.Fc + s_u;
-            s_coef = lz_coefs(j, s, e_u, m, sX.e, sX.m, sX.beta, sX.ib, sP.e, sP.m, sP.ib, s_status);
-            if (blockIdx.x == 0) {
-                lz->s_u = s_u;
-                lz->e_u = e_u;
-                lz->m_u = m;
-                lz_store_coefs(lz, j, s_coef);
+            const LzCoefs c = lz_coefs_warp(j, s, e_u, m, sX.e, sX.m, sX.beta, sX.ib, sP.e, sP.m, sP.ib, s_status);
+            if (tid == 0) {
+                s_coef = c;
+                if (blockIdx.x == 0) {
+                    if (rM >= 2) f.red[(rM - 2) % 4] = LzRedSet{0, 0, 0, 0};
+                    // the other queue counter was last taken from in step j-1 and
+                    // is next taken from in step j+1, after the next barrier
+                    f.taken[(j + 1) & 1] = 0;
+                    lz->s_u = s_u;
+                    lz->e_u = e_u;
+                    lz->m_u = m;
+                    lz_store_coefs(lz, j, c);
+                }
             }
             if (stamp) st[4] = global_ns();
         }

@@ -273,21 +273,24 @@ __global__ void __launch_bounds__(kRoThreads, 1) k_lz_reorth_run(const MvArgs a,
             if (tid == 0) red_push(&red[0], dot, mx);
         }
         if (!grid_sync(f.gbar, target, &give_up, a.err, f.wait)) return;
-        if (tid == 0) {
+        if (tid < 32) {
             i128 s;
             uint64_t m;
             red_pull(&red[0], s, m);
-            // the other parity's sets were last read before this barrier
-            if (blockIdx.x == 0)
-                for (int r = 0; r < 3; ++r) f.red[3 * ((j + 1) & 1) + r] = LzRedSet{0, 0, 0, 0};
             const int e_u = s_e[0] - a.Fc + s_u;
-            s_coef = lz_coefs(j, s, e_u, m, s_e[0], s_m[0], s_beta[0], s_ib[0], s_e[1], s_m[1], s_ib[1], s_status);
-            if (store) {
-                lz->s_u = s_u;
-                lz->e_u = e_u;
-                lz->m_u = m;
-                lz_store_coefs(lz, j, s_coef);
-                lz->e[j + 1] = s_coef.e_w;
+            const LzCoefs c = lz_coefs_warp(j, s, e_u, m, s_e[0], s_m[0], s_beta[0], s_ib[0], s_e[1], s_m[1], s_ib[1], s_status);
+            if (tid == 0) {
+                s_coef = c;
+                // the other parity's sets were last read before this barrier
+                if (blockIdx.x == 0)
+                    for (int r = 0; r < 3; ++r) f.red[3 * ((j + 1) & 1) + r] = LzRedSet{0, 0, 0, 0};
+                if (store) {
+                    lz->s_u = s_u;
+                    lz->e_u = e_u;
+                    lz->m_u = m;
+                    lz_store_coefs(lz, j, c);
+                    lz->e[j + 1] = c.e_w;
+                }
             }
         }
         __syncthreads();
