@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
         if (f.mirror && blockIdx.x == 0 && j == 0) mirror_slot(f.mirror, lz, 0);
     }
     if (SCHED || (CPLX && SEG)) tma_zero_slots(a, S);
+    if (FAST && has_row && tid >= 32 && tid < 64) tma_stage_up(a, u0, uoff, tid - 32, 32);
     __syncthreads();
     if (!tma::mbar_wait(&S.bar[2], 0)) {
         if (tid == 0) atomicExch(a.err, 1);
@@ -195,13 +196,15 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_lz_fused(const MvArgs a, con
         {
             i128 dot = 0;
             uint64_t mx = 0;
-            tma_rows<CPLX, 1, FAST, true, SCHED, true, SEG, false, true>(a, S, xq, f.u, nullptr, rc, 0, s_u, dot, mx,
+            tma_rows<CPLX, 1, FAST, true, SCHED, true, SEG, false, true, FAST>(a, S, xq, f.u, nullptr, rc, 0, s_u, dot, mx,
                                                        f.taken + (j & 1), &s_next);
             if (give_up) return;
             if (stamp) st[1] = global_ns();
             if (f.cta_stamps && tid == 0) f.cta_stamps[(size_t)j * 2 * G + blockIdx.x] = global_ns();
             block_sum_max(dot, mx, s128, s64);
             if (tid == 0) red_push(&f.red[rM % 4], dot, mx);
+            // the first row's up offsets, for the next step
+            if (FAST && has_row && tid >= 32 && tid < 64) tma_stage_up(a, u0, uoff, tid - 32, 32);
             if (stamp) st[2] = global_ns();
         }
         if (!grid_sync(f.gbar, target, &give_up, a.err, f.wait)) return;

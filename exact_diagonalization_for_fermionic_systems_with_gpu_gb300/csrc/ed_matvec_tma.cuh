@@ -298,6 +298,12 @@ __device__ __forceinline__ void class_products(i128& ar, i128& ai, const ClassSu
     one(s3, 3);
 }
 
+// Up offsets of row u into uo: thread i of n.
+__device__ __forceinline__ void tma_stage_up(const MvArgs& a, uint32_t u, uint32_t* uo, uint32_t i, uint32_t n) {
+    const uint32_t p0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - p0, dimDN = (uint32_t)a.dimDN;
+    for (uint32_t k = i; k < len; k += n) uo[k] = (__ldg(a.upEntC + p0 + k) & kColMask) * dimDN;
+}
+
 // First row of this CTA (rowList[rowStart[b]]); false when it has none.
 __device__ __forceinline__ bool tma_first_row(const MvArgs& a, uint32_t* u) {
     const uint32_t r0 = __ldg(a.rowStart + blockIdx.x);
@@ -330,8 +336,9 @@ __device__ __forceinline__ bool tma_first_row_dyn(const MvArgs& a, uint32_t* u) 
 // GDIAG: the folded down diagonal is read from a.dDNq in global memory
 // instead of the staged copy (instances that share staged tables but not
 // their on-site terms, k_lz_multi).
+// PRE: the caller has staged the first row's up offsets in S.uoff (FAST).
 template <bool CPLX, int OUT, bool FAST, bool COH, bool SCHED, bool DYN, bool SEG = false, bool GDIAG = false,
-          bool SPLIT = false>
+          bool SPLIT = false, bool PRE = false>
 __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, const int64_t* __restrict__ xq,
                                          int64_t* __restrict__ uq, double* __restrict__ y, uint32_t& rc, int E_out,
                                          int s_u, i128& dot, uint64_t& mx, unsigned int* taken = nullptr,
@@ -351,6 +358,8 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
     // then keep no thread from that barrier.
     const int qt = T - 1;
     const uint32_t r1 = DYN ? nq : __ldg(a.rowStart + blockIdx.x + 1);
+    uint32_t ub = 0;      // FAST: which of uoff, uent holds the row's up offsets
+    bool staged = PRE;
     for (uint32_t r = DYN ? blockIdx.x : __ldg(a.rowStart + blockIdx.x); r < r1; ++rc) {
         const uint32_t qe = DYN ? __ldg(queue + r) : __ldg(a.rowList + r);
         const uint32_t u = SPLIT ? (qe & 0xFFFFFFu) : qe;
@@ -368,10 +377,13 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
         if (DYN && tid == qt) taken_at = atomicAdd(taken, 1u);  // consumed after the barrier
         const uint32_t p0 = __ldg(a.upPtr + u), lenU = __ldg(a.upPtr + u + 1) - p0;
         const int nposU = FAST ? (int)__ldg(a.upNpos + u) : 0;
-        for (uint32_t k = tid; k < lenU; k += T) {
-            const uint32_t e = __ldg(a.upEntC + p0 + k);
-            S.uoff[k] = (e & kColMask) * dimDN;
-            S.uent[k] = e;
+        uint32_t* const uo = FAST && ub ? S.uent : S.uoff;
+        if (!staged) {
+            for (uint32_t k = tid; k < lenU; k += T) {
+                const uint32_t e = __ldg(a.upEntC + p0 + k);
+                uo[k] = (e & kColMask) * dimDN;
+                if (!FAST) S.uent[k] = e;
+            }
         }
         if (!tma::mbar_wait(&S.bar[buf], parity)) {
             if (tid == 0) atomicExch(a.err, 1);
@@ -391,14 +403,20 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
             return;
         }
         // prefetch the next row into the other buffer (its readers finished
-        // at the barrier that closed the previous iteration)
-        if (tid == qt) {
-            const uint32_t rn = DYN ? gridDim.x + taken_at : r + 1;
-            if (DYN) *snext = rn;
+        // at the barrier that closed the previous iteration); in the
+        // single-class kernel the same warp stages that row's up offsets, two
+        // dependent L2 reads that kept every thread from the next row's sums
+        // (Kagome12 6+6 step 32.8 -> 32.2 us)
+        if (tid >= qt - 31) {
+            const uint32_t rn = DYN ? gridDim.x + __shfl_sync(0xffffffffu, taken_at, 31) : r + 1;
+            if (DYN && tid == qt) *snext = rn;
             if (rn < r1) {
                 const uint32_t un = DYN ? (__ldg(queue + rn) & (SPLIT ? 0xFFFFFFu : 0xFFFFFFFFu)) : __ldg(a.rowList + rn);
-                tma::fence_proxy_async_smem();
-                tma_issue_row<CPLX>(a, S, xq, un, buf ^ 1);
+                if (tid == qt) {
+                    tma::fence_proxy_async_smem();
+                    tma_issue_row<CPLX>(a, S, xq, un, buf ^ 1);
+                }
+                if (FAST) tma_stage_up(a, un, ub ? S.uoff : S.uent, tid & 31, 32);
             }
         }
         const int64_t* xrow = (buf ? S.row1 : S.row0) + tma_row_off<CPLX>(a, u);
@@ -418,21 +436,21 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
                 if (v1) {
 #pragma unroll 4
                     for (; k < nposU; ++k) {
-                        const uint32_t o = S.uoff[k];
+                        const uint32_t o = uo[k];
                         acc_up<CPLX, COH>(xq, o + d0, upr0, upi0);
                         acc_up<CPLX, COH>(xq, o + d1, upr1, upi1);
                     }
 #pragma unroll 4
                     for (; k < (int)lenU; ++k) {
-                        const uint32_t o = S.uoff[k];
+                        const uint32_t o = uo[k];
                         acc_up<CPLX, COH>(xq, o + d0, unr0, uni0);
                         acc_up<CPLX, COH>(xq, o + d1, unr1, uni1);
                     }
                 } else {
 #pragma unroll 4
-                    for (; k < nposU; ++k) acc_up<CPLX, COH>(xq, S.uoff[k] + d0, upr0, upi0);
+                    for (; k < nposU; ++k) acc_up<CPLX, COH>(xq, uo[k] + d0, upr0, upi0);
 #pragma unroll 4
-                    for (; k < (int)lenU; ++k) acc_up<CPLX, COH>(xq, S.uoff[k] + d0, unr0, uni0);
+                    for (; k < (int)lenU; ++k) acc_up<CPLX, COH>(xq, uo[k] + d0, unr0, uni0);
                 }
                 int64_t dr0 = 0, di0 = 0, dr1 = 0, di1 = 0;
                 if (SCHED) {
@@ -745,6 +763,10 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
         }
         __syncthreads();  // row buffer and uoff are free for the next iteration; *snext is written
         r = DYN ? *snext : r + 1;
+        if (FAST) {
+            ub ^= 1;
+            staged = true;
+        }
     }
 }
 
