@@ -280,16 +280,33 @@ static ed_status plan_striped(ed_op* op, bool forced, int64_t chunk_cap = 16384)
 // leave it no shared memory (from about 3,000 down states), and for vectors that
 // are large enough to pay for its launches where they do.  A Lanczos step (100
 // steps, open chains), row engine -> pairs, with two row CTAs an SM: 14-site 7+4
-// (3.4 M elements) 88 -> 95 us, 15-site 5+4 (4.1 M) 104 -> 98, 16-site 6+3 (4.5 M)
-// 152 -> 139, 15-site 7+4 (8.8 M) 214 -> 186; with one, whose 16 warps leave the
-// loads' latency open: 13-site 4+6 (1.2 M) 47 -> 47, 15 sites in a 3 x 5 torus 4+4
-// (1.9 M) 86 -> 71, 14-site 4+5 (2.0 M) 64 -> 63, 13-site 5+6 (2.2 M) 76 -> 63,
-// 13-site 6+6 (2.9 M) 102 -> 74, 16-site 8+4 (23 M) 894 -> 413.
+// (3.4 M elements) 87 -> 85 us, 15-site 5+4 (4.1 M) 104 -> 94, 16-site 6+3 (4.5 M)
+// 152 -> 117, 15-site 7+4 (8.8 M) 214 -> 172, but 13-site 6+5 (2.2 M) 59 -> 62;
+// with one, whose 16 warps leave the loads' latency open: 13-site 4+6 (1.2 M)
+// 44 -> 46, 15 sites in a 3 x 5 torus 4+4 (1.9 M) 86 -> 71, 14-site 4+5 (2.0 M)
+// 64 -> 63, 13-site 5+6 (2.2 M) 76 -> 61, 13-site 6+6 (2.9 M) 102 -> 75, 16-site
+// 8+4 (23 M) 894 -> 403.
 static bool prefer_pair(const ed_op* op) {
     if (op->tma_smem == 0) return true;
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
     return op->D >= (op->tma_grid >= 2 * sms ? 4000000 : 1500000);
+}
+
+static ed_status set_pair(ed_op* op, const ed::PairSchedule& g) {
+    if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
+        upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
+        upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
+        return ED_ERR_ALLOC;
+    op->pair_args = {op->d_pairWords, op->d_pairSteps, op->d_pairNeg, g.groups, (int)g.blocks, (int)g.zbase, g.sign};
+    op->pair_smem = ed::pair_smem_bytes(g.zbase);
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
+    // one CTA of 1,024 threads an SM
+    op->pair_nbuf = ed::pair_buffers((int)g.zbase, g.blocks);
+    op->pair_threads = 1024;
+    op->pair_grid = sms;
+    return ED_OK;
 }
 
 // Plans and uploads the row-pair matvec where two rows fit shared memory;
@@ -301,22 +318,9 @@ static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
     if (!schedule_cached(op->bdn, dn_terms, n_dn_terms, false, &SpinEntry::pair_state, &SpinEntry::pair, &g,
                          [&] { return ed::build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err); }))
         return ED_OK;
-    if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
-        upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
-        upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
-        return ED_ERR_ALLOC;
-    op->pair_args = {op->d_pairWords, op->d_pairSteps, op->d_pairNeg, g.groups, (int)g.blocks, (int)g.zbase, g.sign};
-    op->pair_smem = ed::pair_smem_bytes(g.zbase);
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
-    // one CTA of 1,024 threads an SM; two row pairs in shared memory where they
-    // fit (dim_dn up to 7,032: 14- and 15-site sectors), the second staged while
-    // the first is summed
-    op->pair_nbuf = 2 * op->pair_smem <= ed::kPairMaxSmem ? 2 : 1;
-    op->pair_threads = 1024;
-    op->pair_grid = sms;
-    op->pair = true;
-    return ED_OK;
+    const ed_status st = set_pair(op, g);
+    op->pair = st == ED_OK;
+    return st;
 }
 
 // The Lanczos workspace pointer rides on the op (opaque to the header).
@@ -325,6 +329,16 @@ struct ed_op_ext : ed_op {
 };
 
 namespace ed {
+// The row-pair schedule of an operator that its matvec does not use (the batched
+// Lanczos kernel's); false when it has none.
+bool ensure_pair(ed_op* op) {
+    if (op->pair_smem > 0) return true;
+    if (pair_smem_bytes((op->dimDN + 7) / 8 * 8) == 0) return false;
+    PairSchedule g;
+    std::string err;
+    return build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err) && set_pair(op, g) == ED_OK;
+}
+
 void** lanczos_ws_slot(ed_op* op) { return &static_cast<ed_op_ext*>(op)->extra.lz_ws; }
 }  // namespace ed
 

@@ -46,6 +46,23 @@ __device__ __forceinline__ void red_pull(const LzRedSet* r, i128& v, uint64_t& m
     v = (i128)((u128)l0 + ((u128)l1 << 42) + ((u128)(i128)(int64_t)l2 << 84));
 }
 
+// A warp's (v, m) into per-instance shared limb sums (all 32 lanes call it).
+__device__ __forceinline__ void batch_flush(i128 v, uint64_t m, unsigned long long* accl, unsigned long long* accm) {
+    v = warp_sum_i128(v);
+    m = warp_max_u64(m);
+    if ((threadIdx.x & 31) == 0) {
+        const u128 uv = (u128)v;
+        atomicAdd(&accl[0], (unsigned long long)(uv & kLimb));
+        atomicAdd(&accl[1], (unsigned long long)((uv >> 42) & kLimb));
+        atomicAdd(&accl[2], (unsigned long long)(int64_t)(v >> 84));
+        atomicMax(accm, (unsigned long long)m);
+    }
+}
+
+__device__ __forceinline__ i128 batch_total(const unsigned long long* accl) {
+    return (i128)((u128)accl[0] + ((u128)accl[1] << 42) + ((u128)(i128)(int64_t)accl[2] << 84));
+}
+
 // Grid-wide barrier on a monotone arrival counter: the k-th barrier of the
 // launch completes when k * gridDim.x CTAs have arrived.  Writes and atomics
 // before it (by any thread of any CTA) are visible after it.  False when the

@@ -233,8 +233,15 @@ int tma_grid(const ed_op* op);
 void row_plan(const SpinTable& up, int G, std::vector<uint32_t>* start, std::vector<uint32_t>* list,
               std::vector<uint32_t>* queue, double w = -1.0);
 // Shared memory of a row pair of zbase + 8 slots (0: does not fit).
-constexpr int kPairMaxSmem = 220 * 1024;
+constexpr int kPairMaxSmem = 220 * 1024;  // of the rows of one pair
+constexpr int kPairMaxDyn = 222 * 1024;   // of a CTA's buffers
+constexpr int kPairUp = 256;              // up entries staged per row (the longest row has 255)
+constexpr int kPairBufs = 16;
+// a buffer: rows, eight zero slots, 2 x kPairUp up offsets, two PairRows
+constexpr __host__ __device__ int pair_buf_bytes(int zbase) { return (zbase + 8) * 16 + 2 * kPairUp * 4 + 64; }
+int pair_buffers(int zbase, int64_t blocks);
 int pair_smem_bytes(int64_t zbase);
+bool ensure_pair(ed_op* op);
 cudaError_t launch_matvec_pair(const ed_op* op, const MvArgs& a, int out, cudaStream_t s);
 cudaError_t launch_matvec_tma(const ed_op* op, const MvArgs& a, cudaStream_t s);
 // y = H x from FP64 x: the FX copy into xq (DW + 2 values), then the matvec.

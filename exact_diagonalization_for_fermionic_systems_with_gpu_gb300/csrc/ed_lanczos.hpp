@@ -143,7 +143,6 @@ struct LzBatchArgs {
     int64_t n;             // stored values per vector
     unsigned int* gbar;    // grid-barrier arrivals, zero at launch
     LzRedSet* red;         // 4 * B accumulator sets (set r % 4 of instance b at (r % 4) * B + b), zero at launch
-    unsigned int* taken;   // two item-queue counters (step parity), zero at launch
     GridWait wait;
 };
 

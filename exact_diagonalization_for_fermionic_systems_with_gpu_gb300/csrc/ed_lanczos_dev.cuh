@@ -216,5 +216,33 @@ __device__ inline void lz_after_axpy(LzState* lz, int j, i128 sumsq, uint64_t m_
     lz->steps_done = j + 1;
 }
 
+struct SlotScalars {
+    int e;
+    uint64_t m;
+    double beta;
+    double ib;  // 1 / beta (0 when beta is 0)
+};
+
+// Thread 0: slot k (= w_k) is complete with exponent e, exact sum of
+// (q q) >> 16 and max |q|: beta_k, breakdown and precision bookkeeping
+// (lz_after_axpy's), shift the slot scalars, block 0 stores them.
+__device__ __forceinline__ void slot_done(LzState* lz, int k, int e, i128 ss, uint64_t m, SlotScalars& sX,
+                                          SlotScalars& sP, int& status, int& min_bits, bool store) {
+    const double beta = lz_beta(ss, e);
+    const int bits = bitlen_u64(m);
+    if (bits < min_bits) min_bits = bits;
+    if (m == 0 && status == 0) status = 7;  // breakdown
+    if (store) {
+        lz->e[k] = e;
+        lz->m[k] = m;
+        lz->beta[k] = beta;
+        lz->min_bits = min_bits;
+        lz->status = status;
+        lz->steps_done = k;
+    }
+    sP = sX;
+    sX = {e, m, beta, lz_inv(beta)};
+}
+
 }  // namespace dev
 }  // namespace ed

@@ -11,9 +11,11 @@
 // of both rows: down sums from shared memory, then the up neighbours of each
 // row with 16-byte loads of its column pair (dim_dn even; two 8-byte loads
 // otherwise), the diagonal, one rounding, and the Lanczos partials.
-// Where two pairs fit in shared memory the last warp stages the next one with
-// 8-byte asynchronous copies (each row is contiguous, the pair is not) while the
-// other 31 compute, with a full and an empty barrier a buffer: units of 64 columns
+// Where two or more pairs fit in shared memory the last warp stages the next ones
+// with 8-byte asynchronous copies (each row is contiguous, the pair is not) while the
+// other 31 compute, with a full and an empty barrier a buffer (as many buffers as
+// give every warp two units: 16-site 8+3, nine units a pair, 205 -> 157 us with seven
+// for two): units of 64 columns
 // go round the computing warps across pairs, so that no warp waits at the end of
 // a pair for the slowest (54 units on 16 warps: four rounds for 3.4).  Longer rows
 // are staged by all threads between two barriers; the next pair is prefetched into
@@ -34,105 +36,23 @@
 #include <algorithm>
 #include <cstdint>
 
-#include "ed_device.cuh"
-#include "ed_internal.hpp"
-#include "ed_matvec_common.cuh"
-#include "ed_matvec_tma.cuh"
+#include "ed_pair.cuh"
 
 namespace ed {
 using namespace dev;
 
-namespace {
-
-constexpr int kPairUp = 256;  // up entries staged per row (the longest row has 255)
-
-struct Two {
-    int64_t a, b;  // rows u, u + 1
-};
-
-// 16 bytes of shared memory at a 32-bit address (volatile: ordered with the
-// barriers around the staged rows)
-__device__ __forceinline__ void lds2(uint32_t addr, int64_t& x, int64_t& y) {
-    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(addr));
-}
-
-__device__ __forceinline__ void cp_async8(uint32_t dst, const int64_t* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tma::smem_u32(bar)) : "memory");
-}
-
-// One step of both rows: slot word w (low 15 bits; sign in bit 15).
-template <bool SIGN>
-__device__ __forceinline__ void pair_step(uint32_t addr, uint32_t m, Two& acc) {
-    int64_t x, y;
-    lds2(addr, x, y);
-    if (SIGN) {
-        uint64_t mm;
-        asm("mov.b64 %0, {%1, %1};" : "=l"(mm) : "r"(m));
-        x ^= (int64_t)mm;
-        y ^= (int64_t)mm;
-    }
-    acc.a += x;
-    acc.b += y;
-}
-
-template <bool SIGN>
-__device__ __forceinline__ void pair_lo(uint32_t xs, uint32_t w, Two& acc) {
-    uint32_t m = 0;
-    if (SIGN) asm("prmt.b32 %0, %1, 0, 0x9999;" : "=r"(m) : "r"(w));  // bit 15 replicated
-    pair_step<SIGN>(xs + ((w & 0x7FFFu) << 4), m, acc);
-}
-
-template <bool SIGN>
-__device__ __forceinline__ void pair_hi(uint32_t xs, uint32_t w, Two& acc) {
-    pair_step<SIGN>(xs + ((w >> 12) & 0x7FFF0u), (uint32_t)((int32_t)w >> 31), acc);
-}
-
-// n (0..8, the same for the warp) steps of a schedule word
-template <bool SIGN>
-__device__ __forceinline__ void pair_group(uint32_t xs, const uint4 w, int n, Two& acc) {
-    switch (n) {
-        case 8: pair_hi<SIGN>(xs, w.w, acc); [[fallthrough]];
-        case 7: pair_lo<SIGN>(xs, w.w, acc); [[fallthrough]];
-        case 6: pair_hi<SIGN>(xs, w.z, acc); [[fallthrough]];
-        case 5: pair_lo<SIGN>(xs, w.z, acc); [[fallthrough]];
-        case 4: pair_hi<SIGN>(xs, w.y, acc); [[fallthrough]];
-        case 3: pair_lo<SIGN>(xs, w.y, acc); [[fallthrough]];
-        case 2: pair_hi<SIGN>(xs, w.x, acc); [[fallthrough]];
-        case 1: pair_lo<SIGN>(xs, w.x, acc); [[fallthrough]];
-        default: break;
-    }
-}
-
-// What a unit needs of one staged row.
-struct PairRow {
-    uint64_t st;
-    int64_t du;
-    int len, npos;
-};
-
-}  // namespace
-
 // OUT = 0: FP64 y; OUT = 1: FX u with the Lanczos epilogue.  VEC: dim_dn even,
 // lane l has columns 2l, 2l + 1 of a 64-column block; otherwise l, l + 32.
 // MERGE: equal hopping coefficients, one product for the up and down sums.
-// nbuf: row pairs in shared memory (2: the last warp stages, 1: all do).
+// nbuf: row pairs in shared memory (several: the last warp stages, one: all do).
 template <int OUT, bool VEC, bool SIGN, bool MERGE>
 __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairArgs g, const int nbuf) {
     extern __shared__ __align__(128) unsigned char xs[];
-    __shared__ uint32_t uoff_s[2][2][kPairUp];
-    __shared__ PairRow rows_s[2][2];
-    __shared__ uint64_t full[2], empty[2];
+    __shared__ uint64_t full[kPairBufs], empty[kPairBufs];
     const uint32_t dimUP = (uint32_t)a.dimUP, dimDN = (uint32_t)a.dimDN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int nc = nbuf == 1 ? nwarps : nwarps - 1;  // computing warps
     const int64_t* __restrict__ xq = a.xq;
-    const uint4* __restrict__ words = reinterpret_cast<const uint4*>(g.words);
-    const uint32_t xs_base = (uint32_t)__cvta_generic_to_shared(xs);
-    const uint32_t pair_bytes = (uint32_t)(g.zbase + 8) * 16u;
     int E_out = 0, s_u = 0;
     if (OUT == 0) {
         E_out = fx_exp_from_emax(*a.p_emax) - a.Fc;
@@ -145,49 +65,24 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
     const bool y16 = OUT == 1 || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;  // y may start on any double
     i128 dot = 0;
     uint64_t mx = 0;
-    if (tid < 8 * nbuf)
-        *reinterpret_cast<longlong2*>(xs + (tid >> 3) * pair_bytes + (g.zbase + (tid & 7)) * 16) = make_longlong2(0, 0);
-    if (tid == 0) {
-        for (int k = 0; k < 2; ++k) {
-            tma::mbar_init(&full[k], 64);
-            tma::mbar_init(&empty[k], nc);
-        }
-        tma::fence_mbar_init();
-    }
+    pair_init(xs, g, nbuf, nc, full, empty);
     __syncthreads();
     const uint32_t npairs = (dimUP + 1) / 2;
     int buf = 0;
     uint32_t parity = 0;  // of the buffer's current use
-    // row pair `it` into buffer k: thread i of n
-    auto stage = [&](uint32_t it, int k, uint32_t i0, uint32_t n) {
-        const uint32_t u0 = 2 * it;
-        const int nrow = u0 + 1 < dimUP ? 2 : 1;  // an odd count ends on a pair of one row
-        for (int r = 0; r < nrow; ++r) {
-            const uint32_t u = u0 + r, q0 = __ldg(a.upPtr + u), len = __ldg(a.upPtr + u + 1) - q0;
-            for (uint32_t i = i0; i < len; i += n) uoff_s[k][r][i] = (__ldg(a.upEntC + q0 + i) & kColMask) * dimDN;
-            if (i0 == r) rows_s[k][r] = {__ldg(a.stUP + u), __ldg(a.dUPq + u), (int)len, (int)__ldg(a.upNpos + u)};
-        }
-        const int64_t* const r0 = xq + (size_t)u0 * dimDN;
-        const int64_t* const r1 = nrow == 2 ? r0 + dimDN : r0;
-        const uint32_t xb = xs_base + k * pair_bytes;
-#pragma unroll 4
-        for (uint32_t c = i0; c < dimDN; c += n) {
-            const uint32_t d = xb + pair_slot(c) * 16u;
-            cp_async8(d, r0 + c);
-            cp_async8(d + 8, r1 + c);
-        }
-    };
     if (warp == nc) {
         for (uint32_t it = blockIdx.x; it < npairs; it += gridDim.x) {
             if (!tma::mbar_wait(&empty[buf], parity ^ 1)) {  // at once in the buffer's first use
                 if (lane == 0) atomicExch(a.err, 1);
                 break;
             }
-            stage(it, buf, lane, 32);
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tma::smem_u32(&full[buf])) : "memory");
+            pair_stage(a, xq, a.dUPq, 2 * it, PairBuf(xs, g, buf), lane, 32);
+            cp_async_arrive(&full[buf]);
             mbar_arrive(&full[buf]);
-            buf ^= 1;
-            if (buf == 0) parity ^= 1;
+            if (++buf == nbuf) {
+                buf = 0;
+                parity ^= 1;
+            }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
@@ -195,12 +90,10 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
     for (uint32_t it = warp == nc ? npairs : blockIdx.x; it < npairs; it += gridDim.x) {
         const uint32_t u0 = 2 * it;
         const bool has1 = u0 + 1 < dimUP;
-        const uint32_t xs32 = xs_base + buf * pair_bytes;
-        const uint32_t(*uoff)[kPairUp] = uoff_s[buf];
-        const PairRow* const rows = rows_s[buf];
+        const PairBuf B(xs, g, buf);
         if (nbuf == 1) {
             __syncthreads();  // the previous rows are no longer read
-            stage(it, 0, tid, blockDim.x);
+            pair_stage(a, xq, a.dUPq, 2 * it, B, tid, blockDim.x);
             if (tid == 0 && it + gridDim.x < npairs) {
                 // an even row starts on a 16-byte boundary
                 const uint32_t un = 2 * (it + gridDim.x);
@@ -219,72 +112,20 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
             const uint32_t c0 = 64u * b + (VEC ? 2u * lane : (uint32_t)lane), c1 = VEC ? c0 + 1 : c0 + 32;
             if (c0 >= dimDN) continue;
             const bool v1 = VEC || c1 < dimDN;  // the second column exists
-            const int64_t* const xc = xq + c0;
-            auto get = [&](uint32_t off, int64_t& w0, int64_t& w1) {
-                if (VEC) {
-                    const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(xc + off));
-                    w0 = v.x;
-                    w1 = v.y;
-                } else {
-                    w0 = __ldcg(xc + off);
-                    w1 = v1 ? __ldcg(xc + off + 32) : 0;
-                }
-            };
-            // down sums of columns c0, c1 in both rows
-            Two dn[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint4* sp = words + ((size_t)(2 * b + h) * g.groups) * 32 + lane;
-                int n = __ldg(g.steps + 2 * b + h);
-                const int64_t neg = SIGN && (h == 0 || v1) ? __ldg(g.negcnt + (h ? c1 : c0)) : 0;
-                dn[h] = Two{neg, neg};
-                for (; n > 8; n -= 8, sp += 32) pair_group<SIGN>(xs32, __ldg(sp), 8, dn[h]);
-                pair_group<SIGN>(xs32, __ldg(sp), n, dn[h]);
-                if (!SIGN && g.sign < 0) dn[h] = Two{-dn[h].a, -dn[h].b};
-            }
-            // up sums (added to the down sums where one product serves both)
-            Two up[2];
-            if (MERGE) {
-                up[0] = dn[0];
-                up[1] = dn[1];
-            } else {
-                up[0] = up[1] = Two{0, 0};
-            }
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                if (r == 1 && !has1) break;
-                const int len = rows[r].len, npos = rows[r].npos;
-                int64_t s0 = 0, s1 = 0;
-                int k = 0;
-#pragma unroll 4
-                for (; k < npos; ++k) {
-                    int64_t w0, w1;
-                    get(uoff[r][k], w0, w1);
-                    s0 += w0;
-                    s1 += w1;
-                }
-#pragma unroll 4
-                for (; k < len; ++k) {
-                    int64_t w0, w1;
-                    get(uoff[r][k], w0, w1);
-                    s0 -= w0;
-                    s1 -= w1;
-                }
-                (r ? up[0].b : up[0].a) += s0;
-                (r ? up[1].b : up[1].a) += s1;
-            }
+            Two dn[2], up[2];
+            pair_sums<VEC, SIGN, MERGE>(g, xq, B, has1, b, lane, c0, c1, v1, dn, up);
             int64_t qo[2][2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (h == 1 && !v1) break;
                 const uint32_t c = h ? c1 : c0;
                 int64_t xr[2];
-                lds2(xs32 + pair_slot(c) * 16u, xr[0], xr[1]);
+                lds2(B.x32 + pair_slot(c) * 16u, xr[0], xr[1]);
                 const int64_t ddn = __ldg(a.dDNq + c);
                 const uint64_t std_ = __ldg(a.stDN + c) & a.mask;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const PairRow& R = rows[has1 ? r : 0];
+                    const PairRow& R = B.rows[has1 ? r : 0];
                     const int64_t x = xr[r], us = r ? up[h].b : up[h].a, ds = r ? dn[h].b : dn[h].a;
                     const int64_t dq = R.du + ddn + a.Uq * (int64_t)__popcll(R.st & std_);
                     if (OUT == 1 && fold) {
@@ -321,12 +162,14 @@ __global__ void __launch_bounds__(1024, 1) k_mv_pair(const MvArgs a, const PairA
                 }
             }
         }
-        if (nbuf == 2) {
+        if (nbuf > 1) {
             b0 = b - g.blocks;
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[buf]);
-            buf ^= 1;
-            if (buf == 0) parity ^= 1;
+            if (++buf == nbuf) {
+                buf = 0;
+                parity ^= 1;
+            }
         }
     }
     if (OUT == 1) mv_lanczos_epilogue(a, dot, mx, s_u);
@@ -337,12 +180,21 @@ int pair_smem_bytes(int64_t zbase) {
     return bytes <= kPairMaxSmem ? (int)bytes : 0;
 }
 
+// Buffers of a CTA: units for all the computing warps twice over (a buffer is free
+// when its last unit is done), two where a pair has as many units itself.  More
+// would take the schedule words' L1.
+int pair_buffers(int zbase, int64_t blocks) {
+    const int64_t fit = kPairMaxDyn / pair_buf_bytes(zbase);
+    const int64_t want = blocks >= 31 ? 2 : (62 + blocks - 1) / blocks;
+    return (int)std::max<int64_t>(1, std::min<int64_t>({fit, want, kPairBufs}));
+}
+
 template <int OUT, bool VEC, bool MERGE>
 static cudaError_t launch_pair3(const ed_op* op, const MvArgs& a, cudaStream_t s) {
     auto kern = op->pair_args.sign == 0 ? k_mv_pair<OUT, VEC, true, MERGE> : k_mv_pair<OUT, VEC, false, MERGE>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->pair_nbuf * op->pair_smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, op->pair_nbuf * pair_buf_bytes(op->pair_args.zbase));
     if (e != cudaSuccess) return e;
-    kern<<<op->pair_grid, op->pair_threads, op->pair_nbuf * op->pair_smem, s>>>(a, op->pair_args, op->pair_nbuf);
+    kern<<<op->pair_grid, op->pair_threads, op->pair_nbuf * pair_buf_bytes(op->pair_args.zbase), s>>>(a, op->pair_args, op->pair_nbuf);
     return cudaGetLastError();
 }
 

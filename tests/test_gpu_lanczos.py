@@ -470,3 +470,30 @@ def test_reorth_one_launch_matches_per_step(ed, monkeypatch, case):
     assert got["launch"][0] == got["steps"][0]
     assert np.array_equal(got["launch"][1], got["steps"][1])
     assert got["launch"][2] < got["steps"][2]
+
+
+# batches on the row pairs: one to sixteen buffers' worth of units a pair, odd up
+# and down counts, signs of either kind and mixed, unequal hopping of the spins, one
+# pair, vectors above and below a pass of the grid, more items than CTAs or fewer
+@pytest.mark.parametrize("N,qu,qd,B,ring,t_dn", [(8, 4, 4, 2, True, -1.0), (9, 4, 2, 8, False, -1.0), (7, 3, 4, 3, True, -1.0),
+                                                 (10, 5, 5, 7, False, 1.0), (11, 5, 5, 3, True, -0.7), (6, 0, 3, 2, True, -1.0),
+                                                 (6, 1, 6, 2, True, -1.0), (12, 6, 5, 2, True, -1.0)])
+def test_lanczos_batch_sectors(ed, N, qu, qd, B, ring, t_dn):
+    from conftest import philox_uniform
+    ops = []
+    for r in range(B):
+        eps = philox_uniform(40 + r, 2 * N, 2.0)
+        bonds = [(i, (i + 1) % N) for i in range(N if ring else N - 1)]
+        tu = [("H", i, j, -1.0, 0.0) for i, j in bonds] + [("N", i, 0, eps[i], 0.0) for i in range(N)]
+        td = [("H", i, j, t_dn, 0.0) for i, j in bonds] + [("N", i, 0, eps[N + i], 0.0) for i in range(N)]
+        ops.append(ed.Hubbard(ed.H_TBq(N, qu).extend(tu), ed.H_TBq(N, qd).extend(td), 1.0 + 0.25 * r))
+    steps = min(15, ops[0].rows())
+    e0, ev, al, be = ed.lanczos_batch(ops, steps, seed=3)
+    for b, op in enumerate(ops):
+        lz = ed.Lanczos()
+        e, v = lz.eigen(op, max_steps=steps, mode="fixed", seed=3 + b)
+        n = len(lz.a)
+        assert e0[b] == e
+        assert np.array_equal(al[b][:n], np.array(lz.a)) and np.array_equal(be[b][:n + 1], np.array(lz.b)[:n + 1])
+        assert np.array_equal(ev[b], v)
+        op.close()
