@@ -114,19 +114,20 @@ __device__ __forceinline__ i128 mul_wide(int64_t a, int64_t b) {
     return (i128)(((u128)(uint64_t)hi << 64) | (u128)lo);
 }
 
-// Exact sums of 54-bit x 57-bit products in 32-bit multiply-adds.  A vector
-// element |q| < 2^54 and a coefficient |c| < 2^57 are split at 27 bits
-// (value = h 2^27 + l, 0 <= l < 2^27); the four partial products go to three
-// 64-bit accumulators of weights 2^54, 2^27 and 1, one 32 x 32 + 64
-// multiply-add each, where a double-precision multiply-add would hold the
-// FP64 pipe for 16 cycles a warp.  Each term adds less than 2^57.2 to mid, so
-// limb_carry is due every kLimbRun terms; hi stays in range while the |c| of
-// a sum total at most 2^61.
+// Exact sums of 54-bit x 57-bit products in 32-bit multiply-adds, where a
+// double-precision multiply-add would hold the FP64 pipe for 16 cycles a warp.  A
+// vector element |q| < 2^54 and a coefficient |c| < 2^57 are split at 27 bits
+// (value = h 2^27 + l, 0 <= l < 2^27).  Three 64-bit accumulators take the high
+// products, the low ones and (h + l)(H + L); the cross products h L + l H are the
+// last less the first two (Karatsuba), modulo 2^64, three multiply-adds for four
+// partial products.  Where the |c| of a sum total at most 2^61, the h H and l H sums
+// stay below 2^61 + n 2^27 each and the h L and l L sums below n 2^54, so limb_carry
+// is due every kLimbRun terms (128: all below 2^62.6).
 constexpr int kLimbBits = 27;
-constexpr int kLimbRun = 16;
+constexpr int kLimbRun = 128;
 
 struct LimbSum {
-    int64_t hi, mid, lo;
+    int64_t hi, all, lo;
 };
 
 __device__ __forceinline__ void limb_split(int64_t v, int& h, int& l) {
@@ -140,22 +141,25 @@ __device__ __forceinline__ void mad_wide(int64_t& a, int x, int y) {
 
 __device__ __forceinline__ void limb_mac(LimbSum& a, int qh, int ql, int ch, int cl) {
     mad_wide(a.hi, qh, ch);
-    mad_wide(a.mid, qh, cl);
-    mad_wide(a.mid, ql, ch);
     mad_wide(a.lo, ql, cl);
+    mad_wide(a.all, qh + ql, ch + cl);
 }
 
+// The low and cross sums reduced to 27 bits each.
 __device__ __forceinline__ void limb_carry(LimbSum& a) {
     constexpr int64_t m = (1LL << kLimbBits) - 1;
-    a.mid += a.lo >> kLimbBits;
+    int64_t mid = (int64_t)((uint64_t)a.all - (uint64_t)a.hi - (uint64_t)a.lo);
+    mid += a.lo >> kLimbBits;
     a.lo &= m;
-    a.hi += a.mid >> kLimbBits;
-    a.mid &= m;
+    a.hi += mid >> kLimbBits;
+    mid &= m;
+    a.all = (int64_t)((uint64_t)a.hi + (uint64_t)a.lo + (uint64_t)mid);
 }
 
 // The sum (after limb_carry) as a 128-bit integer.
 __device__ __forceinline__ i128 limb_total(const LimbSum& a) {
-    return ((i128)a.hi << (2 * kLimbBits)) + (i128)((a.mid << kLimbBits) | a.lo);
+    const int64_t mid = (int64_t)((uint64_t)a.all - (uint64_t)a.hi - (uint64_t)a.lo);
+    return ((i128)a.hi << (2 * kLimbBits)) + (i128)((mid << kLimbBits) | a.lo);
 }
 
 // acc += a b: the compiler's 128-bit multiply-add, 35 cycles a warp scheduler

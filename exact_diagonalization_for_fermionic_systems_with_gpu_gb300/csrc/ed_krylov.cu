@@ -30,9 +30,10 @@ namespace {
 constexpr int kKrThreads = 256;
 constexpr int kKrTimes = 4;  // times formed per pass over the basis
 constexpr int kKcThreads = 128;
-constexpr int kKcGroup = 8;    // basis vectors per copy group (a complex product adds two terms: kLimbRun / 2)
+constexpr int kKcGroup = 8;    // basis vectors per copy group
 constexpr int kKcChunk = 128;  // basis vectors whose coefficients are staged at a time
-static_assert(2 * kKcGroup <= dev::kLimbRun && kKcChunk % kKcGroup == 0, "carry interval");
+constexpr int kKcCarry = dev::kLimbRun / 2;  // vectors between carries (a complex product adds two terms)
+static_assert(kKcCarry % kKcGroup == 0 && kKcChunk % kKcGroup == 0, "carry interval");
 constexpr int kKrBlocks = 152 * 8;
 
 int kr_grid(int64_t n) {
@@ -76,9 +77,10 @@ __global__ void k_part(const double* __restrict__ z, int64_t n, int p, double* _
 // for each k the NT times' (re high, re low, im high, im low) limbs, scaled
 // by 2^F[t].
 //
-// Bound by instruction issue: the sums are exact integers (limb_mac, four
-// 32-bit multiplies and their 64-bit adds per real product), where FP64
-// multiply-adds issue at 1/64 of the FP32 rate.  A thread forms two adjacent
+// Bound by instruction issue: the sums are exact integers (limb_mac, three
+// 32-bit multiplies and their 64-bit adds per real product; four, before the
+// cross products came from one, took 594 us for 470 at 140 vectors of 853,776
+// elements and 4 times), where FP64 multiply-adds issue at 1/64 of the FP32 rate.  A thread forms two adjacent
 // real elements (or one complex one) at NT = 4 times from 16 bytes of every
 // basis vector; at the 48 accumulator registers x 2 that takes, 12 warps an
 // SM are resident, too few to hide load latency, so each thread copies its
@@ -167,13 +169,15 @@ __global__ void __launch_bounds__(kKcThreads, 3) k_krylov_combine(const int64_t*
                     }
                 }
             }
+            if ((k0 + kKcGroup) % kKcCarry == 0 || g + 1 == ngroups) {
 #pragma unroll
-            for (int e = 0; e < E; ++e)
+                for (int e = 0; e < E; ++e)
 #pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    limb_carry(re[e][t]);
-                    limb_carry(im[e][t]);
-                }
+                    for (int t = 0; t < NT; ++t) {
+                        limb_carry(re[e][t]);
+                        limb_carry(im[e][t]);
+                    }
+            }
         }
         if (!live) continue;
 #pragma unroll

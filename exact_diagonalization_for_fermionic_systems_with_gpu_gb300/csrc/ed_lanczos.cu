@@ -254,7 +254,8 @@ __global__ void __launch_bounds__(kLzThreads) k_lz_reorth(int64_t* __restrict__ 
 // A thread forms two adjacent elements from 16-byte loads of every slot
 // (slots are 256-byte aligned), kRitzSlots slots per iteration with all their
 // loads issued before the sums; the basis is read once.
-constexpr int kRitzSlots = kLimbRun;
+constexpr int kRitzSlots = 16;
+static_assert(kLimbRun % kRitzSlots == 0, "carry interval");
 
 __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__ basis, int64_t n, int64_t stride,
                                                      int nk, const int2* __restrict__ c, int F,
@@ -282,8 +283,10 @@ __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__
                 add(a0, v[t].x, ck);
                 add(a1, v[t].y, ck);
             }
-            limb_carry(a0);
-            limb_carry(a1);
+            if ((k + kRitzSlots) % kLimbRun == 0) {
+                limb_carry(a0);
+                limb_carry(a1);
+            }
         }
         for (; k < nk; ++k) {
             const longlong2 v = __ldg(q + k * s2);

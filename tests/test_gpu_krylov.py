@@ -201,3 +201,30 @@ def test_krylov_one_launch_stops_like_per_step(ed, monkeypatch, steps):
         assert got[0][1] == got[1][1]
         assert np.array_equal(got[0][0], got[1][0])
         op.close()
+
+
+@pytest.mark.parametrize("case", ["real", "complex"])
+def test_krylov_combine_long_sums(ed, orc, case):
+    """Sums over more basis vectors than two carry intervals (64 vectors), with
+    weight on all of them: t W / 2 reaches 100, so about 120 of the 150
+    coefficients matter and the space still holds the result.  Against dense
+    exp(-iHt); the rounding of T's eigensolve and the lost orthogonality of 150
+    steps stay far below 1e-9 |psi0|."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import evolution as ev, lattices as L
+    from conftest import philox_uniform
+    if case == "complex":
+        N, qu, qd, t = 12, 1, 2, L.kagome12(flux=0.7)
+    else:
+        N, qu, qd = 7, 3, 2
+        t = L.chain(N, periodic=False, eps=list(philox_uniform(3, N, 2.0)))
+    op = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 2.0)
+    Hd = orc.hamiltonian(N, qu, qd, t, t, 2.0).toarray()
+    w, V = np.linalg.eigh(Hd)
+    x = philox_uniform(31, 2 * op.rows())
+    psi0 = x[0::2] + 1j * x[1::2]
+    times = [T * 40.0 / (w[-1] - w[0]) for T in (1.0, 3.0, 5.0)]
+    out = ev.krylov_evolve(op, psi0, times, max_steps=150)
+    for k, T in enumerate(times):
+        exact = V @ (np.exp(-1j * w * T) * (V.conj().T @ psi0))
+        assert np.linalg.norm(out[k] - exact) < 1e-9 * np.linalg.norm(psi0)
+    op.close()
