@@ -318,9 +318,10 @@ __global__ void __launch_bounds__(kLzThreads) k_ritz(const int64_t* __restrict__
     const double bs = block_sum_f64(ss, sd);
     if (threadIdx.x == 0) part[blockIdx.x] = bs;
     if (elect_last_block(counter)) {
+        double t = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += __ldcg(part + i);
+        t = block_sum_f64(t, sd);
         if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int i = 0; i < (int)gridDim.x; ++i) t += __ldcg(part + i);
             *inv_norm = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
             *counter = 0;
         }
@@ -385,9 +386,10 @@ __global__ void __launch_bounds__(kLzThreads) k_inv_norm(const double* __restric
     const double bs = block_sum_f64(ss, sd);
     if (threadIdx.x == 0) part[blockIdx.x] = bs;
     if (elect_last_block(counter)) {
+        double t = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += __ldcg(part + i);
+        t = block_sum_f64(t, sd);
         if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int i = 0; i < (int)gridDim.x; ++i) t += __ldcg(part + i);
             *inv_norm = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
             *counter = 0;
         }
