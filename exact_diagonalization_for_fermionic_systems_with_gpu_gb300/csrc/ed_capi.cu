@@ -294,6 +294,9 @@ static bool prefer_pair(const ed_op* op) {
 }
 
 static ed_status set_pair(ed_op* op, const ed::PairSchedule& g) {
+    cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);  // of an upload that failed
+    op->d_pairWords = nullptr;
+    op->d_pairSteps = op->d_pairNeg = nullptr;
     if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
         upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
         upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
