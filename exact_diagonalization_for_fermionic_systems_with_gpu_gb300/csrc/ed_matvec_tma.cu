@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_matvec_tma(const MvArgs a) {
 // CTAs, and nothing is cleared by the host.  The conversion reads x again from
 // L2.  The barriers are the runtime's (cooperative launch: every CTA is
 // resident), so a CTA whose table copy gave up still takes part in both.
-// Kagome12 42.0 -> 30.7 us, Kagome12 with flux 95 -> 84 us, 8-site ring 17.0 ->
-// 10.2 us (calls in a row, host and device).
+// Kagome12 42.0 -> 30.7 us, Kagome12 with flux 95 -> 84 us (69 with the class
+// schedule and split rows), 8-site ring 17.0 -> 10.2 us (calls in a row, host and device).
 template <bool CPLX, bool FAST, bool SCHED, bool SEG = false>
 __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const ApplyArgs f) {
     extern __shared__ __align__(128) unsigned char sm[];
