@@ -45,28 +45,33 @@ constexpr int kEgThreads = 256;
 constexpr int kEgWarps = kEgThreads / 32;
 constexpr int kEgDots = 16;  // dots whose partial sums a thread holds at a time
 constexpr int kEgBlocks = 152 * 4;
+constexpr int kEgDotBlocks = 152 * 2;  // one wave at 128 registers
 constexpr int kEgOut = 8;    // vectors formed per pass of the combination kernel
 
 // The kernels below are bound by the FP64 pipe (1/64 of the FP32 rate: one
 // multiply-add holds a warp scheduler's pipe for 64 cycles), not by memory, so
 // they spend none of it on anything but the sums: scalars are computed by one
-// thread of one block, and the sixteen partial sums of a warp are reduced
-// together (16 additions a lane instead of 80).
+// thread of one block, and the partial sums of a warp are reduced together
+// (16 additions a lane for sixteen instead of 80).
 
-// 16 values per lane, summed over the 32 lanes: lane l gets the total of value
-// l >> 1.  Every step halves the values a lane keeps; fixed order.
-__device__ __forceinline__ double reduce16(double* s) {
+// D values per lane (a power of two up to 16), summed over the 32 lanes: lane l
+// gets the total of value l >> (5 - log2 D).  Every step halves the values a lane
+// keeps, until one is left; fixed order.
+template <int D>
+__device__ __forceinline__ double reduce_lanes(double* s) {
     const int lane = threadIdx.x & 31;
+    int bit = 16;
 #pragma unroll
-    for (int h = 8; h > 0; h >>= 1) {  // lanes differing in bit 2h
-        const bool up = lane & (2 * h);
+    for (int h = D / 2; h > 0; h >>= 1, bit >>= 1) {
+        const bool up = lane & bit;
 #pragma unroll
         for (int i = 0; i < h; ++i) {
             const double send = up ? s[i] : s[i + h], keep = up ? s[i + h] : s[i];
-            s[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+            s[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
         }
     }
-    return s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+    for (; bit > 0; bit >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+    return s[0];
 }
 
 // A pair of elements 2i, 2i + 1 of a vector of n values (16-byte aligned; the
@@ -84,46 +89,75 @@ __device__ __forceinline__ void st_pair(double* __restrict__ v, int64_t i, int64
 // w <- w - sum_t loc_c[t] V_{loc0 + t} (t < nloc <= 2, written back), then
 // coef[k] = <V_k, w>, k0 <= k < k0 + nk, and tcol[k] = coef[k] + (loc_c where k
 // is a local vector, or with acc what tcol[k] was).  Block partials; the last
-// block sums them in index order.
-__global__ void __launch_bounds__(kEgThreads) k_eg_dots(const double* __restrict__ V, int64_t stride, int k0, int nk,
-                                                        double* __restrict__ w, int64_t n, int loc0, int nloc,
-                                                        const double* __restrict__ loc_c, double* __restrict__ part,
-                                                        unsigned int* counter, double* __restrict__ coef,
-                                                        double* __restrict__ tcol, int acc) {
-    __shared__ double sh[kEgWarps][kEgDots];
-    const int64_t np = (n + 1) >> 1;
+// block sums them in index order.  D: dots whose partial sums a thread holds.
+// The loads of four vectors are issued before their sums (a branch around each put
+// them one behind the other, 4.3 us a vector at 853,776 rows), and the grid is the
+// resident blocks (half as many warp sums): fourteen vectors 62 -> 37 us, 20 of them
+// the FP64 pipe; eight or two loads at a time: 39 and 43.  Two vectors, with D = 2 for
+// 16 and so fewer additions in the warp sums: 17 -> 9.5 us.
+template <int D>
+__global__ void __launch_bounds__(kEgThreads, 2) k_eg_dots(const double* __restrict__ V, int64_t stride, int k0, int nk,
+                                                           double* __restrict__ w, int64_t n, int loc0, int nloc,
+                                                           const double* __restrict__ loc_c, double* __restrict__ part,
+                                                           unsigned int* counter, double* __restrict__ coef,
+                                                           double* __restrict__ tcol, int acc) {
+    constexpr int kLoad = D < 4 ? D : 4;
+    __shared__ double sh[kEgWarps][D];
+    const int64_t np = n >> 1;  // whole pairs
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double l0 = nloc > 0 ? __ldg(loc_c) : 0.0, l1 = nloc > 1 ? __ldg(loc_c + 1) : 0.0;
-    for (int g0 = 0; g0 < nk; g0 += kEgDots) {
+    const double* const A = V + (size_t)loc0 * stride;
+    const double* const B = A + stride;
+    for (int g0 = 0; g0 < nk; g0 += D) {
         const double* Vg = V + (size_t)(k0 + g0) * stride;
-        const int ng = min(kEgDots, nk - g0);
-        double s[kEgDots];
+        const int ng = min(D, nk - g0);
+        const bool sub = g0 == 0 && nloc > 0;
+        double s[D];
 #pragma unroll
-        for (int t = 0; t < kEgDots; ++t) s[t] = 0.0;
+        for (int t = 0; t < D; ++t) s[t] = 0.0;
         for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < np; i += (int64_t)gridDim.x * kEgThreads) {
-            double2 x = ld_pair(w, i, n);
-            if (g0 == 0 && nloc > 0) {
-                const double2 a = ld_pair(V + (size_t)loc0 * stride, i, n);
-                x.x = fma(-l0, a.x, x.x);
-                x.y = fma(-l0, a.y, x.y);
-                if (nloc > 1) {
-                    const double2 b = ld_pair(V + (size_t)(loc0 + 1) * stride, i, n);
-                    x.x = fma(-l1, b.x, x.x);
-                    x.y = fma(-l1, b.y, x.y);
+            double2 x = reinterpret_cast<const double2*>(w)[i];
+#pragma unroll
+            for (int t0 = 0; t0 < D; t0 += kLoad) {
+                if (t0 >= ng) break;
+                double2 v[kLoad];
+#pragma unroll
+                for (int t = 0; t < kLoad; ++t)
+                    v[t] = reinterpret_cast<const double2*>(Vg + (size_t)min(t0 + t, ng - 1) * stride)[i];
+                if (t0 == 0 && sub) {
+                    const double2 a = reinterpret_cast<const double2*>(A)[i];
+                    const double2 b = nloc > 1 ? reinterpret_cast<const double2*>(B)[i] : make_double2(0.0, 0.0);
+                    x.x = fma(-l0, a.x, x.x);
+                    x.y = fma(-l0, a.y, x.y);
+                    if (nloc > 1) {
+                        x.x = fma(-l1, b.x, x.x);
+                        x.y = fma(-l1, b.y, x.y);
+                    }
+                    reinterpret_cast<double2*>(w)[i] = x;
                 }
-                st_pair(w, i, n, x);
+#pragma unroll
+                for (int t = 0; t < kLoad; ++t)
+                    if (t0 + t < ng) {
+                        s[t0 + t] = fma(v[t].x, x.x, s[t0 + t]);
+                        s[t0 + t] = fma(v[t].y, x.y, s[t0 + t]);
+                    }
+            }
+        }
+        if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+            double x = w[n - 1];
+            if (sub) {
+                x = fma(-l0, A[n - 1], x);
+                if (nloc > 1) x = fma(-l1, B[n - 1], x);
+                w[n - 1] = x;
             }
 #pragma unroll
-            for (int t = 0; t < kEgDots; ++t)
-                if (t < ng) {
-                    const double2 v = ld_pair(Vg + (size_t)t * stride, i, n);
-                    s[t] = fma(v.x, x.x, s[t]);
-                    s[t] = fma(v.y, x.y, s[t]);
-                }
+            for (int t = 0; t < D; ++t)
+                if (t < ng) s[t] = fma(Vg[(size_t)t * stride + n - 1], x, s[t]);
         }
-        const double r = reduce16(s);
+        const double r = reduce_lanes<D>(s);
+        constexpr int kSpan = 32 / D;  // lanes with the same total
         __syncthreads();  // the previous group's sums are read
-        if ((lane & 1) == 0) sh[warp][lane >> 1] = r;
+        if (lane % kSpan == 0) sh[warp][lane / kSpan] = r;
         __syncthreads();
         if (threadIdx.x < ng) {
             double t = 0.0;
@@ -161,22 +195,39 @@ __global__ void __launch_bounds__(kEgThreads) k_eg_update(double* __restrict__ w
                                                           int64_t n, double* __restrict__ part, unsigned int* counter,
                                                           double* __restrict__ beta, double* __restrict__ inv) {
     __shared__ double sh[32];
-    const int64_t np = (n + 1) >> 1;
+    const int64_t np = n >> 1;  // whole pairs
     double ss = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * kEgThreads + threadIdx.x; i < np; i += (int64_t)gridDim.x * kEgThreads) {
-        double2 x = ld_pair(w, i, n);
-#pragma unroll 4
-        for (int k = 0; k < nk; ++k) {
+        double2 x = reinterpret_cast<const double2*>(w)[i];
+        int k = 0;
+        for (; k + 4 <= nk; k += 4) {
+            double2 v[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) v[t] = reinterpret_cast<const double2*>(V + (size_t)(k + t) * stride)[i];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const double c = -__ldg(coef + k + t);
+                x.x = fma(c, v[t].x, x.x);
+                x.y = fma(c, v[t].y, x.y);
+            }
+        }
+        for (; k < nk; ++k) {
             const double c = -__ldg(coef + k);
-            const double2 v = ld_pair(V + (size_t)k * stride, i, n);
+            const double2 v = reinterpret_cast<const double2*>(V + (size_t)k * stride)[i];
             x.x = fma(c, v.x, x.x);
             x.y = fma(c, v.y, x.y);
         }
-        if (nk > 0) st_pair(w, i, n, x);
+        if (nk > 0) reinterpret_cast<double2*>(w)[i] = x;
         if (beta) {
             ss = fma(x.x, x.x, ss);
             ss = fma(x.y, x.y, ss);
         }
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        double x = w[n - 1];
+        for (int k = 0; k < nk; ++k) x = fma(-__ldg(coef + k), V[(size_t)k * stride + n - 1], x);
+        w[n - 1] = x;
+        if (beta) ss = fma(x, x, ss);
     }
     if (!beta) return;
     ss = dev::block_sum_f64(ss, sh);
@@ -234,9 +285,9 @@ int eg_grid(int64_t n) {
 
 // Blocks of the kernels that take pairs of elements (fixed by n: the sums'
 // order, and so every bit of the result, follows from it).
-int eg_pair_grid(int64_t n) {
+int eg_pair_grid(int64_t n, int64_t most = kEgBlocks) {
     const int64_t g = ((n + 1) / 2 + kEgThreads - 1) / kEgThreads;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(g, kEgBlocks));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(g, most));
 }
 
 }  // namespace
@@ -368,7 +419,7 @@ ed_status ed_eigs_lowest(ed_op* op, const ed_eigs_cfg* cfg, const double* start,
         ++launches;
     }
     EG_CK(cudaMemsetAsync(counter, 0, sizeof(unsigned int), s));
-    const int gp = eg_pair_grid(n);
+    const int gp = eg_pair_grid(n), gd = eg_pair_grid(n, kEgDotBlocks);
     double* const inv = coef + m + 1;    // 1 / |w|
     double* const local = coef + m + 2;  // coefficients on v_{j-1}, v_j of the first pass
     // dst = w / |w| after w <- w - V[0..nk) coef, |w| to beta[bidx]
@@ -400,14 +451,14 @@ ed_status ed_eigs_lowest(ed_op* op, const ed_eigs_cfg* cfg, const double* start,
             const bool full = j == k0 && j > 0;
             const int nloc = full ? 0 : (j > 0 ? 2 : 1), loc0 = full ? 0 : j + 1 - nloc;
             if (full) {
-                k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, 0, 0, nullptr, part, counter, coef, tcol, 0);
+                k_eg_dots<kEgDots><<<gd, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, 0, 0, nullptr, part, counter, coef, tcol, 0);
                 k_eg_update<<<gp, kEgThreads, 0, s>>>(w, V, stride, j + 1, coef, n, part, counter, nullptr, nullptr);
                 launches += 2;
             } else {
-                k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, loc0, nloc, w, n, 0, 0, nullptr, part, counter, local, nullptr, 0);
+                k_eg_dots<2><<<gd, kEgThreads, 0, s>>>(V, stride, loc0, nloc, w, n, 0, 0, nullptr, part, counter, local, nullptr, 0);
                 ++launches;
             }
-            k_eg_dots<<<gp, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, loc0, nloc, local, part, counter, coef, tcol,
+            k_eg_dots<kEgDots><<<gd, kEgThreads, 0, s>>>(V, stride, 0, j + 1, w, n, loc0, nloc, local, part, counter, coef, tcol,
                                                 full ? 1 : 0);
             ++launches;
             EG_CK(normalise(V + (size_t)(j + 1) * stride, j + 1, j + 1));

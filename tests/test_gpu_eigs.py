@@ -107,3 +107,20 @@ def test_eigs_dot_groups(ed, orc, N, qu, qd, nev, ncv):
     for k in range(nev):
         assert np.linalg.norm(op.matvec(v[k]) - w[k] * v[k]) < 1e-8
     op.close()
+
+
+@pytest.mark.parametrize("N,qu,qd,nev,ncv", [(7, 3, 2, 1, 3), (7, 3, 2, 2, 17), (7, 3, 2, 3, 18), (8, 4, 3, 4, 21), (8, 4, 3, 6, 34)])
+def test_eigs_subspace_sizes(ed, orc, N, qu, qd, nev, ncv):
+    """Subspaces below, at and above the groups of sixteen and four vectors of
+    the Gram-Schmidt dots, an odd and an even number of rows, against dense
+    eigenvalues (tolerance: the solver's 1e-10 on the residual, squared in E)."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L, spectra
+    from conftest import philox_uniform
+    t = L.chain(N, periodic=False, eps=list(philox_uniform(9, N, 1.0)))
+    op = ed.Hubbard(ed.H_TBq(N, qu).extend(t), ed.H_TBq(N, qd).extend(t), 2.0)
+    exact = np.linalg.eigvalsh(orc.hamiltonian(N, qu, qd, t, t, 2.0).toarray())[:nev]
+    w, v, _ = spectra.eigs_lowest(op, nev, ncv=ncv, seed=4)
+    assert np.max(np.abs(np.asarray(w) - exact)) < 1e-9
+    v = np.asarray(v.cpu() if hasattr(v, "cpu") else v)
+    assert np.max(np.abs(v @ v.T - np.eye(nev))) < 1e-10
+    op.close()
