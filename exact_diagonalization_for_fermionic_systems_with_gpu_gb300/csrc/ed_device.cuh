@@ -17,6 +17,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "ed_limbs.hpp"
+
 namespace ed {
 namespace dev {
 
@@ -123,7 +125,6 @@ __device__ __forceinline__ i128 mul_wide(int64_t a, int64_t b) {
 // partial products.  Where the |c| of a sum total at most 2^61, the h H and l H sums
 // stay below 2^61 + n 2^27 each and the h L and l L sums below n 2^54, so limb_carry
 // is due every kLimbRun terms (128: all below 2^62.6).
-constexpr int kLimbBits = 27;
 constexpr int kLimbRun = 128;
 
 struct LimbSum {

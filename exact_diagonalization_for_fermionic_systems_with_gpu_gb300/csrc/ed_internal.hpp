@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/ed_hubbard.h"
+#include "ed_limbs.hpp"
 #include "ed_tables.hpp"
 
 namespace ed {
@@ -279,10 +280,6 @@ ed_status lanczos_batch_run(ed_op* const* ops, int B, const ed_lanczos_cfg* cfg,
 ed_status ee_bidiag_blocks(int device, cudaStream_t s, const double* blocks, const std::vector<int64_t>& off,
                            const std::vector<int>& mm, const std::vector<int>& nn, const std::vector<int64_t>& svo,
                            std::vector<double>* sv_host, std::vector<char>* handled);
-// Integer coefficients of an exact sum over basis vectors (limb_mac): the real
-// r[0..n) scaled to c_k = round(r_k 2^F), |c_k| < 2^57 and sum |c_k| < 2^61,
-// each split at 27 bits into (high, low); returns F.
-int limb_coefs(const double* r, int n, int32_t* hl);
 void lanczos_basis(void* ws_slot, const int64_t** basis, int64_t* stride, const int** e_dev);
 // The vectors of the last non-stored run on a workspace, regenerated one by
 // one for visit(k, q_k) (ed_lanczos.cu).

@@ -497,3 +497,25 @@ def test_lanczos_batch_sectors(ed, N, qu, qd, B, ring, t_dn):
         assert np.array_equal(al[b][:n], np.array(lz.a)) and np.array_equal(be[b][:n + 1], np.array(lz.b)[:n + 1])
         assert np.array_equal(ev[b], v)
         op.close()
+
+
+@pytest.mark.parametrize("steps", [127, 128, 129, 257])
+@pytest.mark.parametrize("N,qu,qd,near", [(10, 4, 3, False), (11, 3, 3, False), (10, 4, 3, True), (11, 3, 3, True)])
+def test_ritz_sum_long(ed, N, qu, qd, near, steps):
+    """The stored-basis Ritz sum past its carry interval (128 terms), even and
+    odd row counts, against the second-pass sum; near: a start vector 1e-5 from
+    the ground state, whose coefficients fall so fast that a segment ends inside
+    a batch of vectors.  Each sum is off by a rounding of 2^-53 a term and two
+    of the normalisation at most."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    t = L.chain(N, eps=list(philox_uniform(9, N, 1.5)))
+    op = op_for(ed, N, qu, qd, t, t, 3.0)
+    f = None
+    if near:
+        _, f = ed.Lanczos().eigen(op, max_steps=100, mode="fixed", reorth=True, seed=2)
+        f = f + 1e-5 * ed.Lanczos().random_vector(op.rows(), 3)
+    e1, v1 = ed.Lanczos().eigen(op, f, max_steps=steps, mode="fixed", ritz="stored", seed=4)
+    e2, v2 = ed.Lanczos().eigen(op, f, max_steps=steps, mode="fixed", ritz="recompute", seed=4)
+    assert e1 == e2
+    assert np.linalg.norm(v1 - v2) < 2 * (steps + 2) * 2.0**-53
+    op.close()
