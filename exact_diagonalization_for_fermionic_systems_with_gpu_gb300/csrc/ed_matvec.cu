@@ -322,7 +322,9 @@ cudaError_t launch_apply(const ed_op* op, const double* x, double* y, int64_t* x
         MvArgs a = op->mv;
         a.y = y;
         const ApplyArgs f{x, n, xq, d_emax, d_flag, words, reinterpret_cast<unsigned int*>(words + kApplyPart)};
-        return launch_apply_rows(op, a, f, s);
+        const cudaError_t e = launch_apply_rows(op, a, f, s);
+        if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return e;
+        cudaGetLastError();  // fewer SMs here than the device has: the grid would not be resident
     }
     cudaError_t e = launch_emax(x, n, d_emax, d_flag, s);
     if (e == cudaSuccess) e = launch_to_fx(x, n, d_emax, xq, s);
