@@ -1288,8 +1288,8 @@ static ed_status lanczos_multi_run(ed_op* const* ops, int B, const ed_lanczos_cf
 // workspace (the op's) and start vector; then each run's T and Ritz vector as
 // lanczos_run forms them from the stored basis.  Operators that share their
 // hopping tables (real, one class, gather schedule, 2 <= B <= kLzBatchMax) run
-// in k_lz_batch; any other mix of sectors and kinds in k_lz_multi
-// (ED_LZ_BATCH=multi sends every batch there).
+// in k_lz_batch; any other mix of sectors and kinds, and a batch whose grid cannot
+// be resident, in k_lz_multi (ED_LZ_BATCH=multi sends every batch there).
 ed_status lanczos_batch_run(ed_op* const* ops, int B, const ed_lanczos_cfg* cfg, const double* starts, int start_mem,
                             double* evecs, int evec_mem, double* alpha_h, double* beta_h, ed_lanczos_result* res,
                             cudaStream_t s) {
@@ -1374,7 +1374,9 @@ ed_status lanczos_batch_run(ed_op* const* ops, int B, const ed_lanczos_cfg* cfg,
         if (le != cudaSuccess) {
             cudaGetLastError();
             cudaStreamSynchronize(s);
-            return le == cudaErrorNotSupported || le == cudaErrorCooperativeLaunchTooLarge ? ED_ERR_NOT_BUILT : ED_ERR_CUDA;
+            if (le == cudaErrorNotSupported || le == cudaErrorCooperativeLaunchTooLarge)  // a CTA an SM of 1,024 threads
+                return lanczos_multi_run(ops, B, cfg, starts, start_mem, evecs, evec_mem, alpha_h, beta_h, res, s);
+            return ED_ERR_CUDA;
         }
         ++launches;
     }

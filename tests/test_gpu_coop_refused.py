@@ -78,3 +78,9 @@ def run(tmp_path, what, refuse):
 
 def test_apply_without_cooperative_launch(ed, tmp_path):
     run(tmp_path, "apply", 1)
+
+
+def test_batch_without_its_own_grid(ed, tmp_path):
+    """The batch kernel's blocks of 1,024 threads refused: k_lz_multi, whose
+    blocks are smaller."""
+    run(tmp_path, "batch", 1024)
