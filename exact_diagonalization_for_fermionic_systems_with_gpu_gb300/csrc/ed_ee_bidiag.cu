@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/ed_hubbard.h"
+#include "ed_ee_plan.hpp"
 #include "ed_internal.hpp"
 #include "ed_tridiag.hpp"
 
@@ -44,19 +45,7 @@ struct EeJob {
     int64_t de;   // d at dd + de (n values), e at ee + de (n - 1 values)
 };
 
-// Rows are summed in kBdGroups fixed groups combined in a binary tree, whatever
-// the cluster size, so that a block's result does not depend on how many CTAs
-// it got (and a state's not on the batch it came in).
-constexpr int kBdGroups = 32;
 constexpr int kBdChunk = 8;  // rows of an update unit
-
-int bd_group_rows(int m) { return (m + kBdGroups - 1) / kBdGroups; }
-
-// dynamic shared memory (doubles) of a CTA holding G groups of an m x n block
-size_t bd_smem_doubles(int m, int n, int G) {
-    const size_t R = (size_t)bd_group_rows(m) * G;
-    return R * n + (size_t)G * n + 5 * (size_t)n + 2 + R + 2;
-}
 
 // LAPACK dlarfg convention: H = I - tau v v^T, v_0 = 1, H [alpha; x] = [beta; 0]
 __device__ __forceinline__ void bd_reflector(double alpha, double xnorm2, double* beta, double* tau, double* scale) {
@@ -91,21 +80,22 @@ __global__ void __launch_bounds__(kBdThreads, 1) k_ee_bidiag(const EeJob* __rest
                                                              double* __restrict__ dd, double* __restrict__ ee) {
     cg::cluster_group cl = cg::this_cluster();
     constexpr int G = kBdGroups / CS;  // groups of this CTA
+    static_assert(G >= 2, "wv lies on group 1's sums");
     const int rank = (int)cl.block_rank();
     const EeJob J = jobs[blockIdx.x / CS];
     const int m = J.m, n = J.n;
-    const int Rg = (m + kBdGroups - 1) / kBdGroups, R = Rg * G;
+    const int Rg = bd_group_rows(m), R = Rg * G;
     const int r0 = min(m, rank * R), r1 = min(m, r0 + R);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     extern __shared__ double sm[];
     double* slab = sm;                    // own rows, row-major, stride n
     double* pg = slab + (size_t)R * n;    // [g][j]: group g's part of the column sums
-    double* part = pg + (size_t)G * n;    // [j] = sum over own rows i > k of A_ik A_ij, j >= k
-    double* rowk = part + n + 1;          // row k (columns >= k), written by its owner
-    double* wv = rowk + n;                // tau w_j of the left reflector
-    double* ubuf = wv + n;                // right reflector u_j (j > k), tau' at [n]
-    double* uu = ubuf + n + 1;            // local copy of u
-    double* zz = uu + n;                  // v_i of the left reflector, then tau' z_i of the right one
+    double* part = pg;                    // [j] = sum over own rows i > k of A_ik A_ij, j >= k (on group 0's)
+    double* wv = pg + n;                  // tau w_j of the left reflector (on group 1's, read by then)
+    double* uu = wv;                      // local copy of u, once wv has been used
+    double* rowk = pg + (size_t)G * n;    // row k (columns >= k), written by its owner
+    double* ubuf = rowk + n;              // right reflector u_j (j > k), tau' at [n]
+    double* zz = ubuf + n + 1;            // v_i of the left reflector, then tau' z_i of the right one
     double* sc = zz + R;                  // tau, scale of the left reflector
     const double* src = blocks + J.off;
     for (int64_t idx = tid; idx < (int64_t)(r1 - r0) * n; idx += kBdThreads) {
@@ -265,25 +255,6 @@ cudaStream_t bd_stream(int device, int i) {
         st[device].push_back(x);
     }
     return st[device][i];
-}
-
-// Cluster size (log2) of an m x n block that is `share` times the largest one's
-// work when that gets `top` CTAs: in proportion to the work, and large enough
-// for the rows to fit the CTAs' shared memory (kBdSizes: it fits none).
-constexpr int kBdSizes = 5;  // cluster sizes 1, 2, 4, 8, 16
-
-static int bd_cluster(int m, int n, double share, int top, size_t cap) {
-    int g = 0;
-    while (g < kBdSizes - 1 && (double)(1 << g) < top * share) ++g;
-    while (g < kBdSizes && bd_smem_doubles(m, n, kBdGroups >> g) > cap) ++g;
-    return g;
-}
-
-// Time of a block on 2^g CTAs: 7.5 us of barriers and scalar code a step and
-// 2.4e9 multiply-adds/s a CTA (300 x 300 on 16, 8 and 4 CTAs: 3.32, 3.98, 5.83 ms).
-static double bd_seconds(int m, int n, int g) {
-    const double fma = 2.0 * n * n * ((double)m - n / 3.0);
-    return 7.5e-6 * n + fma / (2.4e9 * (1 << g));
 }
 
 // Singular values of the blocks that fit the cluster kernel: handled[k] = 1

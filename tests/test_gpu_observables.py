@@ -379,3 +379,21 @@ def test_entropy_independent_of_cluster_size(ed, monkeypatch, N, qu, qd, a):
     ref = ob.entanglement_entropy(op, psi[0], range(a))
     assert abs(one[0][0] - ref[0]) < 1e-8 and abs(one[0][1] - ref[1]) < 1e-8
     op.close()
+
+
+def test_entropy_blocks_at_the_cluster_limit(ed, monkeypatch):
+    """A 14-site cut of six sites, whose 1960 x 225 blocks fill the shared memory
+    of 16 CTAs: the same bits alone and in a batch, and gesvd's entropies to 1e-8."""
+    import torch
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L, observables as ob
+    t = L.chain(14, periodic=False)
+    op = ed.Hubbard(ed.H_TBq(14, 6).extend(t), ed.H_TBq(14, 6).extend(t), 1.0)
+    psi = torch.randn((2, op.rows()), dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    psi /= torch.linalg.vector_norm(psi, dim=1, keepdim=True)
+    svn, sref = ob.entanglement_entropy_batch(op, psi, range(6))
+    one = ob.entanglement_entropy(op, psi[0], range(6))
+    assert one == (svn[0], sref[0])
+    monkeypatch.setenv("ED_EE_METHOD", "gesvd")
+    ref = ob.entanglement_entropy(op, psi[0], range(6))
+    assert abs(one[0] - ref[0]) < 1e-8 and abs(one[1] - ref[1]) < 1e-8
+    op.close()

@@ -154,3 +154,19 @@ def test_bidiag_singular_values_against_numpy(edlib, k):
     assert np.max(np.abs(s - ref)) < 8e-16 * n * ref[0]
     if k == 5:  # graded values keep about eps * |B| absolute accuracy
         assert np.max(np.abs(s - ref)) < 1e-15
+
+
+def test_entanglement_block_plan(tmp_path):
+    """Cluster sizes of the entanglement blocks (tests/cpp/ee_plan_check.cpp)."""
+    import shutil
+    import subprocess
+    from conftest import ROOT
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    csrc = ROOT / "exact_diagonalization_for_fermionic_systems_with_gpu_gb300" / "csrc"
+    exe = tmp_path / "ee_plan_check"
+    subprocess.run([cxx, "-std=c++17", "-O2", "-I", str(csrc), str(ROOT / "tests/cpp/ee_plan_check.cpp"), "-o",
+                    str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.endswith(" ok\n"), r.stdout
