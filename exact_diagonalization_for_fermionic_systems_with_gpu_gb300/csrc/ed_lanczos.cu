@@ -746,10 +746,10 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
     // plan chose the persistent kernel.
     const bool pick = op->lz_mode == 2 || (op->lz_mode == 0 && !op->pair);
     bool fused = op->tma_smem > 0 && !cfg->reorth && !prof && !never && (force || pick);
-    // Reorthogonalised runs of small sectors: all steps in one cooperative
-    // launch (ed_lanczos_reorth.cu).
-    bool fused_reorth = cfg->reorth && !op->striped && !prof && !never && max_steps <= kReorthMaxSteps &&
-                        DW <= kReorthMaxN;
+    // Reorthogonalised runs of small sectors: the steps, or the first ones, in
+    // one cooperative launch (ed_lanczos_reorth.cu).
+    const int reorth_end = std::min(max_steps, reorth_launch_steps(DW, !op->cplx && op->mv_fast));
+    bool fused_reorth = cfg->reorth && !op->striped && !prof && !never && max_steps <= kReorthMaxSteps;
     int steps_run = 0;
     int n_fused = 0;  // persistent launches
     int j = 0;
@@ -827,9 +827,9 @@ ed_status lanczos_run(ed_op* op, void** ws_slot, const ed_lanczos_cfg* cfg, cons
                 break;
             }
             j = j1;
-        } else if (fused_reorth) {
-            const int j1 = (cfg->mode == ED_LANCZOS_REFERENCE || stop_beta >= 0.0) ? std::min(max_steps, (j / 10 + 1) * 10)
-                                                                                  : max_steps;
+        } else if (fused_reorth && j < reorth_end) {
+            const int j1 = (cfg->mode == ED_LANCZOS_REFERENCE || stop_beta >= 0.0) ? std::min(reorth_end, (j / 10 + 1) * 10)
+                                                                                  : reorth_end;
             LZ_CK(cudaMemsetAsync(w->gbar, 0, kFusedSync, s));
             LZ_CK(cudaMemsetAsync(w->dot_lo, 0, sizeof(unsigned long long) * 6 * max_steps, s));
             LzReorthArgs ra{w->basis, w->stride, j, j1, DW, lz, w->gbar,

@@ -99,7 +99,25 @@ struct LzFusedArgs {
 // Arguments of the reorthogonalised run in one launch (k_lz_reorth_run):
 // steps j0 .. j1-1 on the stored basis.
 constexpr int kReorthMaxSteps = 1024;        // coefficients of a pass held in shared memory
-constexpr int64_t kReorthMaxN = 1LL << 20;   // stored values up to which one launch is the faster form
+
+// Steps of a reorthogonalised run that one launch does faster than the per-step
+// kernels, n stored values: the steps after them take the per-step kernels, whose
+// dots read a basis larger than L2 at its bandwidth with more warps.  Us a step,
+// launch / per-step kernels, around step 20, 90, 175, 250, 350 and 500:
+//   one class, real: 63,504 values 33/82, 75/128, 131/216, 216/310, 328/424, 495/589;
+//   245,025 67/126, 342/382, 593/670, 857/925, 1230/1254, 1847/1745; 457,380 99/165,
+//   569/623, 1074/1113, 1606/1547, 2300/2113, 3555/2961; 853,776 202/277, 1036/1063,
+//   2138/1937, 3299/2703, 4790/3712, 7407/5222: the lines cross near 1e8 / n.
+//   complex or several classes (a general row sum an element instead of the row
+//   engine's): 48,400 36/84, 85/113, 121/157, 169/226, 281/298, 431/400; 217,800
+//   86/120, 350/351, 595/616, 813/851, 1071/1156, 1630/1603; 245,025 88/142, 406/393;
+//   392,040 127/169, 618/555; 490,050 187/186, 792/668; 784,080 342/278, 1264/1009.
+constexpr int64_t kReorthMaxN = 1LL << 20;
+inline int reorth_launch_steps(int64_t n, bool one_class_real) {
+    if (n > kReorthMaxN) return 0;
+    if (one_class_real) return (int)(100000000 / n);
+    return n <= 220000 ? 400 : (n <= 450000 ? (int)(10000000 / n) : 0);
+}
 
 struct LzReorthArgs {
     int64_t* basis;            // slot j at basis + j * stride

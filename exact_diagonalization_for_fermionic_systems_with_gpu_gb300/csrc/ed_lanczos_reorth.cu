@@ -18,9 +18,10 @@
 // scalar code is that of the per-step kernels, so alpha, beta and the vectors
 // equal theirs bit for bit.  What is left is the barriers (1.9 to 4.5 us
 // each with the reductions before them) and FP64 scalar code (1.7 us for the
-// axpy coefficients, 1.8 us for those of a pass).  Us a step,
-// per-step kernels and this one: 400 rows 62 / 23, 4,900 rows 69 / 25, 63,504
-// rows 102 / 49, 213,444 rows 188 / 127, 853,776 rows 466 / 393.
+// axpy coefficients, 1.8 us for those of a pass).  Us a step of
+// 100, per-step kernels and this one: 400 rows 62 / 23, 4,900 rows 69 / 25, 63,504
+// rows 102 / 49, 213,444 rows 188 / 127, 853,776 rows 466 / 393; longer runs of
+// large sectors go over to the per-step kernels (reorth_launch_steps).
 // Vectors written in the launch are read through L2; barriers
 // are bounded (grid_sync).
 #include <cuda_runtime.h>

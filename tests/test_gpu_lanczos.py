@@ -519,3 +519,31 @@ def test_ritz_sum_long(ed, N, qu, qd, near, steps):
     assert e1 == e2
     assert np.linalg.norm(v1 - v2) < 2 * (steps + 2) * 2.0**-53
     op.close()
+
+
+@pytest.mark.parametrize("case", ["one_class", "complex", "classes", "reference"])
+def test_reorth_goes_over_to_per_step(ed, monkeypatch, case):
+    """Reorthogonalised runs of large sectors: the first steps in one launch, the
+    others by the per-step kernels (nine launches a step), with the bits of a
+    run that takes those from the start; the stop test on both sides."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    N, qu, qd, steps, mode, per_step = 12, 6, 6, 125, "fixed", 8  # 853,776 values: 117 steps in one launch
+    t = L.chain(12, eps=list(philox_uniform(6, 12, 1.0)))
+    if case == "complex":
+        t, qu, qd, steps, per_step = L.kagome12(flux=0.4), 3, 5, 40, 12  # 348,480 values: 28
+    elif case == "classes":
+        t, qu, qd, steps, per_step = L.lieb12(list(philox_uniform(8, 12, 0.5) + 1.0)), 4, 4, 50, 10  # 245,025 values: 40
+    elif case == "reference":
+        t, qu, qd, steps, mode, per_step = L.kagome12(flux=0.4), 3, 5, 100, "reference", 30
+    got = {}
+    for form in ("default", "steps"):
+        monkeypatch.setenv("ED_LZ_FUSED", "0") if form == "steps" else monkeypatch.delenv("ED_LZ_FUSED", raising=False)
+        op = op_for(ed, N, qu, qd, t, t, 4.0)
+        lz = ed.Lanczos()
+        e0, v = lz.eigen(op, max_steps=steps, mode=mode, ritz="stored", reorth=True, seed=5)
+        r = lz.result
+        got[form] = (e0, lz.a, lz.b, r.steps, r.status, r.min_bits, r.converged, r.residual), v, r.launches
+        op.close()
+    assert got["default"][0] == got["steps"][0]
+    assert np.array_equal(got["default"][1], got["steps"][1])
+    assert 9 * per_step <= got["default"][2] < got["steps"][2]
