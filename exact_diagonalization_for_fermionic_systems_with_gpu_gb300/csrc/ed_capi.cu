@@ -183,9 +183,7 @@ ed_status build_spin_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bo
 
 // A schedule of a table built through the cache, kept in its entry.
 template <typename S, typename F>
-bool schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx, int SpinEntry::*state,
-                     S SpinEntry::*kept, S* out, const F& build) {
-    const SpinKey k = spin_key(b.n_sites, b.n_part, cplx, t, nt);
+bool schedule_cached(const SpinKey& k, int SpinEntry::*state, S SpinEntry::*kept, S* out, const F& build) {
     {
         std::lock_guard<std::mutex> g(g_spin_mu);
         for (SpinEntry& e : g_spin_cache)
@@ -207,13 +205,26 @@ bool schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx
 }
 
 // The row engine's gather schedule.
-bool gather_schedule_cached(const ed::SpinBasis& b, const ed_term* t, int nt, bool cplx, const ed::SpinTable& td,
-                            ed::GatherSchedule* gs, std::string* err) {
-    return schedule_cached(b, t, nt, cplx, &SpinEntry::sched_state, &SpinEntry::sched, gs,
+bool gather_schedule_cached(const SpinKey& k, const ed::SpinTable& td, ed::GatherSchedule* gs, std::string* err) {
+    return schedule_cached(k, &SpinEntry::sched_state, &SpinEntry::sched, gs,
                            [&] { return ed::build_gather_schedule(td, gs, err); });
 }
 
+// The row pairs' (adjacent: an even count, part of the key).
+bool pair_schedule_cached(const SpinKey& k, const ed::SpinTable& td, ed::PairSchedule* g) {
+    std::string err;
+    return schedule_cached(k, &SpinEntry::pair_state, &SpinEntry::pair, g,
+                           [&] { return ed::build_pair_schedule(td, td.count % 2 == 0, g, &err); });
+}
+
 }  // namespace
+
+// The Lanczos workspace pointer rides on the op (opaque to the header), and the
+// cache's key of the down table.
+struct ed_op_ext : ed_op {
+    OpExtra extra;
+    SpinKey dn_key;
+};
 
 constexpr int kDegreeBlock = 256;  // columns reordered by hop count within each block
 
@@ -294,14 +305,17 @@ static bool prefer_pair(const ed_op* op) {
 }
 
 static ed_status set_pair(ed_op* op, const ed::PairSchedule& g) {
-    cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);  // of an upload that failed
-    op->d_pairWords = nullptr;
-    op->d_pairSteps = op->d_pairNeg = nullptr;
-    if (upload(&op->d_pairWords, g.words.data(), g.words.size()) != cudaSuccess ||
-        upload(&op->d_pairSteps, g.steps.data(), g.steps.size()) != cudaSuccess ||
-        upload(&op->d_pairNeg, g.negcnt.data(), g.negcnt.size()) != cudaSuccess)
-        return ED_ERR_ALLOC;
-    op->pair_args = {op->d_pairWords, op->d_pairSteps, op->d_pairNeg, g.groups, (int)g.blocks, (int)g.zbase, g.sign};
+    cudaFree(op->d_pairTab);  // of an upload that failed
+    op->d_pairTab = nullptr;
+    // one upload: words (512 bytes a group of a half block), steps, negative counts
+    const size_t at_steps = g.words.size() * sizeof(uint16_t), at_neg = at_steps + g.steps.size();
+    std::vector<uint8_t> all(at_neg + g.negcnt.size());
+    std::memcpy(all.data(), g.words.data(), at_steps);
+    std::copy(g.steps.begin(), g.steps.end(), all.begin() + at_steps);
+    std::copy(g.negcnt.begin(), g.negcnt.end(), all.begin() + at_neg);
+    if (upload(&op->d_pairTab, all.data(), all.size()) != cudaSuccess) return ED_ERR_ALLOC;
+    op->pair_args = {reinterpret_cast<const uint16_t*>(op->d_pairTab), op->d_pairTab + at_steps, op->d_pairTab + at_neg,
+                     g.groups, (int)g.blocks, (int)g.zbase, g.sign};
     op->pair_smem = ed::pair_smem_bytes(g.zbase);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device);
@@ -314,22 +328,14 @@ static ed_status set_pair(ed_op* op, const ed::PairSchedule& g) {
 
 // Plans and uploads the row-pair matvec where two rows fit shared memory;
 // leaves op->pair false otherwise.
-static ed_status plan_pair(ed_op* op, const ed_term* dn_terms, int n_dn_terms) {
+static ed_status plan_pair(ed_op_ext* op) {
     if (ed::pair_smem_bytes((op->dimDN + 7) / 8 * 8) == 0) return ED_OK;
     ed::PairSchedule g;
-    std::string err;
-    if (!schedule_cached(op->bdn, dn_terms, n_dn_terms, false, &SpinEntry::pair_state, &SpinEntry::pair, &g,
-                         [&] { return ed::build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err); }))
-        return ED_OK;
+    if (!pair_schedule_cached(op->dn_key, op->tdn, &g)) return ED_OK;
     const ed_status st = set_pair(op, g);
     op->pair = st == ED_OK;
     return st;
 }
-
-// The Lanczos workspace pointer rides on the op (opaque to the header).
-struct ed_op_ext : ed_op {
-    OpExtra extra;
-};
 
 namespace ed {
 // The row-pair schedule of an operator that its matvec does not use (the batched
@@ -338,8 +344,7 @@ bool ensure_pair(ed_op* op) {
     if (op->pair_smem > 0) return true;
     if (pair_smem_bytes((op->dimDN + 7) / 8 * 8) == 0) return false;
     PairSchedule g;
-    std::string err;
-    return build_pair_schedule(op->tdn, op->dimDN % 2 == 0, &g, &err) && set_pair(op, g) == ED_OK;
+    return pair_schedule_cached(static_cast<ed_op_ext*>(op)->dn_key, op->tdn, &g) && set_pair(op, g) == ED_OK;
 }
 
 void** lanczos_ws_slot(ed_op* op) { return &static_cast<ed_op_ext*>(op)->extra.lz_ws; }
@@ -485,6 +490,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     ed_status st = build_spin_cached(op->bup, desc->up_terms, desc->n_up_terms, cplx, &op->tup, &err);
     if (st == ED_OK) st = build_spin_cached(op->bdn, desc->dn_terms, desc->n_dn_terms, cplx, &op->tdn, &err);
     if (st != ED_OK) { delete op; return st; }
+    op->dn_key = spin_key(N, desc->n_dn, cplx, desc->dn_terms, desc->n_dn_terms);
 
     // ---- fixed-point scale of the coefficients ----------------------------
     const ed::SpinTable& tu = op->tup;
@@ -670,7 +676,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     if (!cplx && td.coef.size() <= 1 && !std::getenv("ED_NO_SCHED")) {
         ed::GatherSchedule gs;
         std::string serr;
-        if (gather_schedule_cached(op->bdn, desc->dn_terms, desc->n_dn_terms, cplx, td, &gs, &serr)) {
+        if (gather_schedule_cached(op->dn_key, td, &gs, &serr)) {
             if (upload(&op->d_dnSched, gs.ent.data(), gs.ent.size()) != cudaSuccess ||
                 upload(&op->d_dnSteps, gs.steps32.data(), gs.steps32.size()) != cudaSuccess) {
                 ed_op_destroy(op);
@@ -708,7 +714,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     if (want != "generic" && want != "striped" && want != "pair") op->tma_smem = ed::tma_plan(op, &a);
     if (op->tma_smem > 0) op->tma_grid = ed::tma_grid(op);
     if (!cplx && op->mv_fast && (want.empty() || want == "pair") && prefer_pair(op)) {
-        const ed_status pst = plan_pair(op, desc->dn_terms, desc->n_dn_terms);
+        const ed_status pst = plan_pair(op);
         if (pst != ED_OK) {
             ed_op_destroy(op);
             return pst;
@@ -762,7 +768,7 @@ ed_status ed_op_destroy(ed_op* op) {
     cudaFree(op->d_permDN); cudaFree(op->d_sched16); cudaFree(op->d_steps32); cudaFree(op->d_dDNqP);
     cudaFree(op->d_stDNp); cudaFree(op->d_sdn); cudaFree(op->d_negDN);
     cudaFree(op->d_clsSched);
-    cudaFree(op->d_pairWords); cudaFree(op->d_pairSteps); cudaFree(op->d_pairNeg);
+    cudaFree(op->d_pairTab);
     cudaFree(op->d_dUPq); cudaFree(op->d_dDNq); cudaFree(op->d_stUP); cudaFree(op->d_stDN);
     cudaFree(op->d_xq); cudaFree(op->d_emax); cudaFree(op->d_io);
     if (op->h_stage) cudaFreeHost(op->h_stage);

@@ -204,8 +204,7 @@ struct ed_op {
     bool pair = false;
     ed::PairArgs pair_args{};
     int pair_smem = 0, pair_nbuf = 1, pair_threads = 0, pair_grid = 0;  // bytes of a row pair, pairs staged, launch
-    uint16_t* d_pairWords = nullptr;
-    uint8_t *d_pairSteps = nullptr, *d_pairNeg = nullptr;
+    uint8_t* d_pairTab = nullptr;  // the pair schedule's three tables
     std::string last_error;
 };
 

@@ -1307,18 +1307,16 @@ ed_status lanczos_batch_run(ed_op* const* ops, int B, const ed_lanczos_cfg* cfg,
             homogeneous = false;
     }
     const char* force = std::getenv("ED_LZ_BATCH");
-    if (homogeneous) {
-        if (cudaSetDevice(op0->device) != cudaSuccess) return ED_ERR_CUDA;
-        homogeneous = ensure_pair(op0);
-    }
-    if (!homogeneous || (force && std::strcmp(force, "multi") == 0))
-        return lanczos_multi_run(ops, B, cfg, starts, start_mem, evecs, evec_mem, alpha_h, beta_h, res, s);
-    if (B == 1) {
+    const bool multi = force && std::strcmp(force, "multi") == 0;
+    if (homogeneous && B == 1 && !multi) {
         // a run by itself: the single-run kernels (10-site 5+5 18.2 -> 12.4 us a step)
         ed_lanczos_cfg one = *cfg;
         one.profile = 0;
         return lanczos_run(op0, lanczos_ws_slot(op0), &one, starts, start_mem, evecs, evec_mem, alpha_h, beta_h, res, s);
     }
+    if (cudaSetDevice(op0->device) != cudaSuccess) return ED_ERR_CUDA;
+    if (!homogeneous || multi || !ensure_pair(op0))
+        return lanczos_multi_run(ops, B, cfg, starts, start_mem, evecs, evec_mem, alpha_h, beta_h, res, s);
     const int64_t DW = op0->D;
     const int max_steps = cfg->max_steps;
     const bool want_ritz = cfg->ritz == ED_RITZ_STORED && evecs;
