@@ -20,6 +20,7 @@
 #include "../../include/ed_hubbard.h"
 #include "ed_device.cuh"
 #include "ed_internal.hpp"
+#include "ed_tridiag.hpp"
 
 namespace ed {
 using namespace dev;
@@ -710,7 +711,8 @@ namespace {
 // <x|(H - E0)^-1|x> for a device vector x orthogonal to the ground level:
 // -|x|^2 g(0), with g from the continued fraction of a `steps`-step Lanczos
 // run of H started at x, at w = 0 without broadening:
-// g(0) = 1/(E0 - a0 - b1^2/(E0 - a1 - ...)).
+// g(0) = 1/(E0 - a0 - b1^2/(E0 - a1 - ...)), the ground level left out where
+// rounding has brought it back (tridiag_resolvent).
 ed_status resolvent_form(ed_op* H, const double* x, double e0, int steps, double* out, cudaStream_t s) {
     std::vector<double> a(steps), bt(steps + 1);
     ed_lanczos_cfg lc;
@@ -722,9 +724,7 @@ ed_status resolvent_form(ed_op* H, const double* x, double e0, int steps, double
     ed_lanczos_result lr;
     const ed_status st = ed_lanczos_run(H, &lc, x, ED_MEM_DEVICE, nullptr, ED_MEM_DEVICE, a.data(), bt.data(), &lr, s);
     if (st != ED_OK) return st;
-    const int m = lr.steps;
-    long double gz = 1.0L / ((long double)e0 - a[m - 1]);
-    for (int i = m - 2; i >= 0; --i) gz = 1.0L / ((long double)e0 - a[i] - gz * (long double)bt[i + 1] * bt[i + 1]);
+    const long double gz = ed::tridiag_resolvent(lr.steps, a.data(), bt.data() + 1, e0);
     *out = -(double)((long double)bt[0] * bt[0] * gz);
     return ED_OK;
 }
@@ -839,10 +839,7 @@ ed_status ed_response_batch(ed_op* const* H, ed_op* const* dH, ed_op* const* d2H
             for (int i = 0; i < n && st == ED_OK; ++i) {
                 const double* ai = a.data() + (size_t)i * steps;
                 const double* bi = bt.data() + (size_t)i * (steps + 1);
-                const int m = lr[i].steps;
-                long double gz = 1.0L / ((long double)e0[i] - ai[m - 1]);
-                for (int k = m - 2; k >= 0; --k)
-                    gz = 1.0L / ((long double)e0[i] - ai[k] - gz * (long double)bi[k + 1] * bi[k + 1]);
+                const long double gz = ed::tridiag_resolvent(lr[i].steps, ai, bi + 1, e0[i]);
                 const double resp = -(double)((long double)bi[0] * bi[0] * gz) / nn[i];
                 double d2[2] = {0.0, 0.0};
                 st = ed_op_expect(d2H[i], psis + off[i], ED_MEM_DEVICE, d2, stream);

@@ -197,6 +197,38 @@ bool tridiag_eigen_rotations(int n, const double* a_in, const double* off, std::
     return true;
 }
 
+long double tridiag_resolvent(int n, const double* a, const double* off, double z) {
+    long double g = 1.0L / ((long double)z - a[n - 1]);
+    double norm = std::fabs(a[n - 1]);
+    for (int k = n - 2; k >= 0; --k) {
+        g = 1.0L / ((long double)z - a[k] - g * (long double)off[k] * off[k]);
+        norm = std::max(norm, std::fabs(a[k]) + 2.0 * std::fabs(off[k]));
+    }
+    // Four points at 45 degrees on a circle of radius rho, two of them by symmetry.
+    // A pole at distance d outside it enters the mean as at z, to (rho / d)^4; those
+    // inside not at all, and the mean of value x radius is their weight: a level
+    // that close with a weight to be seen is one, and stays.
+    const double rho = 1e-10 * norm, h = rho * std::sqrt(0.5);
+    if (!(rho > 0.0)) return g;
+    double mean = 0.0, weight = 0.0;
+    for (const double x : {h, -h}) {
+        // (re, im) of 1 / (z + x + i h - a_k - off_k^2 (re, im))
+        double re = 0.0, im = 0.0;
+        for (int k = n - 1; k >= 0; --k) {
+            const double b2 = k + 1 < n ? off[k] * off[k] : 0.0;
+            const double dr = (z - a[k]) + x - b2 * re, di = h - b2 * im;
+            const double d2 = dr * dr + di * di;
+            re = dr / d2;
+            im = -di / d2;
+        }
+        mean += 0.5 * re;
+        weight += 0.5 * (re * x - im * h);
+    }
+    if (!(std::fabs(weight) < 1e-12)) return g;
+    // 1e-11: the mean, in FP64, is good to about 1e-13
+    return std::fabs((double)g - mean) <= 1e-11 * std::fabs(mean) ? g : (long double)mean;
+}
+
 // v <- Z^T v: G_1^T first
 void tri_apply_zt(const std::vector<TriRot>& rots, double* v) {
     for (const TriRot& g : rots) {

@@ -170,3 +170,19 @@ def test_entanglement_block_plan(tmp_path):
                     str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.endswith(" ok\n"), r.stdout
+
+
+def test_resolvent_leaves_the_ground_level_out(tmp_path):
+    """The linear response's resolvent (tests/cpp/resolvent_check.cpp)."""
+    import shutil
+    import subprocess
+    from conftest import ROOT
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    csrc = ROOT / "exact_diagonalization_for_fermionic_systems_with_gpu_gb300" / "csrc"
+    exe = tmp_path / "resolvent_check"
+    subprocess.run([cxx, "-std=c++17", "-O2", "-I", str(csrc), str(ROOT / "tests/cpp/resolvent_check.cpp"),
+                    str(csrc / "ed_tridiag.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
