@@ -516,6 +516,7 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     a.Uq = (int64_t)std::llrint(std::ldexp(desc->U, Fc));
     a.nclsUP = (int)tu.coef.size();
     a.nclsDN = (int)td.coef.size();
+    op->mv_fast = a.nclsUP <= 1 && a.nclsDN <= 1;
     for (int c = 0; c < a.nclsUP; ++c) {
         a.coefUP[2 * c] = (int64_t)std::llrint(std::ldexp(tu.coef[c].real(), Fc));
         a.coefUP[2 * c + 1] = (int64_t)std::llrint(std::ldexp(tu.coef[c].imag(), Fc));
@@ -571,30 +572,32 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
          upload(&op->d_dnPtr, dn_ptr.data(), dn_ptr.size()) == cudaSuccess &&
          upload(&op->d_dnEntC, dn_ent.data(), dn_ent.size()) == cudaSuccess;
     if (!ok) { ed_op_destroy(op); return ED_ERR_ALLOC; }
-    // class segments for multi-class tables with at most kSegCls classes
-    auto segments = [](const ed::SpinTable& t, std::vector<uint32_t>* se, std::vector<uint32_t>* sp) {
-        se->assign(t.count, 0u);
-        sp->assign(t.count, 0u);
-        for (int64_t r = 0; r < t.count; ++r) {
-            int k = 0;
-            uint32_t e = 0, p = 0;
-            for (int c = 0; c < ed::kSegCls; ++c) {
-                while (k < t.len[r] && ((t.ent[(size_t)k * t.count + r] >> ed::kClassShift) & ed::kClassMask) == (uint32_t)c &&
-                       !(t.ent[(size_t)k * t.count + r] & ed::kSignBit))
-                    ++k;
-                p |= (uint32_t)k << (8 * c);
-                while (k < t.len[r] && ((t.ent[(size_t)k * t.count + r] >> ed::kClassShift) & ed::kClassMask) == (uint32_t)c)
-                    ++k;
-                e |= (uint32_t)k << (8 * c);
-            }
-            (*se)[r] = e;
-            (*sp)[r] = p;
-        }
-    };
+    // at most kSegCls classes: class segments of the rows (real) or a class
+    // schedule of the columns (complex; without one, and where the row engine
+    // cannot hold two rows, the general path)
+    a.mergeMC = a.perEntry = 0;
     a.upSegE = a.upSegP = a.dnSegE = a.dnSegP = nullptr;
-    a.mergeMC = 0;
-    if ((a.nclsUP > 1 || a.nclsDN > 1) && a.nclsUP <= ed::kSegCls && a.nclsDN <= ed::kSegCls &&
-        !std::getenv("ED_NO_SEG")) {
+    const bool few = a.nclsUP <= ed::kSegCls && a.nclsDN <= ed::kSegCls && !std::getenv("ED_NO_SEG");
+    if (!op->mv_fast && few && !cplx) {
+        auto segments = [](const ed::SpinTable& t, std::vector<uint32_t>* se, std::vector<uint32_t>* sp) {
+            se->assign(t.count, 0u);
+            sp->assign(t.count, 0u);
+            for (int64_t r = 0; r < t.count; ++r) {
+                int k = 0;
+                uint32_t e = 0, p = 0;
+                for (int c = 0; c < ed::kSegCls; ++c) {
+                    while (k < t.len[r] && ((t.ent[(size_t)k * t.count + r] >> ed::kClassShift) & ed::kClassMask) == (uint32_t)c &&
+                           !(t.ent[(size_t)k * t.count + r] & ed::kSignBit))
+                        ++k;
+                    p |= (uint32_t)k << (8 * c);
+                    while (k < t.len[r] && ((t.ent[(size_t)k * t.count + r] >> ed::kClassShift) & ed::kClassMask) == (uint32_t)c)
+                        ++k;
+                    e |= (uint32_t)k << (8 * c);
+                }
+                (*se)[r] = e;
+                (*sp)[r] = p;
+            }
+        };
         std::vector<uint32_t> use, usp, dse, dsp;
         segments(tu, &use, &usp);
         segments(td, &dse, &dsp);
@@ -609,49 +612,46 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
         a.upSegP = op->d_upSegP;
         a.dnSegE = op->d_dnSegE;
         a.dnSegP = op->d_dnSegP;
-        a.mergeMC = (a.nclsUP == a.nclsDN && tu.coef == td.coef) ? 1 : 0;
-        if (cplx) {
-            // the complex row engine's schedule; without one the operator takes
-            // the general path
-            ed::ClassSchedule cs;
-            std::string cerr;
-            if (ed::build_class_schedule(td, &cs, &cerr)) {
-                // one upload: words (64 bytes a step of a block), counts, steps
-                std::vector<uint32_t> all(cs.words.size() / 2 + cs.negcnt.size() + cs.steps4.size());
-                std::memcpy(all.data(), cs.words.data(), cs.words.size() * 2);
-                std::copy(cs.negcnt.begin(), cs.negcnt.end(), all.begin() + cs.words.size() / 2);
-                std::copy(cs.steps4.begin(), cs.steps4.end(), all.begin() + cs.words.size() / 2 + cs.negcnt.size());
-                if (upload(&op->d_clsSched, all.data(), all.size()) != cudaSuccess) {
-                    ed_op_destroy(op);
-                    return ED_ERR_ALLOC;
-                }
-                a.clsSched = reinterpret_cast<const uint16_t*>(op->d_clsSched);
-                a.clsNeg = op->d_clsSched + cs.words.size() / 2;
-                a.clsSteps = a.clsNeg + cs.negcnt.size();
-                a.schedSteps = cs.steps;
-                a.dimDNp = (int)cs.cpad;
-            } else {
-                a.upSegE = a.upSegP = a.dnSegE = a.dnSegP = nullptr;
-            }
-            auto partners = [](const int64_t* coef, int n, int8_t* part) {
-                for (int c = 0; c < ed::kSegCls; ++c) part[c] = (int8_t)c;
-                for (int c = 0; c < n; ++c) {
-                    if (part[c] != c || coef[2 * c + 1] == 0) continue;
-                    for (int q = c + 1; q < n; ++q)
-                        if (part[q] == q && coef[2 * q] == coef[2 * c] && coef[2 * q + 1] == -coef[2 * c + 1]) {
-                            part[c] = (int8_t)q;
-                            part[q] = -1;
-                            break;
-                        }
-                }
-            };
-            partners(a.coefUP, a.nclsUP, a.partUP);
-            partners(a.coefDN, a.nclsDN, a.partDN);
-        }
     }
-    // entries per (row, class) run of the two tables: below 2, a product per
-    // entry replaces the running class sums
-    {
+    // (48 bytes a column: two rows, diagonal and state)
+    if (!op->mv_fast && few && cplx && 48 * op->dimDN < 227 * 1024) {
+        ed::ClassSchedule cs;
+        std::string cerr;
+        if (ed::build_class_schedule(td, &cs, &cerr)) {
+            // one upload: words (64 bytes a step of a block), counts, steps
+            std::vector<uint32_t> all(cs.words.size() / 2 + cs.negcnt.size() + cs.steps4.size());
+            std::memcpy(all.data(), cs.words.data(), cs.words.size() * 2);
+            std::copy(cs.negcnt.begin(), cs.negcnt.end(), all.begin() + cs.words.size() / 2);
+            std::copy(cs.steps4.begin(), cs.steps4.end(), all.begin() + cs.words.size() / 2 + cs.negcnt.size());
+            if (upload(&op->d_clsSched, all.data(), all.size()) != cudaSuccess) {
+                ed_op_destroy(op);
+                return ED_ERR_ALLOC;
+            }
+                a.clsSched = reinterpret_cast<const uint16_t*>(op->d_clsSched);
+            a.clsNeg = op->d_clsSched + cs.words.size() / 2;
+            a.clsSteps = a.clsNeg + cs.negcnt.size();
+            a.schedSteps = cs.steps;
+            a.dimDNp = (int)cs.cpad;
+        }
+        auto partners = [](const int64_t* coef, int n, int8_t* part) {
+            for (int c = 0; c < ed::kSegCls; ++c) part[c] = (int8_t)c;
+            for (int c = 0; c < n; ++c) {
+                if (part[c] != c || coef[2 * c + 1] == 0) continue;
+                for (int q = c + 1; q < n; ++q)
+                    if (part[q] == q && coef[2 * q] == coef[2 * c] && coef[2 * q + 1] == -coef[2 * c + 1]) {
+                        part[c] = (int8_t)q;
+                        part[q] = -1;
+                        break;
+                    }
+            }
+        };
+        partners(a.coefUP, a.nclsUP, a.partUP);
+        partners(a.coefDN, a.nclsDN, a.partDN);
+    }
+    if (ed::seg_kernels(a)) a.mergeMC = (a.nclsUP == a.nclsDN && tu.coef == td.coef) ? 1 : 0;
+    // the general path: entries per (row, class) run of the two tables; below 2, a
+    // product per entry replaces the running class sums
+    if (!op->mv_fast && !ed::seg_kernels(a)) {
         int64_t runs = 0;
         for (const ed::SpinTable* t : {&tu, &td})
             for (int64_t r = 0; r < t->count; ++r) {
@@ -705,7 +705,6 @@ ed_status ed_op_create(ed_op** out, const ed_model_desc* desc, int device) {
     op->stage_smem = row_bytes <= 160 * 1024 ? (int)row_bytes : 0;
     op->grid = ed::matvec_grid(op);
     op->mv_threads = ed::matvec_threads(op->dimDN);
-    op->mv_fast = a.nclsUP <= 1 && a.nclsDN <= 1;
     // kernel choice: the row-staged TMA kernel where the down table fits in
     // shared memory, else the generic kernel; ED_MATVEC=generic forces the
     // generic kernel (tests compare the two)

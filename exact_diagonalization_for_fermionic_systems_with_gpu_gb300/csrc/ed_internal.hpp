@@ -74,16 +74,16 @@ struct MvArgs {
     // Lanczos per-step reduction outputs
     void* lz;             // LzState* (device)
     int step;
-    // class segments of every row (tables with at most kSegCls classes,
+    // class segments of every row (real tables with at most kSegCls classes,
     // entries sorted by class, + before -): byte c of segE[r] is the end of
     // class c's entries in row r, byte c of segP[r] the end of its + entries
-    // (both relative to the row start); null for tables with more classes
+    // (both relative to the row start); null for other tables
     const uint32_t* upSegE;
     const uint32_t* upSegP;
     const uint32_t* dnSegE;
     const uint32_t* dnSegP;
-    // class schedule of the down term (complex operators with class segments;
-    // null otherwise), ed::ClassSchedule
+    // class schedule of the down term (such complex operators; null otherwise),
+    // ed::ClassSchedule
     const uint16_t* clsSched;
     const uint32_t* clsSteps;
     const uint32_t* clsNeg;
@@ -96,6 +96,9 @@ struct MvArgs {
     int64_t coefUP[2 * kMaxCls];
     int64_t coefDN[2 * kMaxCls];
 };
+
+// At most kSegCls classes and several: the kernels that sum class by class.
+inline bool seg_kernels(const MvArgs& a) { return a.upSegE || a.clsSched; }
 
 // FP64 apply in one cooperative launch (k_apply): FX copy of x and the words
 // its grid shares.

@@ -1117,9 +1117,9 @@ ed_status lanczos_replay(ed_op* op, void* ws_slot, int n, const std::function<cu
 
 // Row-engine variant of an operator's persistent Lanczos kernel.
 static int lz_kind(const ed_op* o) {
-    if (o->cplx) return o->mv_fast ? kKindCplxFast : (o->mv.upSegE ? kKindCplxSeg : kKindCplx);
+    if (o->cplx) return o->mv_fast ? kKindCplxFast : (seg_kernels(o->mv) ? kKindCplxSeg : kKindCplx);
     if (o->mv_fast) return o->mv.dnSched ? kKindRealSched : kKindRealFast;
-    return o->mv.upSegE ? kKindRealSeg : kKindReal;
+    return seg_kernels(o->mv) ? kKindRealSeg : kKindReal;
 }
 
 static bool same_tables(const ed_op* a, const ed_op* b) {

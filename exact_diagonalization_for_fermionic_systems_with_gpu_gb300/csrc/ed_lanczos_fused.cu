@@ -548,10 +548,10 @@ cudaError_t launch_lz_fused(const ed_op* op, const LzFusedArgs& f, cudaStream_t 
     const void* fn;
     if (op->cplx)
         fn = op->mv_fast ? (const void*)k_lz_fused<true, true, false>
-             : op->mv.upSegE ? (const void*)k_lz_fused<true, false, false, true>
+             : seg_kernels(op->mv) ? (const void*)k_lz_fused<true, false, false, true>
                              : (const void*)k_lz_fused<true, false, false>;
     else if (!op->mv_fast)
-        fn = op->mv.upSegE ? (const void*)k_lz_fused<false, false, false, true>
+        fn = seg_kernels(op->mv) ? (const void*)k_lz_fused<false, false, false, true>
                            : (const void*)k_lz_fused<false, false, false>;
     else
         fn = op->mv.dnSched ? (const void*)k_lz_fused<false, true, true> : (const void*)k_lz_fused<false, true, false>;

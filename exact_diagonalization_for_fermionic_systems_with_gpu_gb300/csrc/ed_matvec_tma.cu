@@ -144,10 +144,10 @@ __global__ void __launch_bounds__(kTmaThreads, 2) k_apply(const MvArgs a, const 
 static const void* apply_kernel(const ed_op* op) {
     if (op->cplx)
         return op->mv_fast ? (const void*)k_apply<true, true, false>
-               : op->mv.upSegE ? (const void*)k_apply<true, false, false, true>
+               : seg_kernels(op->mv) ? (const void*)k_apply<true, false, false, true>
                                : (const void*)k_apply<true, false, false>;
     if (!op->mv_fast)
-        return op->mv.upSegE ? (const void*)k_apply<false, false, false, true> : (const void*)k_apply<false, false, false>;
+        return seg_kernels(op->mv) ? (const void*)k_apply<false, false, false, true> : (const void*)k_apply<false, false, false>;
     return op->mv.dnSched ? (const void*)k_apply<false, true, true> : (const void*)k_apply<false, true, false>;
 }
 
@@ -226,7 +226,7 @@ int tma_plan(const ed_op* op, MvArgs* a) {
     a->sm_stdn = (int)off;
     off += up128(dimDN * 8);
     // uoff, uent, reduction scratch; the general kernels' coefficient classes
-    const int64_t static_bytes = 2 * kTmaUpStage * 4 + 64 + 24 * 64 + (op->mv_fast || a->upSegE ? 0 : 4 * kMaxCls * 8);
+    const int64_t static_bytes = 2 * kTmaUpStage * 4 + 64 + 24 * 64 + (op->mv_fast || seg_kernels(*a) ? 0 : 4 * kMaxCls * 8);
     if (off + static_bytes > 227 * 1024) return 0;
     return (int)off;
 }
@@ -234,10 +234,10 @@ int tma_plan(const ed_op* op, MvArgs* a) {
 static const void* matvec_kernel(const ed_op* op) {
     if (op->cplx)
         return op->mv_fast ? (const void*)k_matvec_tma<true, true, false>
-               : op->mv.upSegE ? (const void*)k_matvec_tma<true, false, false, true>
+               : seg_kernels(op->mv) ? (const void*)k_matvec_tma<true, false, false, true>
                                : (const void*)k_matvec_tma<true, false, false>;
     if (!op->mv_fast)
-        return op->mv.upSegE ? (const void*)k_matvec_tma<false, false, false, true>
+        return seg_kernels(op->mv) ? (const void*)k_matvec_tma<false, false, false, true>
                              : (const void*)k_matvec_tma<false, false, false>;
     return op->mv.dnSched ? (const void*)k_matvec_tma<false, true, true> : (const void*)k_matvec_tma<false, true, false>;
 }

@@ -509,7 +509,7 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
                         apply_class<CPLX>(ar1, ai1, dr1, di1, a.coefDN, 0, unitD, a.Fc);
                     }
                 }
-            } else if (SEG && CPLX) {
+            } else if constexpr (SEG && CPLX) {
                 // at most kSegCls classes, one sum for each, products at the end.
                 // Up entries (the same for every lane) are loaded four at a time
                 // and added by class; the down schedule's steps go class by
@@ -565,69 +565,40 @@ __device__ __forceinline__ void tma_rows(const MvArgs& a, const TmaSmem& S, cons
                 steps(s2, (ns >> 16) & 0xFFu, (ng >> 16) & 0xFFu);
                 steps(s3, ns >> 24, ng >> 24);
                 class_products(ar0, ai0, s0, s1, s2, s3, a.coefDN, a.partDN, a.nclsDN);
-            } else if (SEG) {
+            } else if constexpr (SEG) {
                 // at most kSegCls classes: class by class over segments taken
                 // from the rows' class-end bytes (+ entries first), the same
                 // loop bounds for every lane in the up row; with equal class
                 // lists the up and down sums of a class share one product.
                 const uint32_t se_u = __ldg(a.upSegE + u), sp_u = __ldg(a.upSegP + u);
+                const uint32_t se = __ldg(a.dnSegE + d0), sp = __ldg(a.dnSegP + d0);
+                const uint32_t q0 = S.dptr[d0];
                 const int ncl = max(a.nclsUP, a.nclsDN);
-#pragma unroll 1
-                for (int cc = 0; cc < (v1 ? 2 : 1); ++cc) {
-                    const uint32_t d = cc ? d1c : d0;
-                    // this column's accumulators, stored into ar0/ai0 or
-                    // ar1/ai1 at the end (not a reference chosen at run time,
-                    // which would put all four in local memory)
-                    i128 ar = 0, ai = 0;
-                    const uint32_t se = __ldg(a.dnSegE + d), sp = __ldg(a.dnSegP + d);
-                    const uint32_t q0 = S.dptr[d];
-                    uint32_t ub = 0, b = 0;
-                    for (int c = 0; c < ncl; ++c) {
-                        int64_t r = 0, i = 0;
-                        if (c < a.nclsUP) {
-                            const uint32_t up = (sp_u >> (8 * c)) & 0xFFu, ue = (se_u >> (8 * c)) & 0xFFu;
-                            for (uint32_t k = ub; k < up; ++k) acc_up<CPLX, COH>(xq, S.uoff[k] + d, r, i);
-                            for (uint32_t k = up; k < ue; ++k) {
-                                int64_t vr, vi;
-                                up_load<CPLX, COH>(xq, S.uoff[k] + d, vr, vi);
-                                r -= vr;
-                                i -= vi;
-                            }
-                            ub = ue;
-                            if (!a.mergeMC) {
-                                apply_class<CPLX>(ar, ai, r, i, a.coefUP, c, unitU, a.Fc);
-                                r = 0;
-                                i = 0;
-                            }
+                uint32_t ub = 0, b = 0;
+                for (int c = 0; c < ncl; ++c) {
+                    int64_t r = 0, none = 0;
+                    if (c < a.nclsUP) {
+                        const uint32_t up = (sp_u >> (8 * c)) & 0xFFu, ue = (se_u >> (8 * c)) & 0xFFu;
+                        for (uint32_t k = ub; k < up; ++k) acc_up<false, COH>(xq, S.uoff[k] + d0, r, none);
+                        for (uint32_t k = up; k < ue; ++k) {
+                            int64_t vr;
+                            up_load<false, COH>(xq, S.uoff[k] + d0, vr, none);
+                            r -= vr;
                         }
-                        if (c < a.nclsDN) {
-                            const uint32_t pc = (sp >> (8 * c)) & 0xFFu, ec = (se >> (8 * c)) & 0xFFu;
-                            for (uint32_t q = q0 + b; q < q0 + pc; ++q) {
-                                const uint32_t col = (S.dent[q] & kColMask) * W;
-                                int64_t vr, vi;
-                                row_elem<CPLX>(xrow, col, vr, vi);
-                                r += vr;
-                                if (CPLX) i += vi;
-                            }
-                            for (uint32_t q = q0 + pc; q < q0 + ec; ++q) {
-                                const uint32_t col = (S.dent[q] & kColMask) * W;
-                                int64_t vr, vi;
-                                row_elem<CPLX>(xrow, col, vr, vi);
-                                r -= vr;
-                                if (CPLX) i -= vi;
-                            }
-                            b = ec;
-                            apply_class<CPLX>(ar, ai, r, i, a.coefDN, c, unitD, a.Fc);
-                        } else if (a.mergeMC) {
-                            apply_class<CPLX>(ar, ai, r, i, a.coefUP, c, unitU, a.Fc);
+                        ub = ue;
+                        if (!a.mergeMC) {
+                            apply_class<false>(ar0, ai0, r, 0, a.coefUP, c, unitU, a.Fc);
+                            r = 0;
                         }
                     }
-                    if (cc) {
-                        ar1 = ar;
-                        ai1 = ai;
-                    } else {
-                        ar0 = ar;
-                        ai0 = ai;
+                    if (c < a.nclsDN) {
+                        const uint32_t pc = (sp >> (8 * c)) & 0xFFu, ec = (se >> (8 * c)) & 0xFFu;
+                        for (uint32_t q = q0 + b; q < q0 + pc; ++q) r += xrow[S.dent[q] & kColMask];
+                        for (uint32_t q = q0 + pc; q < q0 + ec; ++q) r -= xrow[S.dent[q] & kColMask];
+                        b = ec;
+                        apply_class<false>(ar0, ai0, r, 0, a.coefDN, c, unitD, a.Fc);
+                    } else if (a.mergeMC) {
+                        apply_class<false>(ar0, ai0, r, 0, a.coefUP, c, unitU, a.Fc);
                     }
                 }
             } else if (a.perEntry) {

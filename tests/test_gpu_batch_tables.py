@@ -47,3 +47,37 @@ def test_batch_builds_the_tables_it_uses(ed, tmp_path):
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     assert [int(v) for v in r.stdout.split()] == [0, 0, 1, 0]
+
+
+CREATE = r"""
+import ctypes
+import exact_diagonalization_for_fermionic_systems_with_gpu_gb300 as ed
+from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+
+calls = ctypes.CDLL(None).malloc_calls
+
+def made(t):
+    n = calls()
+    op = ed.Hubbard(ed.H_TBq(12, 3).extend(t), ed.H_TBq(12, 4).extend(t), 2.0)
+    return calls() - n
+
+made(L.chain(12))
+many = made(L.lieb12([1.0 + 0.1 * i for i in range(12)]))
+two = made(L.chain(12) + [("H", i, (i + 2) % 12, -0.5, 0.0) for i in range(12)])
+print(two - many, made(L.kagome12(flux=0.3)) - many)
+"""
+
+
+def test_operator_uploads_the_tables_it_uses(ed, tmp_path):
+    """Beyond what every operator has: four segment tables for a few real
+    classes, one class schedule for complex ones."""
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if cc is None:
+        pytest.skip("no C compiler")
+    so = tmp_path / "count_malloc.so"
+    subprocess.run([cc, "-shared", "-fPIC", "-O1", str(ROOT / "tests/cpp/count_malloc.c"), "-o", str(so), "-ldl"],
+                   check=True)
+    r = subprocess.run([sys.executable, "-c", CREATE], env=dict(os.environ, PYTHONPATH=str(ROOT), LD_PRELOAD=str(so)),
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert [int(v) for v in r.stdout.split()] == [4, 1]
