@@ -786,6 +786,8 @@ int ed_op_matvec_kind(const ed_op* op) {
     return op->striped ? ED_MV_TWO_PASS : (op->tma_smem > 0 ? ED_MV_ROWS : ED_MV_GENERIC);
 }
 
+int ed_op_row_pairs(const ed_op* op) { return op && op->pair ? 1 : 0; }
+
 ed_status ed_op_perform(ed_op* op, const double* x, double* y, int mem, void* stream) {
     if (!op || !x || !y || (mem != ED_MEM_HOST && mem != ED_MEM_DEVICE)) return ED_ERR_ARG;
     if (cudaSetDevice(op->device) != cudaSuccess) return ED_ERR_CUDA;

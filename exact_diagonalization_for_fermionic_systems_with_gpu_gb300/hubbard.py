@@ -177,6 +177,7 @@ class Hubbard:
         self.dimDN = int(lib.ed_op_dim_dn(h))
         self.is_complex = bool(lib.ed_op_is_complex(h))
         self.matvec_kind = ("generic", "rows", "two_pass")[lib.ed_op_matvec_kind(h)]
+        self.row_pairs = bool(lib.ed_op_row_pairs(h))  # its applies and steps run on row pairs
 
     # -- Spectra concept (TotalSpin/include/HubMatrix_TotalSpin.cuh:279-311) --
     def rows(self) -> int:

@@ -133,13 +133,19 @@ int64_t ed_op_dim_up(const ed_op* op);
 int64_t ed_op_dim_dn(const ed_op* op);
 int ed_op_is_complex(const ed_op* op);
 
-/* The matvec kernel of the operator's Lanczos steps: ED_MV_GENERIC (one
- * thread per element, or row pairs in shared memory), ED_MV_ROWS (rows staged in shared memory by bulk
- * copies) or ED_MV_TWO_PASS (down sums over a bandwidth-reduced down index,
+/* The matvec that the operator's tables are laid out for: ED_MV_GENERIC (one
+ * thread per element), ED_MV_ROWS (rows and tables staged in shared memory by
+ * bulk copies) or ED_MV_TWO_PASS (down sums over a bandwidth-reduced down index,
  * then the up term over L2-resident column stripes); -1 for a null op.
- * Chosen at ed_op_create from the sector's shape (ED_MATVEC overrides). */
+ * Chosen at ed_op_create from the sector's shape (ED_MATVEC overrides).  Its
+ * Lanczos steps and applies take it, except where ed_op_row_pairs says 1. */
 enum { ED_MV_GENERIC = 0, ED_MV_ROWS = 1, ED_MV_TWO_PASS = 2 };
 int ed_op_matvec_kind(const ed_op* op);
+/* 1: the operator's applies and Lanczos steps run on pairs of rows in shared
+ * memory (real operators with one coefficient per spin: GENERIC sectors whose
+ * rows fit without tables, and ROWS ones from a few million states, whose
+ * tables a tuned plan may still choose for the steps); 0 otherwise. */
+int ed_op_row_pairs(const ed_op* op);
 
 /* y = H x.  mem = ED_MEM_HOST: x, y are host pointers and the call is
  * synchronous — the cuSpectra::Hubbard::perform_op semantics

@@ -90,8 +90,10 @@ public:
     int64_t cols() const { return ed_op_cols(op_); }
     int64_t dimUP() const { return ed_op_dim_up(op_); }
     int64_t dimDN() const { return ed_op_dim_dn(op_); }
-    // ED_MV_ROWS, ED_MV_TWO_PASS or ED_MV_GENERIC: the matvec of its Lanczos steps
+    // ED_MV_ROWS, ED_MV_TWO_PASS or ED_MV_GENERIC: the matvec its tables are for
     int matvec_kind() const { return ed_op_matvec_kind(op_); }
+    // its applies and Lanczos steps run on row pairs
+    bool row_pairs() const { return ed_op_row_pairs(op_) != 0; }
     ed_op* handle() const { return op_; }
 
 private:

@@ -192,3 +192,7 @@ def test_tridiagonal_lowest_vs_scipy(edlib, n):
     assert abs(lam - w[0]) < 1e-12 * max(1.0, np.max(np.abs(w)))
     assert abs(abs(z @ V[:, 0]) - 1.0) < 1e-9
     assert np.max(np.abs(z)) == np.max(z)  # largest component positive
+
+
+def test_row_pairs_of_no_operator(edlib):
+    assert edlib.ed_op_row_pairs(None) == 0

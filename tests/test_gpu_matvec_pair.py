@@ -125,3 +125,28 @@ def test_pair_chosen_by_size(ed, monkeypatch, N, qu, qd):
         assert np.array_equal(r[1], runs[0][1])
     op.close()
     ref.close()
+
+
+def test_operators_say_whether_they_run_row_pairs(ed, monkeypatch):
+    """row_pairs: true for every operator the tests above force onto the pairs (so
+    that they compare two kernels) and for those the size rule sends there, false
+    for the generic kernel, small, complex, multi-class and two-pass ones."""
+    from exact_diagonalization_for_fermionic_systems_with_gpu_gb300 import lattices as L
+    def op(N, qu, qd, ut, dt=None):
+        return ed.Hubbard(ed.H_TBq(N, qu).extend(ut), ed.H_TBq(N, qd).extend(ut if dt is None else dt), 2.0)
+    forced = [c[1:6] for c in pair_cases()] + [(N, qu, qd, L.chain(N, periodic=N % 2 == 1), None) for N, qu, qd in
+                                               ((12, 6, 2), (13, 6, 4), (14, 6, 7), (15, 4, 6), (16, 4, 8), (23, 3, 4))]
+    for N, qu, qd, ut, dt in forced:
+        for kind in ("pair", "generic"):
+            monkeypatch.setenv("ED_MATVEC", kind)
+            o = op(N, qu, qd, ut, dt)
+            assert o.row_pairs == (kind == "pair"), (N, qu, qd, kind)
+            o.close()
+    monkeypatch.delenv("ED_MATVEC")
+    by_size = [(13, 5, 6), (13, 6, 7), (14, 5, 5), (15, 5, 4), (16, 6, 3), (14, 3, 7), (16, 2, 8)]
+    others = [(12, 6, 6, L.kagome12()), (12, 6, 6, L.kagome12(flux=0.2)), (13, 5, 6, L.chain(13) + [("H", 0, 2, -0.5, 0.0)]),
+              (18, 1, 9, L.lieb18())]
+    for N, qu, qd, t in [(*k, L.chain(k[0])) for k in by_size] + others:
+        o = op(N, qu, qd, t)
+        assert o.row_pairs == ((N, qu, qd) in by_size and len(t) == N), (N, qu, qd, o.matvec_kind)
+        o.close()
