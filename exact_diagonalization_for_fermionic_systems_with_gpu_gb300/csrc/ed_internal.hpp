@@ -132,8 +132,9 @@ struct StripedArgs {
     int* err;
 };
 
-// Row-pair matvec (ed_matvec_pair.cu) for real single-class sectors whose
-// tables do not fit shared memory beside the rows but two rows do.
+// Row-pair matvec (ed_matvec_pair.cu) for real single-class sectors of which two
+// rows fit shared memory: those whose tables do not fit beside them, large ones
+// (prefer_pair), and the batched Lanczos runs of all others.
 struct PairArgs {
     const uint16_t* words;   // PairSchedule
     const uint8_t* steps;

@@ -14,6 +14,12 @@
 // kernel's, so every instance's coefficients are bit-identical to its own run;
 // the batch saves the per-step barrier and scalar time of B - 1 runs.
 //
+// Rows are staged through L1 (pair_stage), which keeps lines of vectors that other
+// CTAs write: right only because every step writes a slot that no CTA has read in
+// this launch (the whole basis is stored) and slots are whole 256-byte blocks, so
+// that no line holds two of them.  Runs that reuse slots cannot go this way.  u,
+// written anew in every step, and the axpy's operands are read past L1.
+//
 // Against the row engine's items (512 threads, two barriers a row) that this
 // replaces, an instance's step in batches of eight (200 steps, Ritz sums included):
 // 12-site chain 7+5 24.2 -> 17.5 us (20.4 with two buffers, 26 units for 31 warps,

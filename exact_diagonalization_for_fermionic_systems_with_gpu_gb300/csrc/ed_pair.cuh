@@ -116,7 +116,8 @@ __device__ __forceinline__ void pair_init(unsigned char* xs, const PairArgs& g, 
 }
 
 // Rows u0 and u0 + 1 (an odd count ends on a pair of one row) into a buffer:
-// thread i0 of n.  dUPq: the folded up diagonal.
+// thread i0 of n.  dUPq: the folded up diagonal.  The copies go through L1: xq was
+// written before the launch, or lies where nothing has been read since it began.
 __device__ __forceinline__ void pair_stage(const MvArgs& a, const int64_t* xq, const int64_t* dUPq, uint32_t u0,
                                            const PairBuf& B, uint32_t i0, uint32_t n) {
     const uint32_t dimDN = (uint32_t)a.dimDN;
