@@ -12,6 +12,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 ROOT = Path(__file__).resolve().parents[1]
+PYPATH = os.pathsep.join([str(ROOT)] + ([os.environ["PYTHONPATH"]] if os.environ.get("PYTHONPATH") else []))
 
 CHILD = r"""
 import ctypes, os
@@ -43,7 +44,7 @@ def test_batch_builds_the_tables_it_uses(ed, tmp_path):
     so = tmp_path / "count_malloc.so"
     subprocess.run([cc, "-shared", "-fPIC", "-O1", str(ROOT / "tests/cpp/count_malloc.c"), "-o", str(so), "-ldl"],
                    check=True)
-    r = subprocess.run([sys.executable, "-c", CHILD], env=dict(os.environ, PYTHONPATH=str(ROOT), LD_PRELOAD=str(so)),
+    r = subprocess.run([sys.executable, "-c", CHILD], env=dict(os.environ, PYTHONPATH=PYPATH, LD_PRELOAD=str(so)),
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     assert [int(v) for v in r.stdout.split()] == [0, 0, 1, 0]
@@ -77,7 +78,7 @@ def test_operator_uploads_the_tables_it_uses(ed, tmp_path):
     so = tmp_path / "count_malloc.so"
     subprocess.run([cc, "-shared", "-fPIC", "-O1", str(ROOT / "tests/cpp/count_malloc.c"), "-o", str(so), "-ldl"],
                    check=True)
-    r = subprocess.run([sys.executable, "-c", CREATE], env=dict(os.environ, PYTHONPATH=str(ROOT), LD_PRELOAD=str(so)),
+    r = subprocess.run([sys.executable, "-c", CREATE], env=dict(os.environ, PYTHONPATH=PYPATH, LD_PRELOAD=str(so)),
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     assert [int(v) for v in r.stdout.split()] == [4, 1]

@@ -13,6 +13,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 ROOT = Path(__file__).resolve().parents[1]
+PYPATH = os.pathsep.join([str(ROOT)] + ([os.environ["PYTHONPATH"]] if os.environ.get("PYTHONPATH") else []))
 
 CHILD = r"""
 import sys
@@ -65,7 +66,7 @@ def run(tmp_path, what, refuse):
     got = {}
     for form in ("refused", "plain"):
         out = tmp_path / f"{form}.npz"
-        env = dict(os.environ, PYTHONPATH=str(ROOT), LD_PRELOAD=str(so))
+        env = dict(os.environ, PYTHONPATH=PYPATH, LD_PRELOAD=str(so))
         if form == "refused":
             env["REFUSE_COOP"] = str(refuse)
         r = subprocess.run([sys.executable, "-c", CHILD, what, str(out)], env=env, capture_output=True, text=True)
